@@ -352,6 +352,7 @@ __global__ void kb_reorder_bodies(BumpySys *bs) {
     d.v.rad_t[s] = d.v.rad[o];
     d.v.mass_t[s] = d.v.mass[o];
     d.v.sidx_t[s] = d.v.sidx[o];
+    d.v.q[s] = quant_of(d.p, p, d.v.rad[o]);  // nothing in this kernel reads q
     x.w_t[s] = x.w[o];
     x.th_t[s] = x.th[o];
     x.tq_t[s] = x.tq[o];

@@ -46,6 +46,10 @@ struct dpg_bumpy_system {
     bool adam_ready = false, have_snapshot = false;
     double snap_box[2] = {0.0, 0.0};
     double switch_fmax = 1e-6;  // mixed form: FP32 vertex pairs until max(|F|, |tau|) <= this
+    // body list rows: nlg lanes per body, ntpb threads per block
+    int nlg = 1, ntpb = kTPB;
+    int ngrid() const { return std::max(1, (int)(((long long)nb * nlg + ntpb - 1) / ntpb)); }
+    void *nlist_fn() const { return nlg == 8 ? (void *)k_nlist_cell<8> : (void *)k_nlist_cell<1>; }
     int gb(int count) const { return std::max(1, (count + kTPB - 1) / kTPB); }
     int gw(int bodies) const { return std::max(1, (bodies + kWarpsPerBlock - 1) / kWarpsPerBlock); }
     DevSys *ds() const { return &d->b; }
@@ -143,10 +147,15 @@ extern "C" int dpg_bumpy_create(const dpg_bumpy_params *p, void *cuda_stream, dp
     A((void **)&v.pos_t, nb * 16); A((void **)&v.vel_t, nb * 16); A((void **)&v.frc_t, nb * 16);
     A((void **)&v.rad_t, nb * 8); A((void **)&v.mass_t, nb * 8); A((void **)&v.sidx_t, nb * 4);
     A((void **)&v.m1, nb * 16); A((void **)&v.m2, nb * 16); A((void **)&v.m1_t, nb * 16); A((void **)&v.m2_t, nb * 16);
+    A((void **)&v.q, nb * 16);
     A((void **)&w.pos_n, nb * 16); A((void **)&w.pos_c, nb * 16); A((void **)&w.pe, nb * 8);
     A((void **)&w.count, nb * 4); A((void **)&w.cell_raw, nb * 4); A((void **)&w.cell_of, nb * 4);
     A((void **)&w.perm, nb * 4);
-    w.max_blocks = std::max(s->gb(s->nb), s->gw(s->nb));
+    int dev = 0, nsm = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    s->nlg = (long long)s->nb < (long long)nsm * 1024 ? 8 : 1;
+    s->ntpb = (long long)s->nb * s->nlg < (long long)nsm * 2 * kTPB ? 64 : kTPB;
+    w.max_blocks = std::max(std::max(s->gb(s->nb), s->gw(s->nb)), s->ngrid());
     A((void **)&w.partials, (size_t)w.max_blocks * 8 * 8);
     A((void **)&x.w, nb * 8); A((void **)&x.th, nb * 8); A((void **)&x.tq, nb * 8); A((void **)&x.I, nb * 8);
     A((void **)&x.nvb, nb * 4); A((void **)&x.start, nb * 4);
@@ -176,10 +185,8 @@ extern "C" int dpg_bumpy_create(const dpg_bumpy_params *p, void *cuda_stream, dp
     // the vertex kernels (BumpyExt.mixed, vpk) on the same mixed grid
     pp.n = s->nb; pp.method = -1; pp.cap = 4; pp.precision = DPG_FP64;
     pp.box[0] = p->box_x; pp.box[1] = p->box_y; pp.e_c = p->e_c; pp.n_c = p->n_c;
-    if (p->precision == DPG_MIXED) {
-        mixed_grid_init(pp);
-        mixed_grid_update(pp);
-    }
+    if (p->precision == DPG_MIXED) mixed_grid_init(pp);
+    params_update(pp);
     memset(&s->h.b.s, 0, sizeof(DevState));
     x.nv = s->nv; x.capv = 4; x.rotation = p->rotation ? 1 : 0; x.rv = p->vertex_radius;
     x.mixed = p->precision == DPG_MIXED ? 1 : 0;
@@ -391,8 +398,17 @@ static int alloc_lists(BS *s, int cap, int capv) {
     return DPG_OK;
 }
 
+// the body list alone (cell method), from the current cell list
+static int launch_nlist_cell(BS *s) {
+    DevSys *ds = &s->d->b;
+    void *args[] = {&ds};
+    CK(cudaLaunchKernel(s->nlist_fn(), dim3(s->ngrid()), dim3(s->ntpb), args, 0, s->stream));
+    return DPG_OK;
+}
+
 static int enqueue_rebuild(BS *s) {
     DevSys *ds = &s->d->b;
+    LAUNCH(k_quant_rebuild, s->gb(s->nb), kTPB, ds);
     if (s->method == DPG_NEIGH_CELL) {
         LAUNCH(k_cell_index, s->gb(s->nb), kTPB, ds);
         LAUNCH(k_cell_scan, 1, kScanTPB, ds);
@@ -401,7 +417,7 @@ static int enqueue_rebuild(BS *s) {
         LAUNCH(kb_reorder_bodies, s->gb(s->nb), kTPB, s->d);
         LAUNCH(kb_scan_starts, 1, kScanTPB, s->d);
         LAUNCH(kb_reorder_vertices, s->gw(s->nb), kTPB, s->d);
-        LAUNCH(k_nlist_cell, s->gb(s->nb), kTPB, ds);
+        TRY(launch_nlist_cell(s));
     } else {
         LAUNCH(k_nlist_all, s->gb(s->nb), kTPB, ds);
     }
@@ -430,7 +446,7 @@ static int resolve_overflow(BS *s) {
             TRY(put(s, &s->d->b.s.n_rebuilds, s->hs->n_rebuilds - 1));
             // the vertex list was built from the truncated body list: rebuild it too
             TRY(put(s, &s->d->x.vlist_built, -1LL));
-            if (s->method == DPG_NEIGH_CELL) LAUNCH(k_nlist_cell, s->gb(s->nb), kTPB, &s->d->b);
+            if (s->method == DPG_NEIGH_CELL) TRY(launch_nlist_cell(s));
             else LAUNCH(k_nlist_all, s->gb(s->nb), kTPB, &s->d->b);
         } else {
             TRY(put(s, &s->d->x.vlist_built, s->hs->n_rebuilds - 1));
@@ -504,7 +520,7 @@ extern "C" int dpg_bumpy_setup_neighbors(dpg_bumpy_handle s, const dpg_neighbor_
     DevParams &p = s->h.b.p;
     p.method = s->method; p.ncd = s->ncd; p.ncells = s->ncells; p.cap = s->cap;
     p.cutoff2 = s->cutoff * s->cutoff; p.cell_size = s->cs; p.nthr2 = s->nthr2; p.cthr2 = s->cthr2;
-    mixed_grid_update(p);
+    params_update(p);
     CK(cudaMemcpyAsync(&s->d->b.p, &p, sizeof(DevParams), cudaMemcpyHostToDevice, s->stream));
     TRY(put(s, &s->d->x.vcut2, s->vcutoff * s->vcutoff));
     TRY(put(s, &s->d->x.vpcut2, s->vpcutoff * s->vpcutoff));
@@ -618,7 +634,7 @@ extern "C" int dpg_bumpy_scale_box(dpg_bumpy_handle s, double factor) {
     s->h.b.p.box[0] = nl;
     s->h.b.p.box[1] = nl;
     if (s->ncd > 0) { s->cs = nl / s->ncd; s->h.b.p.cell_size = s->cs; }
-    mixed_grid_update(s->h.b.p);
+    params_update(s->h.b.p);
     CK(cudaMemcpyAsync(&s->d->b.p, &s->h.b.p, sizeof(DevParams), cudaMemcpyHostToDevice, s->stream));
     return DPG_OK;
 }
@@ -688,7 +704,7 @@ static int build_graph(BS *s, int kind) {
     if (err == cudaSuccess) err = cudaGraphAddNode(&inode, body, &last, nullptr, 1, &ip);
     if (err == cudaSuccess) {
         cudaGraph_t ib = ip.conditional.phGraph_out[0];
-        cudaGraphNode_t prev = nullptr;
+        cudaGraphNode_t prev = addk(ib, nullptr, (void *)k_quant_rebuild, GB, kTPB, a_d, &err);
         if (s->method == DPG_NEIGH_CELL) {
             prev = addk(ib, prev, (void *)k_cell_index, GB, kTPB, a_d, &err);
             prev = addk(ib, prev, (void *)k_cell_scan, 1, kScanTPB, a_d, &err);
@@ -697,7 +713,7 @@ static int build_graph(BS *s, int kind) {
             prev = addk(ib, prev, (void *)kb_reorder_bodies, GB, kTPB, a_b, &err);
             prev = addk(ib, prev, (void *)kb_scan_starts, 1, kScanTPB, a_b, &err);
             prev = addk(ib, prev, (void *)kb_reorder_vertices, GW, kTPB, a_b, &err);
-            prev = addk(ib, prev, (void *)k_nlist_cell, GB, kTPB, a_d, &err);
+            prev = addk(ib, prev, s->nlist_fn(), s->ngrid(), s->ntpb, a_d, &err);
         } else {
             prev = addk(ib, prev, (void *)k_nlist_all, GB, kTPB, a_d, &err);
         }
@@ -1009,7 +1025,7 @@ extern "C" int dpg_bumpy_restore_state(dpg_bumpy_handle s) {
     // Particle::setBoxSize: the box only; the cell size keeps its value
     s->h.b.p.box[0] = s->snap_box[0];
     s->h.b.p.box[1] = s->snap_box[1];
-    mixed_grid_update(s->h.b.p);
+    params_update(s->h.b.p);
     CK(cudaMemcpyAsync(&s->d->b.p, &s->h.b.p, sizeof(DevParams), cudaMemcpyHostToDevice, s->stream));
     TRY(rebuild_now(s, 1));
     return vrefresh(s);
@@ -1119,7 +1135,7 @@ extern "C" int dpg_bumpy_set_box(dpg_bumpy_handle s, double bx, double by) {
     s->h.b.p.box[0] = bx;
     s->h.b.p.box[1] = by;
     if (s->ncd > 0) { s->cs = bx / s->ncd; s->h.b.p.cell_size = s->cs; }
-    mixed_grid_update(s->h.b.p);
+    params_update(s->h.b.p);
     CK(cudaMemcpyAsync(&s->d->b.p, &s->h.b.p, sizeof(DevParams), cudaMemcpyHostToDevice, s->stream));
     return DPG_OK;
 }

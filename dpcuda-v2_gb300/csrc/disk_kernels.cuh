@@ -44,75 +44,215 @@ __device__ __forceinline__ double disk_pair(double xi, double yi, double ri, dou
     return energy;
 }
 
-// sum of pair forces / energies over particle i's neighbour row
-// (kernelCalcDiskForces, src/particles/disk/kernels.cu:11-57)
-__device__ __forceinline__ void disk_force_sum(const DevSys *__restrict__ ds, int i, double2 pi,
-                                               double ri, const double2 *__restrict__ pos,
-                                               const double *__restrict__ rad,
-                                               const int *__restrict__ nbr, double &ax, double &ay,
-                                               double &en) {
-    const int n = ds->p.n;
-    const double bx = ds->p.box[0], by = ds->p.box[1], e_c = ds->p.e_c, n_c = ds->p.n_c;
-    int cnt = ds->w.count[i];
-    if (cnt > ds->p.cap) cnt = ds->p.cap;
-    ax = 0.0; ay = 0.0; en = 0.0;
-    for (int k = 0; k < cnt; k++) {
-        int j = __ldg(&nbr[(size_t)k * n + i]);
-        double2 pj = pos[j];
-        double fx, fy;
-        double e = disk_pair(pi.x, pi.y, ri, pj.x, pj.y, __ldg(&rad[j]), bx, by, e_c, n_c, fx, fy);
-        ax += fx;
-        ay += fy;
-        en += e;
+// ---- FP64 pair sums of the particles of a warp ---------------------------------
+// kernelCalcDiskForces (src/particles/disk/kernels.cu:11-57): per particle, the
+// sum of its pair terms in neighbour-slot order.  Pairs that do not touch add
+// +0.0, which leaves a sum that started at +0.0 unchanged, so only the
+// contacts need FP64 work.  Bound: the FP64 pipe (2 lanes a clock on each SM;
+// a contact is ~45 FP64 instructions, one square root and two divisions among
+// them), where an instruction costs the same with one active lane as with 32.
+// So a warp (32 / G particles, G lanes each) works in three steps: G lanes test
+// a particle's slots by the fixed-point filter; the surviving pairs of all its
+// particles are queued in shared memory, ordered by particle and slot, and
+// evaluated 32 at a time, whoever they belong to; each particle then adds its
+// own results in slot order, so the sums are those of the sequential loop, bit
+// for bit, for every G.  A loop over slots instead runs as many FP64 rounds as
+// the longest list of the warp has entries (~12 against ~4 queue rounds at 6.5
+// neighbours and 3.3 contacts a particle).
+// Measured at 2^20 disks of 3.3 contacts: k_nve_second 1219 -> 453 us; at 16384
+// (2 lanes) k_fire_force 46 -> 32 us; k_stress of 131071 disks 262 -> 126 us.
+constexpr int kSlotChunk = 16;   // slots filtered before the queue is worked off
+constexpr int kPairWin = 160;    // queue entries evaluated before they are added up:
+                                 // 32 particles with 5 contacts each
+template <int K>
+struct PairWarp {                // shared memory of one warp
+    unsigned short ent[32 * kSlotChunk];  // owner lane << 5 | slot in the chunk
+    double r[K][kPairWin];                // the terms of each entry
+};
+constexpr int kForceTPB = 256;   // threads per block of the force kernels
+typedef PairWarp<3> ForceWarp;   // force x, force y, energy
+
+// what the pair sums read (the caller may keep it in registers)
+struct PairArgs {
+    const double2 *pos;
+    const double *rad;
+    const int *nbr;
+    const uint4 *q;
+    int n;
+    double bx, by, e_c, n_c;
+    int l4x, l4y;
+    float sx, sy, tol;
+};
+
+__device__ __forceinline__ PairArgs pair_args(const DevSys *ds) {
+    return {ds->v.pos, ds->v.rad, ds->v.nbr, ds->v.q, ds->p.n, ds->p.box[0], ds->p.box[1], ds->p.e_c,
+            ds->p.n_c, ds->p.q_l4[0], ds->p.q_l4[1], ds->p.q_s[0], ds->p.q_s[1], ds->p.q_tol};
+}
+
+// disk_pair for the sums (see pbc_dist_sum)
+__device__ __forceinline__ double disk_pair_sum(const PairArgs &f, double2 pi, double ri, double2 pj,
+                                                double rj, double &dx, double &dy, double &fx,
+                                                double &fy) {
+    dx = pbc_dist_sum(pi.x, pj.x, f.bx, f.l4x);
+    dy = pbc_dist_sum(pi.y, pj.y, f.by, f.l4y);
+    const double rs = ri + rj;
+    const double d2 = dx * dx + dy * dy;
+    fx = 0.0;
+    fy = 0.0;
+    if (d2 >= rs * rs) return 0.0;
+    const double d = sqrt(d2);
+    const double ov = 1.0 - (d / rs);
+    double ovp, energy;
+    if (f.n_c == 2.0) {  // pow(ov, 1) == ov, and x / 4 == x * 0.25 exactly
+        ovp = ov;
+        energy = f.e_c * ov * ovp * 0.25;
+    } else {
+        ovp = pow(ov, f.n_c - 1);
+        energy = f.e_c * ov * ovp / (2.0 * f.n_c);
+    }
+    const double fm = f.e_c * ovp / (rs * d);
+    fx = fm * dx;
+    fy = fm * dy;
+    return energy;
+}
+
+// Slots s0 .. s0 + kSlotChunk - 1 of the particle's list that may touch it, as
+// bits (every lane of the group gets them).  cnt: its list length.  All lanes
+// of the warp call it.
+template <int G>
+__device__ __forceinline__ unsigned touch_bits(const PairArgs &f, int i, uint4 qi, int s0, int cnt) {
+    const int sub = threadIdx.x & (G - 1), lead = (threadIdx.x & 31) - sub;
+    unsigned bits = 0;
+    if (G == 1) {
+#pragma unroll
+        for (int u0 = 0; u0 < kSlotChunk; u0 += 4) {
+            if (s0 + u0 >= cnt) break;
+            int j[4];
+            uint4 qj[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) j[u] = s0 + u0 + u < cnt ? f.nbr[(size_t)(s0 + u0 + u) * f.n + i] : i;
+#pragma unroll
+            for (int u = 0; u < 4; u++) qj[u] = f.q[j[u]];
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (s0 + u0 + u < cnt && quant_touch(f.sx, f.sy, f.tol, qi, qj[u])) bits |= 1u << (u0 + u);
+        }
+    } else {
+        constexpr int R = kSlotChunk / G;
+        int j[R];
+        uint4 qj[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const int k = s0 + r * G + sub;
+            j[r] = k < cnt ? f.nbr[(size_t)k * f.n + i] : i;
+        }
+#pragma unroll
+        for (int r = 0; r < R; r++) qj[r] = f.q[j[r]];
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const bool hit = s0 + r * G + sub < cnt && quant_touch(f.sx, f.sy, f.tol, qi, qj[r]);
+            const unsigned b = __ballot_sync(0xffffffffu, hit);
+            bits |= ((b >> lead) & ((1u << G) - 1u)) << (r * G);
+        }
+    }
+    return bits;
+}
+
+// Adds the terms of particle i's pairs (list length cnt; 0 for lanes past the
+// last particle, whose i must still be a valid index) to acc: K = 3 force x,
+// force y, energy; K = 4 the stress terms xx, xy, yx, yy
+// (kernelCalcDiskStressTensor, src/particles/disk/kernels.cu:203-252).  Every
+// lane of a group passes the same particle and gets its sums.  All lanes of
+// the warp call it.
+template <int G, int K>
+__device__ __forceinline__ void pair_sums(const PairArgs &f, int i, int cnt, PairWarp<K> &w,
+                                          double (&acc)[K]) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31, sub = lane & (G - 1), lead = lane - sub;
+    const uint4 qi = f.q[i];
+    const int most = (int)__reduce_max_sync(kAll, (unsigned)cnt);
+    for (int s0 = 0; s0 < most; s0 += kSlotChunk) {
+        const unsigned bits = touch_bits<G>(f, i, qi, s0, cnt);
+        const int c = __popc(bits);
+        // queue offsets: exclusive scan of the particles' counts
+        int incl = sub == 0 ? c : 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(kAll, incl, o);
+            if (lane >= o) incl += y;
+        }
+        const int total = __shfl_sync(kAll, incl, 31);
+        const int end = __shfl_sync(kAll, incl, lead), off = end - c;
+        // lane sub of the group queues its slots sub, sub + G, ...
+        if (G == 1) {
+            int at = off;
+            for (unsigned m = bits; m; m &= m - 1) w.ent[at++] = (unsigned short)(lane << 5 | (__ffs(m) - 1));
+        } else {
+#pragma unroll
+            for (int r = 0; r < kSlotChunk / G; r++) {
+                const int k = r * G + sub;
+                if (bits >> k & 1u) w.ent[off + __popc(bits & ((1u << k) - 1u))] = (unsigned short)(lane << 5 | k);
+            }
+        }
+        __syncwarp();
+        for (int w0 = 0; w0 < total; w0 += kPairWin) {
+            const int w1 = min(total, w0 + kPairWin);
+            for (int e0 = w0; e0 < w1; e0 += 32) {
+                const int e = e0 + lane;
+                const int ent = e < w1 ? w.ent[e] : lane << 5;
+                const int io = __shfl_sync(kAll, i, ent >> 5);
+                if (e < w1) {
+                    const int j = f.nbr[(size_t)(s0 + (ent & 31)) * f.n + io];
+                    double dx, dy, fx, fy;
+                    const double ee = disk_pair_sum(f, f.pos[io], f.rad[io], f.pos[j], f.rad[j], dx, dy, fx, fy);
+                    if (K == 3) {
+                        w.r[0][e - w0] = fx;
+                        w.r[1][e - w0] = fy;
+                        w.r[2][e - w0] = ee;
+                    } else {
+                        w.r[0][e - w0] = dx * fx / 2;
+                        w.r[1][e - w0] = dx * fy / 2;
+                        w.r[2][e - w0] = dy * fx / 2;
+                        w.r[K - 1][e - w0] = dy * fy / 2;
+                    }
+                }
+            }
+            __syncwarp();
+            const int b0 = max(off, w0) - w0, b1 = min(end, w1) - w0;
+            if (G >= K) {  // lanes 0 .. K - 1 of a group add one term each
+                double s = acc[0];
+#pragma unroll
+                for (int k = 1; k < K; k++) s = sub == k ? acc[k] : s;
+                if (sub < K)
+                    for (int b = b0; b < b1; b++) s += w.r[sub][b];
+#pragma unroll
+                for (int k = 0; k < K; k++) acc[k] = __shfl_sync(kAll, s, lead + k);
+            } else {
+                for (int b = b0; b < b1; b++)
+#pragma unroll
+                    for (int k = 0; k < K; k++) acc[k] += w.r[k][b];
+            }
+            __syncwarp();
+        }
     }
 }
 
-// The same sum with G threads per particle (G a power of two <= 32, groups
-// aligned inside a warp): lane `sub` of the group evaluates neighbour slots
-// sub, sub + G, ...; the pair terms are then shuffled so that every lane of
-// the group adds them in slot order 0, 1, 2, ..., the order of the sequential
-// loop above, so the result is bit-identical to disk_force_sum.  Small systems
-// get G times more warps in flight to hide the FP64 divide / sqrt latency.
-// Every lane of the warp must call this (shuffles); `valid` is false for lanes
-// past the last particle.
-template <int G>
-__device__ __forceinline__ void disk_force_sum_g(const DevSys *__restrict__ ds, int i, bool valid,
-                                                 double &ax, double &ay, double &en) {
-    const int n = ds->p.n;
-    const double bx = ds->p.box[0], by = ds->p.box[1], e_c = ds->p.e_c, n_c = ds->p.n_c;
-    const double2 *__restrict__ pos = ds->v.pos;
-    const double *__restrict__ rad = ds->v.rad;
-    const int *__restrict__ nbr = ds->v.nbr;
-    int cnt = 0;
-    double2 pi = make_double2(0.0, 0.0);
-    double ri = 0.0;
-    if (valid) {
-        cnt = ds->w.count[i];
-        if (cnt > ds->p.cap) cnt = ds->p.cap;
-        pi = pos[i];
-        ri = rad[i];
-    }
-    const int lane = threadIdx.x & 31, sub = lane & (G - 1), lead = lane - sub;
-    const int rounds = __reduce_max_sync(0xffffffffu, (unsigned)((cnt + G - 1) / G));
-    ax = 0.0; ay = 0.0; en = 0.0;
-    for (int r = 0; r < rounds; r++) {
-        const int k = r * G + sub;
-        double fx = 0.0, fy = 0.0, e = 0.0;
-        if (k < cnt) {
-            int j = __ldg(&nbr[(size_t)k * n + i]);
-            double2 pj = pos[j];
-            e = disk_pair(pi.x, pi.y, ri, pj.x, pj.y, __ldg(&rad[j]), bx, by, e_c, n_c, fx, fy);
-        }
-#pragma unroll
-        for (int t = 0; t < G; t++) {
-            double gx = __shfl_sync(0xffffffffu, fx, lead + t);
-            double gy = __shfl_sync(0xffffffffu, fy, lead + t);
-            double ge = __shfl_sync(0xffffffffu, e, lead + t);
-            if (r * G + t < cnt) {
-                ax += gx;
-                ay += gy;
-                en += ge;
-            }
+// The force sums of one thread's particle without the queue: the FP64
+// refinement of a mixed system, whose FP32 kernels should not carry the
+// queue's shared memory.
+__device__ __forceinline__ void pair_sums_thread(const PairArgs &f, int i, int cnt, double &ax, double &ay,
+                                                 double &en) {
+    const uint4 qi = f.q[i];
+    const double2 pi = f.pos[i];
+    const double ri = f.rad[i];
+    for (int s0 = 0; s0 < cnt; s0 += kSlotChunk) {
+        for (unsigned m = touch_bits<1>(f, i, qi, s0, cnt); m; m &= m - 1) {
+            const int j = f.nbr[(size_t)(s0 + __ffs(m) - 1) * f.n + i];
+            double dx, dy, fx, fy;
+            const double e = disk_pair_sum(f, pi, ri, f.pos[j], f.rad[j], dx, dy, fx, fy);
+            ax += fx;
+            ay += fy;
+            en += e;
         }
     }
 }
@@ -145,31 +285,59 @@ __device__ __forceinline__ void disk_force_sum_mixed(const DevSys *__restrict__ 
     }
 }
 
-// Pair sum of particle i for a force kernel with G threads per particle; the
-// mixed instantiation (M) uses FP32 pairs until the FIRE refinement switches
-// the system to FP64 (DevState.fp64_now).  All lanes of the warp call it.
-template <int G, bool M>
-__device__ __forceinline__ void force_sum(const DevSys *__restrict__ ds, int i, bool valid,
-                                          double &ax, double &ay, double &en) {
+// Pair sum of particle i for a force kernel with G threads per particle.  The
+// mixed instantiation (M, one thread per particle) uses FP32 pairs; only the
+// FIRE force kernel (R) also carries the FP64 pairs of the refinement
+// (DevState.fp64_now, clear outside dpg_fire_minimize): with both, the NVE
+// kernel took 234 us at 2^20 disks, 160 with the FP32 pairs alone.  All lanes
+// of the warp call it.
+template <int G, bool M, bool R = false>
+__device__ __forceinline__ void force_sum(const DevSys *ds, int i, bool valid, double &ax, double &ay,
+                                          double &en) {
     ax = 0.0; ay = 0.0; en = 0.0;
-    if (M && !ds->s.fp64_now) {
-        if (valid) disk_force_sum_mixed(ds, i, ax, ay, en);
-        return;
-    }
-    if (G == 1) {
-        if (valid) {
-            const double2 *__restrict__ pos = ds->v.pos;
-            disk_force_sum(ds, i, pos[i], ds->v.rad[i], pos, ds->v.rad, ds->v.nbr, ax, ay, en);
-        }
+    if constexpr (M) {
+        if (!valid) return;
+        if (!R || !ds->s.fp64_now) disk_force_sum_mixed(ds, i, ax, ay, en);
+        else pair_sums_thread(pair_args(ds), i, min(ds->w.count[i], ds->p.cap), ax, ay, en);
     } else {
-        disk_force_sum_g<G>(ds, i, valid, ax, ay, en);
+        __shared__ ForceWarp w[kForceTPB / 32];
+        const int cnt = valid ? min(ds->w.count[i], ds->p.cap) : 0;
+        double acc[3] = {0.0, 0.0, 0.0};
+        pair_sums<G, 3>(pair_args(ds), valid ? i : 0, cnt, w[threadIdx.x >> 5], acc);
+        ax = acc[0]; ay = acc[1]; en = acc[2];
     }
+}
+
+// fixed-point positions of every particle from the current positions
+__global__ void k_quant(DevSys *ds) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= ds->p.n) return;
+    ds->v.q[i] = quant_of(ds->p, ds->v.pos[i], ds->v.rad[i]);
+}
+
+// the same as the first kernel of a rebuild inside a loop whose move kernel
+// does not keep them (mixed form)
+__global__ void k_quant_rebuild(DevSys *ds) {
+    if (ds->s.rebuild == 0) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= ds->p.n) return;
+    ds->v.q[i] = quant_of(ds->p, ds->v.pos[i], ds->v.rad[i]);
 }
 
 // mixed disk systems only (rigid-body systems keep their vertex offsets in
 // BumpyExt and leave the body DevParams at FP64)
 __device__ __forceinline__ void mixed_update(DevSys *ds, int i, double2 p) {
     if (ds->p.precision == kMixed && ds->v.pk) ds->v.pk[i] = mixed_pack(ds->p, p, ds->v.rad[i]);
+}
+
+// what the loops' move kernels keep current with the positions: the mixed
+// form's packed offsets (its FP32 pairs read them), or the fixed-point
+// positions (a mixed system's are refreshed when its lists are rebuilt, and on
+// every move once its pairs are FP64)
+__device__ __forceinline__ void moved_update(DevSys *ds, int i, double2 p) {
+    const double r = ds->v.rad[i];
+    if (ds->p.precision == kMixed) ds->v.pk[i] = mixed_pack(ds->p, p, r);
+    if (ds->p.precision != kMixed || ds->s.fp64_now) ds->v.q[i] = quant_of(ds->p, p, r);
 }
 
 // mixed form: offsets of every particle from the current positions
@@ -269,15 +437,9 @@ __global__ void k_force_acc(DevSys *ds) {
     const int gid = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = gid / G;
     double ax, ay, en;
-    if (G == 1) {
-        if (i >= ds->p.n) return;
-        if (ds->w.count[i] == 0) return;
-        force_sum<1, M>(ds, i, true, ax, ay, en);
-    } else {
-        force_sum<G, M>(ds, i, i < ds->p.n, ax, ay, en);
-        if (i >= ds->p.n || (gid & (G - 1)) != 0) return;
-        if (ds->w.count[i] == 0) return;
-    }
+    force_sum<G, M>(ds, i, i < ds->p.n, ax, ay, en);
+    if (i >= ds->p.n || (gid & (G - 1)) != 0) return;
+    if (ds->w.count[i] == 0) return;
     double2 *frc = ds->v.frc;
     double2 f = frc[i];
     f.x += ax;
@@ -462,53 +624,51 @@ __global__ void k_observables(DevSys *ds) {
 }
 
 // kernelCalcDiskStressTensor: src/particles/disk/kernels.cu:203-252 (summed)
-__global__ void k_stress(DevSys *ds) {
+constexpr int kStressTPB = 128;
+__global__ void __launch_bounds__(kStressTPB) k_stress(DevSys *ds) {
+    __shared__ PairWarp<4> w[kStressTPB / 32];
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double v[4] = {0, 0, 0, 0};
     const int n = ds->p.n;
-    if (i < n) {
-        const double2 *__restrict__ pos = ds->v.pos;
-        const double *__restrict__ rad = ds->v.rad;
-        const int *__restrict__ nbr = ds->v.nbr;
-        const double bx = ds->p.box[0], by = ds->p.box[1], e_c = ds->p.e_c, n_c = ds->p.n_c;
-        double2 pi = pos[i], u = ds->v.vel[i];
-        double m = ds->v.mass[i], ri = rad[i];
-        double axx = m * u.x * u.x, axy = m * u.x * u.y, ayx = axy, ayy = m * u.y * u.y;
-        int cnt = min(ds->w.count[i], ds->p.cap);
-        for (int k = 0; k < cnt; k++) {
-            int j = nbr[(size_t)k * n + i];
-            double2 pj = pos[j];
-            double dx = pbc_dist(pi.x, pj.x, bx), dy = pbc_dist(pi.y, pj.y, by);
-            double fx, fy;
-            disk_pair(pi.x, pi.y, ri, pj.x, pj.y, rad[j], bx, by, e_c, n_c, fx, fy);
-            axx += dx * fx / 2;
-            axy += dx * fy / 2;
-            ayx += dy * fx / 2;
-            ayy += dy * fy / 2;
-        }
-        double area = ds->p.box[0] * ds->p.box[1];
-        v[0] = axx / area; v[1] = axy / area; v[2] = ayx / area; v[3] = ayy / area;
+    double v[4] = {0, 0, 0, 0};
+    const bool valid = i < n;
+    if (valid) {
+        const double2 u = ds->v.vel[i];
+        const double m = ds->v.mass[i];
+        v[0] = m * u.x * u.x;
+        v[1] = m * u.x * u.y;
+        v[2] = v[1];
+        v[3] = m * u.y * u.y;
     }
+    pair_sums<1, 4>(pair_args(ds), valid ? i : 0, valid ? min(ds->w.count[i], ds->p.cap) : 0,
+                    w[threadIdx.x >> 5], v);
+    const double area = ds->p.box[0] * ds->p.box[1];
+#pragma unroll
+    for (int k = 0; k < 4; k++) v[k] = valid ? v[k] / area : 0.0;
     const int ops[4] = {0, 0, 0, 0};
     if (grid_reduce<4>(v, ops, ds))
         for (int k = 0; k < 4; k++) ds->s.stress[k] = v[k];
 }
 
-// kernelCountDiskContacts: src/particles/disk/kernels.cu:177-201 (summed)
+// kernelCountDiskContacts: src/particles/disk/kernels.cu:177-201 (summed); the
+// fixed-point distance decides all pairs but those within 1e-5 of touching
 __global__ void k_contacts(DevSys *ds) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     double v[1] = {0.0};
     const int n = ds->p.n;
     if (i < n) {
-        const double2 *__restrict__ pos = ds->v.pos;
-        const double *__restrict__ rad = ds->v.rad;
-        double2 pi = pos[i];
+        const PairArgs f = pair_args(ds);
+        const uint4 qi = f.q[i];
         int cnt = min(ds->w.count[i], ds->p.cap), c = 0;
         for (int k = 0; k < cnt; k++) {
-            int j = ds->v.nbr[(size_t)k * n + i];
-            double2 pj = pos[j];
-            double dx = pbc_dist(pi.x, pj.x, ds->p.box[0]), dy = pbc_dist(pi.y, pj.y, ds->p.box[1]);
-            if (sqrt(dx * dx + dy * dy) < rad[i] + rad[j]) c++;
+            const int j = f.nbr[(size_t)k * n + i];
+            const uint4 qj = f.q[j];
+            const float rs = __uint_as_float(qi.z) + __uint_as_float(qj.z), d2 = quant_d2(f.sx, f.sy, qi, qj);
+            const float lo = rs * 0.99999f - f.tol, hi = rs * 1.00001f + f.tol;
+            if (d2 > hi * hi) continue;
+            if (lo > 0.f && d2 < lo * lo && rs < INFINITY) { c++; continue; }
+            const double2 pi = f.pos[i], pj = f.pos[j];
+            const double dx = pbc_dist(pi.x, pj.x, f.bx), dy = pbc_dist(pi.y, pj.y, f.by);
+            if (sqrt(dx * dx + dy * dy) < f.rad[i] + f.rad[j]) c++;
         }
         v[0] = (double)c;
     }
@@ -674,6 +834,7 @@ __global__ void k_reorder(DevSys *ds) {
         v.rad_t[s] = v.rad[o];
         v.mass_t[s] = v.mass[o];
         v.sidx_t[s] = v.sidx[o];
+        v.q[s] = quant_of(ds->p, p, v.rad[o]);  // nothing in this kernel reads q
         ds->w.cell_of[s] = ds->w.cell_raw[o];
         ds->w.pos_c[s] = p;
     }
@@ -708,78 +869,130 @@ __device__ __forceinline__ void finish_list_build(DevSys *ds, int cnt) {
     }
 }
 
-// kernelUpdateCellNeighborList: src/particles/base/kernels.cu:440-505
-// (3x3 cells, dy outer / dx inner, ascending slot inside each cell).
-__global__ void k_nlist_cell(DevSys *ds) {
-    if (ds->s.rebuild == 0) return;
-    const int n = ds->p.n;
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+// d2 < cutoff2 for particles i and j, decided by the fixed-point distance where
+// it can, by the FP64 test of the reference where it cannot
+__device__ __forceinline__ bool within_cutoff(const DevSys *ds, const double2 *pos, int i, int j, uint4 qi,
+                                              uint4 qj) {
+    const float d2 = quant_d2(ds->p.q_s[0], ds->p.q_s[1], qi, qj);
+    const bool marked = (qi.w | qj.w) != 0;
+    if (!marked && d2 > ds->p.q_out2) return false;
+    if (!marked && d2 < ds->p.q_in2) return true;
+    const double2 pi = pos[i], pj = pos[j];
+    const double dx = pbc_dist(pi.x, pj.x, ds->p.box[0]), dy = pbc_dist(pi.y, pj.y, ds->p.box[1]);
+    return dx * dx + dy * dy < ds->p.cutoff2;
+}
+
+// The neighbour row of particle i from the 3x3 cells around its own
+// (kernelUpdateCellNeighborList, src/particles/base/kernels.cu:440-505: dy
+// outer, dx inner, ascending slot inside each cell), G lanes per particle.
+// The three cells of a row hold consecutive slots (two ranges where the row
+// wraps), so the group reads G neighbouring 16-byte entries at a time; ballots
+// give each hit its place.  Returns the row's length (every lane of the group).
+// Bound: the FP64 distance tests took 2.7 ms for 2^20 disks; the filter leaves
+// one in ~1e5 of them and the pass runs on FP32 and L1: 209 us with one lane a
+// particle, 106 -> 16 us for 16384 disks with eight.  All lanes of the warp
+// call it, with valid = false past the last particle.
+template <int G>
+__device__ __forceinline__ int nlist_row(const DevSys *ds, int i, bool valid) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31, sub = lane & (G - 1), lead = lane - sub;
+    const int n = ds->p.n, ncd = ds->p.ncd, cap = ds->p.cap;
+    const double2 *pos = ds->v.pos;
+    const uint4 *q = ds->v.q;
+    const int *cstart = ds->w.cell_start;
+    int *nbr = ds->v.nbr;
+    const int c = valid ? ds->w.cell_of[i] : 0, cx = c % ncd, cy = c / ncd;
+    const uint4 qi = q[valid ? i : 0];
     int cnt = 0;
-    if (i < n) {
-        const double2 *__restrict__ pos = ds->v.pos;
-        const int *__restrict__ cstart = ds->w.cell_start;
-        int *__restrict__ nbr = ds->v.nbr;
-        const int ncd = ds->p.ncd, cap = ds->p.cap;
-        const double bx = ds->p.box[0], by = ds->p.box[1], c2 = ds->p.cutoff2;
-        double2 pi = pos[i];
-        int c = ds->w.cell_of[i];
-        int cx = c % ncd, cy = c / ncd;
-        for (int oy = -1; oy <= 1; oy++) {
-            int yy = pmod(cy + oy, ncd);
-            for (int ox = -1; ox <= 1; ox++) {
-                int nc = pmod(cx + ox, ncd) + yy * ncd;
-                int b = cstart[nc], e = cstart[nc + 1];
-                for (int j = b; j < e; j++) {
-                    if (j == i) continue;
-                    double2 pj = pos[j];
-                    double dx = pbc_dist(pi.x, pj.x, bx), dy = pbc_dist(pi.y, pj.y, by);
-                    if (dx * dx + dy * dy < c2) {
-                        if (cnt < cap) nbr[(size_t)cnt * n + i] = j;
-                        cnt++;
-                    }
+    for (int oy = -1; oy <= 1; oy++) {
+        const int row = pmod(cy + oy, ncd) * ncd;
+        // cells cx - 1, cx, cx + 1 in this order, as up to two slot ranges
+        int b[2] = {0, 0}, e[2] = {0, 0};
+        if (valid) {
+            const int x0 = cx == 0 ? ncd - 1 : cx - 1;
+            b[0] = cstart[row + x0];
+            if (cx == 0) {
+                e[0] = cstart[row + ncd];
+                b[1] = cstart[row];
+                e[1] = cstart[row + 2];
+            } else if (cx == ncd - 1) {
+                e[0] = cstart[row + ncd];
+                b[1] = cstart[row];
+                e[1] = cstart[row + 1];
+            } else {
+                e[0] = cstart[row + cx + 2];
+            }
+        }
+#pragma unroll
+        for (int g = 0; g < 2; g++) {
+            if (G == 1) {
+                for (int j = b[g]; j < e[g]; j++) {
+                    if (j == i || !within_cutoff(ds, pos, i, j, qi, q[j])) continue;
+                    if (cnt < cap) nbr[(size_t)cnt * n + i] = j;
+                    cnt++;
+                }
+            } else {
+                const int rounds = (int)__reduce_max_sync(kAll, (unsigned)((e[g] - b[g] + G - 1) / G));
+                for (int r = 0; r < rounds; r++) {
+                    const int j = b[g] + r * G + sub;
+                    const bool hit = j < e[g] && j != i && within_cutoff(ds, pos, i, j, qi, q[j]);
+                    const unsigned m = (__ballot_sync(kAll, hit) >> lead) & ((1u << G) - 1u);
+                    const int at = cnt + __popc(m & ((1u << sub) - 1u));
+                    if (hit && at < cap) nbr[(size_t)at * n + i] = j;
+                    cnt += __popc(m);
                 }
             }
         }
+    }
+    return cnt;
+}
+
+template <int G>
+__global__ void k_nlist_cell(DevSys *ds) {
+    if (ds->s.rebuild == 0) return;
+    const int gid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = gid / G;
+    const bool valid = i < ds->p.n;
+    const int cnt = nlist_row<G>(ds, i, valid);
+    if (valid && (gid & (G - 1)) == 0) {
+        const double2 pi = ds->v.pos[i];
         ds->w.count[i] = cnt;
         ds->w.pos_n[i] = pi;
         mixed_update(ds, i, pi);
     }
-    finish_list_build(ds, cnt);
+    finish_list_build(ds, valid ? cnt : 0);
 }
 
 // kernelUpdateNeighborList (all pairs, methods "verlet" / "all"):
 // src/particles/base/kernels.cu:256-293.  j tiles staged in shared memory.
 __global__ void k_nlist_all(DevSys *ds) {
     if (ds->s.rebuild == 0) return;
-    __shared__ double2 tile[kTPB];
+    __shared__ uint4 tile[kTPB];
     const int n = ds->p.n;
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const double2 *__restrict__ pos = ds->v.pos;
-    int *__restrict__ nbr = ds->v.nbr;
+    const double2 *pos = ds->v.pos;
+    const uint4 *q = ds->v.q;
+    int *nbr = ds->v.nbr;
     const int cap = ds->p.cap;
-    const double bx = ds->p.box[0], by = ds->p.box[1], c2 = ds->p.cutoff2;
-    double2 pi = (i < n) ? pos[i] : make_double2(0.0, 0.0);
+    const uint4 qi = q[i < n ? i : 0];
     int cnt = 0;
     for (int base = 0; base < n; base += kTPB) {
         int j0 = base + threadIdx.x;
-        if (j0 < n) tile[threadIdx.x] = pos[j0];
+        if (j0 < n) tile[threadIdx.x] = q[j0];
         __syncthreads();
         int lim = min(kTPB, n - base);
         if (i < n) {
             for (int t = 0; t < lim; t++) {
                 int j = base + t;
-                if (j == i) continue;
-                double2 pj = tile[t];
-                double dx = pbc_dist(pi.x, pj.x, bx), dy = pbc_dist(pi.y, pj.y, by);
-                if (dx * dx + dy * dy < c2) {
-                    if (cnt < cap) nbr[(size_t)cnt * n + i] = j;
-                    cnt++;
-                }
+                if (j == i || !within_cutoff(ds, pos, i, j, qi, tile[t])) continue;
+                if (cnt < cap) nbr[(size_t)cnt * n + i] = j;
+                cnt++;
             }
         }
         __syncthreads();
     }
     if (i < n) {
+        const double2 pi = pos[i];
         ds->w.count[i] = cnt;
         ds->w.pos_n[i] = pi;
         mixed_update(ds, i, pi);
@@ -807,7 +1020,7 @@ __global__ void k_nve_first(DevSys *ds, double dt_half, double dt) {
         p.x = p.x + u.x * dt;
         p.y = p.y + u.y * dt;
         pos[i] = p;
-        mixed_update(ds, i, p);
+        moved_update(ds, i, p);
         double2 a = ds->w.pos_n[i], c = ds->w.pos_c[i];
         double dxn = p.x - a.x, dyn = p.y - a.y, dxc = p.x - c.x, dyc = p.y - c.y;
         v[0] = dxn * dxn + dyn * dyn;
@@ -920,7 +1133,7 @@ __global__ void k_fire_move(DevSys *ds) {
         p.x = p.x + u.x * dt;
         p.y = p.y + u.y * dt;
         pos[i] = p;
-        mixed_update(ds, i, p);
+        moved_update(ds, i, p);
         double2 a = ds->w.pos_n[i], c = ds->w.pos_c[i];
         double dxn = p.x - a.x, dyn = p.y - a.y, dxc = p.x - c.x, dyc = p.y - c.y;
         v[0] = dxn * dxn + dyn * dyn;
@@ -948,7 +1161,7 @@ __global__ void k_fire_force(DevSys *ds, int mode) {
     const int i = gid / G;
     double v[3] = {0.0, 0.0, 0.0};
     double ax, ay, en;
-    force_sum<G, M>(ds, i, i < ds->p.n, ax, ay, en);
+    force_sum<G, M, true>(ds, i, i < ds->p.n, ax, ay, en);
     if (i < ds->p.n && (gid & (G - 1)) == 0) {
         double2 f = make_double2(0.0 + ax, 0.0 + ay);
         ds->v.frc[i] = f;

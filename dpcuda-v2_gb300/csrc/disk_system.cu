@@ -99,6 +99,14 @@ struct dpg_system {
     int fg = 1;
     int ftpb = kTPB;
     int fgrid() const { return std::max(1, (int)(((long long)n * fg + ftpb - 1) / ftpb)); }
+    // the fixed-point positions (DevView.q) match the positions, radii and box:
+    // the loops' move kernels and the re-sort keep them, every other change
+    // clears the flag and the next list build or force pass refreshes them
+    bool q_fresh = false;
+    // cell-list neighbour rows: nlg lanes per particle, ntpb threads per block
+    int nlg = 1, ntpb = kTPB;
+    int ngrid() const { return std::max(1, (int)(((long long)n * nlg + ntpb - 1) / ntpb)); }
+    void *nlist_fn() const { return nlg == 8 ? (void *)k_nlist_cell<8> : (void *)k_nlist_cell<1>; }
     // mixed form (precision DPG_MIXED): FP32 pair kernels, one thread per particle
     bool mixed = false;
     double switch_fmax = 1e-6;
@@ -148,7 +156,8 @@ static void free_graphs(dpg_system *s) {
 }
 
 static int push_params(dpg_system *s) {
-    mixed_grid_update(s->h.p);
+    params_update(s->h.p);
+    s->q_fresh = false;
     CK(cudaMemcpyAsync(&s->d->p, &s->h.p, sizeof(DevParams), cudaMemcpyHostToDevice, s->stream));
     return DPG_OK;
 }
@@ -195,12 +204,23 @@ static int mixed_refresh(dpg_system *s) {
     return DPG_OK;
 }
 
+// fixed-point positions from the current positions, radii and box
+static int quant_refresh(dpg_system *s) {
+    if (s->q_fresh) return DPG_OK;
+    k_quant<<<s->grid(s->n), s->tpb, 0, s->stream>>>(s->d);
+    CK(cudaGetLastError());
+    s->q_fresh = true;
+    return DPG_OK;
+}
+
 static int launch_force_acc(dpg_system *s) {
     TRY(mixed_refresh(s));
+    TRY(quant_refresh(s));
     return launch_fn(s, s->force_acc_fn(), s->fgrid(), s->ftpb, s->d);
 }
 static int launch_fire_force(dpg_system *s, int mode) {
     if (mode != 0) TRY(mixed_refresh(s));
+    if (mode != 0) TRY(quant_refresh(s));
     return launch_fn(s, s->fire_force_fn(), s->fgrid(), s->ftpb, s->d, mode);
 }
 static int launch_nve_second(dpg_system *s, double dt_half) {
@@ -247,7 +267,12 @@ extern "C" int dpg_create(const dpg_params *p, void *cuda_stream, dpg_handle *ou
         int g = atoi(fgs);
         if (g == 1 || g == 2 || g == 4 || g == 8) s->fg = g;
     }
-    s->ftpb = kTPB;
+    s->ftpb = kForceTPB;
+    // list rows: 8 lanes a particle (consecutive entries, short chains) until a
+    // thread a particle fills the GPU, which needs fewer instructions (131071
+    // disks: 68 us with 8 lanes; 2^20: 209 us with one)
+    s->nlg = (long long)s->n < (long long)nsm * 1024 ? 8 : 1;
+    s->ntpb = (long long)s->n * s->nlg < (long long)nsm * 2 * kTPB ? 64 : kTPB;
     s->mixed = p->precision == DPG_MIXED;
     if (s->mixed) s->fg = 1;
     int rc = DPG_OK;
@@ -260,12 +285,14 @@ extern "C" int dpg_create(const dpg_params *p, void *cuda_stream, dpg_handle *ou
     A((void **)&v.rad_t, n * 8); A((void **)&v.mass_t, n * 8); A((void **)&v.sidx_t, n * 4);
     A((void **)&v.m1, n * 16); A((void **)&v.m2, n * 16); A((void **)&v.m1_t, n * 16); A((void **)&v.m2_t, n * 16);
     if (s->mixed) A((void **)&v.pk, n * 16);
+    A((void **)&v.q, n * 16);
     A((void **)&w.pos_n, n * 16); A((void **)&w.pos_c, n * 16); A((void **)&w.pe, n * 8);
     A((void **)&w.count, n * 4); A((void **)&w.cell_raw, n * 4); A((void **)&w.cell_of, n * 4);
     A((void **)&w.perm, n * 4);
     // partials for the widest force group (8 lanes), so the group can change later
     const int fg8 = std::max(1, (int)(((long long)s->n * 8 + s->ftpb - 1) / s->ftpb));
     w.max_blocks = std::max(std::max(s->grid(s->n), s->grid_full(s->n)), std::max(s->fgrid(), fg8));
+    w.max_blocks = std::max(std::max(w.max_blocks, s->ngrid()), (s->n + kStressTPB - 1) / kStressTPB);
     A((void **)&w.partials, (size_t)w.max_blocks * 8 * 8);
     A((void **)&w.s_pos, n * 16); A((void **)&w.s_vel, n * 16); A((void **)&w.s_frc, n * 16);
     A((void **)&w.s_rad, n * 8); A((void **)&w.s_mass, n * 8); A((void **)&w.s_sidx, n * 4);
@@ -279,10 +306,8 @@ extern "C" int dpg_create(const dpg_params *p, void *cuda_stream, dpg_handle *ou
     DevParams &pp = s->h.p;
     pp.n = s->n; pp.method = -1; pp.cap = 4; pp.precision = p->precision;
     pp.box[0] = p->box_x; pp.box[1] = p->box_y; pp.e_c = p->e_c; pp.n_c = p->n_c;
-    if (s->mixed) {
-        mixed_grid_init(pp);
-        mixed_grid_update(pp);
-    }
+    if (s->mixed) mixed_grid_init(pp);
+    params_update(pp);
     memset(&s->h.s, 0, sizeof(DevState));
     rc = [&]() -> int {
         CK(cudaMemcpyAsync(s->d, &s->h, sizeof(DevSys), cudaMemcpyHostToDevice, s->stream));
@@ -341,6 +366,7 @@ static int put_xy(dpg_system *s, int which, const double *x, const double *y, in
     const double *dx, *dy;
     TRY(stage_in(s, x, where, 0, &dx));
     TRY(stage_in(s, y, where, 1, &dy));
+    if (which == 0) s->q_fresh = false;
     LAUNCH(k_put_xy, s->grid(s->n), s->tpb, s->d, which, dx, dy);
     if (where == DPG_HOST) CK(cudaStreamSynchronize(s->stream));
     return DPG_OK;
@@ -358,6 +384,7 @@ extern "C" int dpg_set_state(dpg_handle s, const double *x, const double *y, con
         if (!scal[k]) continue;
         const double *dp;
         TRY(stage_in(s, scal[k], where, 0, &dp));
+        if (k == 0) s->q_fresh = false;
         LAUNCH(k_put_scalar, s->grid(s->n), s->tpb, s->d, k, dp);
         if (where == DPG_HOST) CK(cudaStreamSynchronize(s->stream));
     }
@@ -540,13 +567,17 @@ static int alloc_nbr(dpg_system *s, int cap) {
 }
 
 static int enqueue_nlist(dpg_system *s) {
-    if (s->method == DPG_NEIGH_CELL) LAUNCH(k_nlist_cell, s->grid(s->n), s->tpb, s->d);
-    else LAUNCH(k_nlist_all, s->grid_full(s->n), kTPB, s->d);
+    TRY(quant_refresh(s));
+    if (s->method == DPG_NEIGH_CELL) return launch_fn(s, s->nlist_fn(), s->ngrid(), s->ntpb, s->d);
+    LAUNCH(k_nlist_all, s->grid_full(s->n), kTPB, s->d);
     return DPG_OK;
 }
 
 // the rebuild kernels; each one checks DevState.rebuild itself
 static int enqueue_rebuild(dpg_system *s) {
+    // a mixed system's move kernels do not keep the fixed-point positions
+    if (s->mixed) LAUNCH(k_quant_rebuild, s->grid(s->n), s->tpb, s->d);
+    else TRY(quant_refresh(s));
     if (s->method == DPG_NEIGH_CELL) {
         LAUNCH(k_cell_index, s->grid(s->n), s->tpb, s->d);
         LAUNCH(k_cell_scan, 1, kScanTPB, s->d);
@@ -736,6 +767,7 @@ extern "C" int dpg_kick(dpg_handle s, double dt) {
 
 extern "C" int dpg_drift(dpg_handle s, double dt) {
     if (!s) return set_err(DPG_ERR_ARG, "null handle");
+    s->q_fresh = false;
     LAUNCH(k_drift, s->grid(s->n), s->tpb, s->d, dt);
     return DPG_OK;
 }
@@ -782,7 +814,8 @@ extern "C" int dpg_force_stats(dpg_handle s, double *max_force, double *balance)
 
 extern "C" int dpg_pressure(dpg_handle s, double *pressure, double stress[4]) {
     TRY(need_neighbors(s));
-    LAUNCH(k_stress, s->grid(s->n), s->tpb, s->d);
+    TRY(quant_refresh(s));
+    LAUNCH(k_stress, (s->n + kStressTPB - 1) / kStressTPB, kStressTPB, s->d);
     TRY(pull_state(s));
     if (stress) for (int k = 0; k < 4; k++) stress[k] = s->hs->stress[k];
     if (pressure) *pressure = (s->hs->stress[0] + s->hs->stress[3]) / 2;
@@ -791,6 +824,7 @@ extern "C" int dpg_pressure(dpg_handle s, double *pressure, double stress[4]) {
 
 extern "C" int dpg_contact_count(dpg_handle s, double *contacts) {
     TRY(need_neighbors(s));
+    TRY(quant_refresh(s));
     LAUNCH(k_contacts, s->grid(s->n), s->tpb, s->d);
     TRY(pull_state(s));
     if (contacts) *contacts = s->hs->contacts;
@@ -851,6 +885,7 @@ extern "C" int dpg_save_state(dpg_handle s) {
 // (neighbour list only; the cell arrays are left as they are, like the reference).
 extern "C" int dpg_restore_state(dpg_handle s) {
     TRY(need_neighbors(s));
+    s->q_fresh = false;
     LAUNCH(k_snapshot, s->grid(s->n), s->tpb, s->d, 1);
     s->h.p.box[0] = s->h.w.s_box[0];
     s->h.p.box[1] = s->h.w.s_box[1];
@@ -876,6 +911,7 @@ extern "C" int dpg_adam_step(dpg_handle s, int64_t step, double alpha, double b1
     if (!s->adam_ready) return set_err(DPG_ERR_STATE, "call dpg_adam_init first");
     double c1 = 1 - std::pow(b1, step + 1);
     double c2 = 1 - std::pow(b2, step + 1);
+    s->q_fresh = false;
     LAUNCH(k_adam, s->grid(s->n), s->tpb, s->d, alpha, b1, b2, c1, c2, eps);
     return DPG_OK;
 }
@@ -919,13 +955,14 @@ struct KNode {
 static std::vector<KNode> rebuild_nodes(const dpg_system *s) {
     std::vector<KNode> rb;
     int G = s->grid(s->n);
+    if (s->mixed) rb.push_back({(void *)k_quant_rebuild, G, s->tpb});
     if (s->method == DPG_NEIGH_CELL) {
         rb.push_back({(void *)k_cell_index, G, s->tpb});
         rb.push_back({(void *)k_cell_scan, 1, kScanTPB});
         rb.push_back({(void *)k_cell_scatter, G, s->tpb});
         rb.push_back({(void *)k_cell_sort, s->grid(s->ncells), s->tpb});
         rb.push_back({(void *)k_reorder, G, s->tpb});
-        rb.push_back({(void *)k_nlist_cell, G, s->tpb});
+        rb.push_back({s->nlist_fn(), s->ngrid(), s->ntpb});
     } else {
         rb.push_back({(void *)k_nlist_all, s->grid_full(s->n), kTPB});
     }
@@ -1036,6 +1073,8 @@ static int build_cond_graph(dpg_system *s, int kind) {
 static int run_loop(dpg_system *s, int kind, int *halted_overflow) {
     *halted_overflow = 0;
     TRY(mixed_refresh(s));
+    if (s->mixed) s->q_fresh = false;
+    else TRY(quant_refresh(s));
     if (s->mode == kModeCond) {
         int rc = build_cond_graph(s, kind);
         if (rc != DPG_OK) {
@@ -1187,6 +1226,7 @@ extern "C" int dpg_nve_wall_steps(dpg_handle s, double dt, int64_t n_steps) {
 
 extern "C" int dpg_grad_desc_step(dpg_handle s, double alpha) {
     if (!s) return set_err(DPG_ERR_ARG, "null handle");
+    s->q_fresh = false;
     LAUNCH(k_grad_desc, s->grid(s->n), s->tpb, s->d, alpha);
     return DPG_OK;
 }
@@ -1231,6 +1271,8 @@ extern "C" int dpg_fire_get(dpg_handle s, double *alpha, double *dt, int64_t *n_
 extern "C" int dpg_fire_step(dpg_handle s, int *stopped) {
     TRY(need_neighbors(s));
     TRY(put_field(s, &s->d->s.flags, 0));
+    if (s->mixed) s->q_fresh = false;
+    else TRY(quant_refresh(s));
     LAUNCH(k_fire_power_decide, s->grid(s->n), s->tpb, s->d);
     LAUNCH(k_fire_move, s->grid(s->n), s->tpb, s->d);
     TRY(enqueue_rebuild(s));
@@ -1242,8 +1284,17 @@ extern "C" int dpg_fire_step(dpg_handle s, int *stopped) {
     return DPG_OK;
 }
 
+static int fire_minimize(dpg_system *s, const dpg_fire_params *p, dpg_fire_result *r);
+
 extern "C" int dpg_fire_minimize(dpg_handle s, const dpg_fire_params *p, dpg_fire_result *r) {
     TRY(need_neighbors(s));
+    const int rc = fire_minimize(s, p, r);
+    // later calls start in FP32 again (the other force kernels know no refinement)
+    const int rc2 = s->mixed ? put_field(s, &s->d->s.fp64_now, 0) : DPG_OK;
+    return rc != DPG_OK ? rc : rc2;
+}
+
+static int fire_minimize(dpg_system *s, const dpg_fire_params *p, dpg_fire_result *r) {
     if (!p) return set_err(DPG_ERR_ARG, "null params");
     if (p->max_steps <= 0) return set_err(DPG_ERR_ARG, "max_steps must be > 0");
     TRY(dpg_fire_init(s, p->alpha_init, p->dt));
@@ -1287,7 +1338,6 @@ extern "C" int dpg_fire_minimize(dpg_handle s, const dpg_fire_params *p, dpg_fir
     // minimizeFire ends with setVelocitiesToZero
     LAUNCH(k_zero_vel, s->grid(s->n), s->tpb, s->d);
     TRY(observe(s));
-    TRY(put_field(s, &s->d->s.fp64_now, 0));  // later calls start in FP32 again
     if (r) {
         r->steps = s->hs->result_step;
         r->stopped = s->hs->f_stopped;
@@ -1329,6 +1379,8 @@ extern "C" int dpg_profile_loop(dpg_handle s, int kind, int iters, double dt, do
         TRY(put_field(s, &s->d->s.max_steps, (long long)iters + 1));
     }
     TRY(mixed_refresh(s));
+    if (s->mixed) s->q_fresh = false;
+    else TRY(quant_refresh(s));
     std::vector<cudaEvent_t> ev(4 * (size_t)iters);
     for (auto &e : ev) CK(cudaEventCreate(&e));
     int rc = DPG_OK;
