@@ -573,7 +573,7 @@ __global__ void kb_fire_force(BumpySys *bs, int mode, double tmax_target) {
     double avg = v[0] / s.dof;
     if (mode == 1) {
         s.last_avg_pe = avg;
-        fire_decide(ds, v[1]);
+        fire_decide(s, v[1]);
         return;
     }
     if (mode == 2) return;
@@ -598,7 +598,7 @@ __global__ void kb_fire_force(BumpySys *bs, int mode, double tmax_target) {
     }
     if (it + 1 >= s.max_steps) { s.result_step = s.max_steps; s.flags |= kDone; return; }
     s.iter = it + 1;
-    fire_decide(ds, v[1]);
+    fire_decide(s, v[1]);
     if (s.f_stopped) { s.result_step = it + 1; s.f_converged = 1; s.flags |= kDone; }
 }
 
@@ -615,7 +615,7 @@ __global__ void kb_fire_power_decide(BumpySys *bs) {
     const int ops[1] = {0};
     if (grid_reduce<1>(v, ops, ds)) {
         ds->s.power = v[0];
-        fire_decide(ds, v[0]);
+        fire_decide(ds->s, v[0]);
     }
 }
 

@@ -258,30 +258,55 @@ __device__ __forceinline__ void pair_sums_thread(const PairArgs &f, int i, int c
 }
 
 // Mixed form: FP32 pair forces from the packed offsets, summed in FP32 over
-// runs of 8 neighbours and in FP64 across runs and for the particle total.
-__device__ __forceinline__ void disk_force_sum_mixed(const DevSys *__restrict__ ds, int i,
-                                                     double &ax, double &ay, double &en) {
-    const int n = ds->p.n;
-    const float4 *__restrict__ pk = ds->v.pk;
-    const int *__restrict__ nbr = ds->v.nbr;
-    const float e_c = (float)ds->p.e_c, n_c = (float)ds->p.n_c;
-    int cnt = ds->w.count[i];
-    if (cnt > ds->p.cap) cnt = ds->p.cap;
+// runs of 8 neighbours and in FP64 across runs and for the particle total.  G
+// lanes share a run's pairs (G = 1: the particle's own thread); its terms are
+// added in slot order whatever G is.  cnt: the list length, 0 for lanes past
+// the last particle.  All lanes of the warp call it.
+template <int G>
+__device__ __forceinline__ void mixed_sums(const DevParams &p, const float4 *pk, const int *nbr, int i,
+                                           int cnt, double &ax, double &ay, double &en) {
+    const int n = p.n;
+    const float e_c = (float)p.e_c, n_c = (float)p.n_c;
     const float4 a = pk[i];
     ax = 0.0; ay = 0.0; en = 0.0;
-    for (int k0 = 0; k0 < cnt; k0 += 8) {
-        float sx = 0.f, sy = 0.f, se = 0.f;
-        const int k1 = min(cnt, k0 + 8);
-        for (int k = k0; k < k1; k++) {
-            int j = __ldg(&nbr[(size_t)k * n + i]);
-            float fx, fy;
-            se += mixed_pair(ds->p, a, pk[j], e_c, n_c, fx, fy);
-            sx += fx;
-            sy += fy;
+    if constexpr (G == 1) {
+        for (int k0 = 0; k0 < cnt; k0 += 8) {
+            float sx = 0.f, sy = 0.f, se = 0.f;
+            const int k1 = min(cnt, k0 + 8);
+            for (int k = k0; k < k1; k++) {
+                int j = nbr[(size_t)k * n + i];
+                float fx, fy;
+                se += mixed_pair(p, a, pk[j], e_c, n_c, fx, fy);
+                sx += fx;
+                sy += fy;
+            }
+            ax += (double)sx;
+            ay += (double)sy;
+            en += (double)se;
         }
-        ax += (double)sx;
-        ay += (double)sy;
-        en += (double)se;
+    } else {
+        constexpr int R = 8 / G;
+        const int lane = threadIdx.x & 31, sub = lane & (G - 1), lead = lane - sub;
+        const int most = (int)__reduce_max_sync(0xffffffffu, (unsigned)cnt);
+        for (int k0 = 0; k0 < most; k0 += 8) {
+            float fx[R], fy[R], e[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const int k = k0 + r * G + sub;
+                fx[r] = 0.f; fy[r] = 0.f; e[r] = 0.f;
+                if (k < cnt) e[r] = mixed_pair(p, a, pk[nbr[(size_t)k * n + i]], e_c, n_c, fx[r], fy[r]);
+            }
+            float sx = 0.f, sy = 0.f, se = 0.f;
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                sx += __shfl_sync(0xffffffffu, fx[u / G], lead + u % G);
+                sy += __shfl_sync(0xffffffffu, fy[u / G], lead + u % G);
+                se += __shfl_sync(0xffffffffu, e[u / G], lead + u % G);
+            }
+            ax += (double)sx;
+            ay += (double)sy;
+            en += (double)se;
+        }
     }
 }
 
@@ -297,8 +322,9 @@ __device__ __forceinline__ void force_sum(const DevSys *ds, int i, bool valid, d
     ax = 0.0; ay = 0.0; en = 0.0;
     if constexpr (M) {
         if (!valid) return;
-        if (!R || !ds->s.fp64_now) disk_force_sum_mixed(ds, i, ax, ay, en);
-        else pair_sums_thread(pair_args(ds), i, min(ds->w.count[i], ds->p.cap), ax, ay, en);
+        const int cnt = min(ds->w.count[i], ds->p.cap);
+        if (!R || !ds->s.fp64_now) mixed_sums<1>(ds->p, ds->v.pk, ds->v.nbr, i, cnt, ax, ay, en);
+        else pair_sums_thread(pair_args(ds), i, cnt, ax, ay, en);
     } else {
         __shared__ ForceWarp w[kForceTPB / 32];
         const int cnt = valid ? min(ds->w.count[i], ds->p.cap) : 0;
@@ -801,10 +827,7 @@ __global__ void k_cell_scatter(DevSys *ds) {
 // Within each cell, restore ascending particle order: the result is the
 // permutation of a stable sort by cell (thrust::sort_by_key in
 // src/particles/base/particle.cu:1293).  Also clears the counters.
-__global__ void k_cell_sort(DevSys *ds) {
-    if (ds->s.rebuild != 2) return;
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ds->p.ncells) return;
+__device__ __forceinline__ void cell_sort_one(DevSys *ds, int c) {
     int b = ds->w.cell_start[c], e = ds->w.cell_start[c + 1];
     int *perm = ds->w.perm;
     for (int k = b + 1; k < e; k++) {
@@ -815,6 +838,12 @@ __global__ void k_cell_sort(DevSys *ds) {
     }
     ds->w.cell_cnt[c] = 0;
     ds->w.cell_cur[c] = 0;
+}
+
+__global__ void k_cell_sort(DevSys *ds) {
+    if (ds->s.rebuild != 2) return;
+    int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c < ds->p.ncells) cell_sort_one(ds, c);
 }
 
 // kernelReorderParticleData (src/particles/base/kernels.cu:508-543) into the
@@ -1036,6 +1065,32 @@ __global__ void k_nve_first(DevSys *ds, double dt_half, double dt) {
     }
 }
 
+// force and energy of particle i in an NVE step from its pair sums (ax, ay, en)
+// and its velocity u, overwriting
+__device__ __forceinline__ double2 nve_force(const DevSys *ds, int i, double2 u, double ax, double ay,
+                                             double en, double &pe) {
+    double2 f;
+    const double g = ds->s.damping;
+    pe = 0.0 + en;
+    if (ds->s.walls) {
+        // NVE::wall_step (src/integrator/nve.cu:33-35): zero, wall forces,
+        // then += the pair sum unless the particle has no neighbours
+        double wx, wy;
+        const double ew = wall_force(ds->p, ds->v.pos[i], ds->v.rad[i], wx, wy);
+        f = make_double2(0.0 + wx, 0.0 + wy);
+        pe = 0.0 + ew;
+        if (ds->w.count[i] != 0) { f.x += ax; f.y += ay; pe += en; }
+    } else if (g != 0.0) {
+        // DampedNVE::step (src/integrator/damped_nve.cu:22-23): F = 0 - g v,
+        // then += the pair sum unless the particle has no neighbours
+        f = make_double2(0.0 - g * u.x, 0.0 - g * u.y);
+        if (ds->w.count[i] != 0) { f.x += ax; f.y += ay; }
+    } else {
+        f = make_double2(0.0 + ax, 0.0 + ay);
+    }
+    return f;
+}
+
 // NVE::step second half (src/integrator/nve.cu:21-24): zero, forces, kick dt/2.
 template <int G, bool M>
 __global__ void k_nve_second(DevSys *ds, double dt_half) {
@@ -1047,27 +1102,10 @@ __global__ void k_nve_second(DevSys *ds, double dt_half) {
     if (i < ds->p.n && (gid & (G - 1)) == 0) {
         double2 *vel = ds->v.vel;
         double2 u = vel[i];
-        double2 f;
-        const double g = ds->s.damping;
-        double pe0 = 0.0;
-        if (ds->s.walls) {
-            // NVE::wall_step (src/integrator/nve.cu:33-35): zero, wall forces,
-            // then += the pair sum unless the particle has no neighbours
-            double wx, wy;
-            const double ew = wall_force(ds->p, ds->v.pos[i], ds->v.rad[i], wx, wy);
-            f = make_double2(0.0 + wx, 0.0 + wy);
-            pe0 = 0.0 + ew;
-            if (ds->w.count[i] != 0) { f.x += ax; f.y += ay; pe0 += en; }
-        } else if (g != 0.0) {
-            // DampedNVE::step (src/integrator/damped_nve.cu:22-23): F = 0 - g v,
-            // then += the pair sum unless the particle has no neighbours
-            f = make_double2(0.0 - g * u.x, 0.0 - g * u.y);
-            if (ds->w.count[i] != 0) { f.x += ax; f.y += ay; }
-        } else {
-            f = make_double2(0.0 + ax, 0.0 + ay);
-        }
+        double pe;
+        const double2 f = nve_force(ds, i, u, ax, ay, en, pe);
         ds->v.frc[i] = f;
-        ds->w.pe[i] = ds->s.walls ? pe0 : 0.0 + en;
+        ds->w.pe[i] = pe;
         double dtm = dt_half / ds->v.mass[i];
         u.x = u.x + f.x * dtm;
         u.y = u.y + f.y * dtm;
@@ -1082,8 +1120,7 @@ __global__ void k_nve_second(DevSys *ds, double dt_half) {
 
 // Fire::step prologue (src/integrator/fire.cu:13-34): decide dt / alpha from
 // the power of the state the next step starts from.
-__device__ void fire_decide(DevSys *ds, double power) {
-    DevState &s = ds->s;
+__device__ __forceinline__ void fire_decide(DevState &s, double power) {
     if (power > 0) {
         s.f_ngood++;
         s.f_nbad = 0;
@@ -1149,9 +1186,45 @@ __global__ void k_fire_move(DevSys *ds) {
     }
 }
 
-// FIRE force phase: forces (overwrite), kick dt/2, then on the last block the
+// End of a FIRE iteration, from its totals (PE, power, max|F|^2): the
 // minimizeFire convergence tests (src/routines/minimization.cu:96-106) and the
-// next step's Fire::step decision.  mode 0 = loop iteration, 1 = setup
+// next step's Fire::step decision.
+template <bool M>
+__device__ __forceinline__ void fire_epilogue(DevState &s, const double (&v)[3]) {
+    s.pe = v[0];
+    s.power = v[1];
+    s.fmax2 = v[2];
+    double avg = v[0] / s.dof;
+    // (no target: no test, and no FP64 division on the iteration's serial path)
+    const bool pe_still = s.pe_diff_target > 0 && fabs(avg / s.last_avg_pe - 1) < s.pe_diff_target;
+    s.last_avg_pe = avg;
+    long long it = s.iter;
+    // mixed form: FP32 pairs until max|F| reaches switch_fmax, FIRE keeps going
+    // uphill, or max|F| stops falling within 100x of switch_fmax (FP32 noise
+    // floor); FP64 pairs after, and only an FP64 state may pass the PE-change
+    // and max|F| tests
+    bool fp64 = true;
+    if (M && !s.fp64_now) {
+        if (v[2] < 0.81 * s.best_f2) { s.best_f2 = v[2]; s.best_it = it; }
+        const double fm = sqrt(v[2]);
+        if (fm <= s.switch_fmax || s.f_nbad > 5 || (fm < 100.0 * s.switch_fmax && it - s.best_it > 2000))
+            s.fp64_now = 1;
+        fp64 = false;
+    }
+    if ((fp64 && pe_still) || avg < s.pe_target) {
+        s.result_step = it; s.f_converged = 1; s.flags |= kDone; return;
+    }
+    if (fp64 && s.fmax_target > 0 && sqrt(v[2]) <= s.fmax_target) {
+        s.result_step = it; s.f_converged = 1; s.flags |= kDone; return;
+    }
+    if (it + 1 >= s.max_steps) { s.result_step = s.max_steps; s.flags |= kDone; return; }
+    s.iter = it + 1;
+    fire_decide(s, v[1]);
+    if (s.f_stopped) { s.result_step = it + 1; s.f_converged = 1; s.flags |= kDone; }
+}
+
+// FIRE force phase: forces (overwrite), kick dt/2, then on the last block
+// fire_epilogue.  mode 0 = loop iteration, 1 = setup
 // (forces only: minimizeFire's initial force call and last_avg_pe), 2 = a
 // single Fire::step (no convergence test, decision for the next step only).
 template <int G, bool M>
@@ -1181,42 +1254,18 @@ __global__ void k_fire_force(DevSys *ds, int mode) {
     const int ops[3] = {0, 0, 1};
     if (!grid_reduce<3>(v, ops, ds)) return;
     DevState &s = ds->s;
+    if (mode == 0) {
+        fire_epilogue<M>(s, v);
+        return;
+    }
     s.pe = v[0];
     s.power = v[1];
     s.fmax2 = v[2];
-    double avg = v[0] / s.dof;
     if (mode == 1) {
-        s.last_avg_pe = avg;
-        fire_decide(ds, v[1]);
+        s.last_avg_pe = v[0] / s.dof;
+        fire_decide(s, v[1]);
         if (s.f_stopped) { s.result_step = 0; s.flags |= kDone; }
-        return;
     }
-    if (mode == 2) return;
-    double diff = fabs(avg / s.last_avg_pe - 1);
-    s.last_avg_pe = avg;
-    long long it = s.iter;
-    // mixed form: FP32 pairs until max|F| reaches switch_fmax, FIRE keeps going
-    // uphill, or max|F| stops falling within 100x of switch_fmax (FP32 noise
-    // floor); FP64 pairs after, and only an FP64 state may pass the PE-change
-    // and max|F| tests
-    bool fp64 = true;
-    if (M && !s.fp64_now) {
-        if (v[2] < 0.81 * s.best_f2) { s.best_f2 = v[2]; s.best_it = it; }
-        const double fm = sqrt(v[2]);
-        if (fm <= s.switch_fmax || s.f_nbad > 5 || (fm < 100.0 * s.switch_fmax && it - s.best_it > 2000))
-            s.fp64_now = 1;
-        fp64 = false;
-    }
-    if ((fp64 && diff < s.pe_diff_target) || avg < s.pe_target) {
-        s.result_step = it; s.f_converged = 1; s.flags |= kDone; return;
-    }
-    if (fp64 && s.fmax_target > 0 && sqrt(v[2]) <= s.fmax_target) {
-        s.result_step = it; s.f_converged = 1; s.flags |= kDone; return;
-    }
-    if (it + 1 >= s.max_steps) { s.result_step = s.max_steps; s.flags |= kDone; return; }
-    s.iter = it + 1;
-    fire_decide(ds, v[1]);
-    if (s.f_stopped) { s.result_step = it + 1; s.f_converged = 1; s.flags |= kDone; }
 }
 
 // Fire::step prologue for a single step: P = F.v over the grid, then decide.
@@ -1231,7 +1280,7 @@ __global__ void k_fire_power_decide(DevSys *ds) {
     const int ops[1] = {0};
     if (grid_reduce<1>(v, ops, ds)) {
         ds->s.power = v[0];
-        fire_decide(ds, v[0]);
+        fire_decide(ds->s, v[0]);
     }
 }
 

@@ -6,9 +6,11 @@
 // the reference's Particle methods.  The loops (dpg_nve_steps,
 // dpg_fire_minimize, dpg_adam_minimize) run device-resident: the rebuild
 // decision, the FIRE dt/alpha logic and the convergence tests are made on
-// the GPU, and the loop body is a CUDA graph whose neighbour rebuild sits
-// under a conditional (IF) node inside a WHILE node, so a whole minimisation is
-// one graph launch with no host round trips.
+// the GPU.  Up to kLoopMaxN particles a loop is one cooperative launch
+// (disk_loop.cuh); above, the loop body is a CUDA graph whose neighbour rebuild
+// sits under a conditional (IF) node inside a WHILE node.  Either way a whole
+// minimisation runs without host round trips.  DPG_LOOP_MODE=cond keeps the
+// graph at every size, graph and stream the chunked forms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -22,6 +24,7 @@
 
 #include "../../include/dpg.h"
 #include "disk_kernels.cuh"
+#include "disk_loop.cuh"
 #include "host_common.h"
 
 using namespace dpg;
@@ -61,7 +64,7 @@ extern "C" int dpg_version(void) { return 1; }
 // the system object
 // ---------------------------------------------------------------------------
 enum LoopKind { kLoopFire = 0, kLoopNve = 1, kLoopCount = 2 };
-enum LoopMode { kModeStream = 0, kModeGraph = 1, kModeCond = 2 };
+enum LoopMode { kModeStream = 0, kModeGraph = 1, kModeCond = 2, kModeResident = 3 };
 
 struct dpg_system {
     int n = 0;
@@ -83,6 +86,13 @@ struct dpg_system {
     double *xfer = nullptr;  // staging for static-order transfers (2 n doubles)
     // loops
     int mode = kModeCond;
+    // resident grid (kModeResident): barrier state; lanes per particle, threads,
+    // blocks, particles per block and shared memory of its two kernels
+    LoopSync *lsync = nullptr;
+    struct Plan {
+        int lanes = 1, threads = 0, blocks = 0, chunk = 0;
+        size_t smem = 0;
+    } tile, loop;
     cudaGraphExec_t loop_exec[kLoopCount] = {nullptr, nullptr};
     cudaGraphConditionalHandle h_loop[kLoopCount] = {0, 0}, h_rb[kLoopCount] = {0, 0};
     cudaGraphExec_t chunk_exec[kLoopCount] = {nullptr, nullptr};
@@ -138,6 +148,11 @@ struct dpg_system {
         }
     }
 };
+
+// The loops run as one resident grid up to kLoopMaxN particles, as a graph of
+// full-size kernels above (see plan_resident).
+constexpr int kLoopMaxN = 1 << 17;
+constexpr int kLoopBlocksPerSM = 2;
 
 static int dalloc(dpg_system *s, void **p, size_t bytes) {
     CK(cudaMalloc(p, bytes > 0 ? bytes : 16));
@@ -250,6 +265,7 @@ extern "C" int dpg_create(const dpg_params *p, void *cuda_stream, dpg_handle *ou
     const char *m = getenv("DPG_LOOP_MODE");
     if (m && !strcmp(m, "stream")) s->mode = kModeStream;
     else if (m && !strcmp(m, "graph")) s->mode = kModeGraph;
+    else if (!(m && !strcmp(m, "cond")) && s->n <= kLoopMaxN) s->mode = kModeResident;
     const size_t n = s->n;
     int dev = 0, nsm = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -286,6 +302,9 @@ extern "C" int dpg_create(const dpg_params *p, void *cuda_stream, dpg_handle *ou
     A((void **)&v.m1, n * 16); A((void **)&v.m2, n * 16); A((void **)&v.m1_t, n * 16); A((void **)&v.m2_t, n * 16);
     if (s->mixed) A((void **)&v.pk, n * 16);
     A((void **)&v.q, n * 16);
+    A((void **)&v.q_t, n * 16);
+    if (s->mixed) A((void **)&v.pk_t, n * 16);
+    A((void **)&s->lsync, sizeof(LoopSync));
     A((void **)&w.pos_n, n * 16); A((void **)&w.pos_c, n * 16); A((void **)&w.pe, n * 8);
     A((void **)&w.count, n * 4); A((void **)&w.cell_raw, n * 4); A((void **)&w.cell_of, n * 4);
     A((void **)&w.perm, n * 4);
@@ -293,6 +312,7 @@ extern "C" int dpg_create(const dpg_params *p, void *cuda_stream, dpg_handle *ou
     const int fg8 = std::max(1, (int)(((long long)s->n * 8 + s->ftpb - 1) / s->ftpb));
     w.max_blocks = std::max(std::max(s->grid(s->n), s->grid_full(s->n)), std::max(s->fgrid(), fg8));
     w.max_blocks = std::max(std::max(w.max_blocks, s->ngrid()), (s->n + kStressTPB - 1) / kStressTPB);
+    w.max_blocks = std::max(w.max_blocks, kLoopBlocksPerSM * nsm);
     A((void **)&w.partials, (size_t)w.max_blocks * 8 * 8);
     A((void **)&w.s_pos, n * 16); A((void **)&w.s_vel, n * 16); A((void **)&w.s_frc, n * 16);
     A((void **)&w.s_rad, n * 8); A((void **)&w.s_mass, n * 8); A((void **)&w.s_sidx, n * 4);
@@ -478,12 +498,6 @@ extern "C" int dpg_get_box(dpg_handle s, double *bx, double *by) {
 // ---------------------------------------------------------------------------
 static double max_diameter(const dpg_system *s) {
     return 2.0 * *std::max_element(s->h_rad.begin(), s->h_rad.end());
-}
-
-static double particle_area(const dpg_system *s) {
-    double a = 0.0;
-    for (double r : s->h_rad) a += r * r;
-    return a * 3.141592653589793238462643383279502884197;
 }
 
 // Disk::getParticleArea (src/particles/disk/disk.cu:205-207) sums r^2 over the
@@ -1067,6 +1081,93 @@ static int build_cond_graph(dpg_system *s, int kind) {
     return DPG_OK;
 }
 
+// ---- the resident grid ------------------------------------------------------
+template <int KIND>
+static void *tile_fn(const dpg_system *s) {
+    if (s->mixed) return s->tile.lanes == 8 ? (void *)k_tile<KIND, 8, true> : (void *)k_tile<KIND, 4, true>;
+    return s->tile.lanes == 8 ? (void *)k_tile<KIND, 8, false> : (void *)k_tile<KIND, 4, false>;
+}
+template <int KIND>
+static void *loop_fn(const dpg_system *s) {
+    if (s->mixed) return s->loop.lanes == 8 ? (void *)k_loop<KIND, 8, true> : (void *)k_loop<KIND, 1, true>;
+    switch (s->loop.lanes) {
+        case 8: return (void *)k_loop<KIND, 8, false>;
+        case 2: return (void *)k_loop<KIND, 2, false>;
+        default: return (void *)k_loop<KIND, 1, false>;
+    }
+}
+
+// Two resident kernels.  k_tile holds a block's particles in registers: up to
+// kTileP of them on each SM, rows of at most kTileSlots neighbours.  k_loop
+// walks any number of tiles through memory.  Few particles leave most of the
+// FP64 pipes idle unless they are spread over every SM, so both take a block an
+// SM and as few warps as cover its particles (k_loop a second block an SM where
+// it fits).  Lanes per neighbour row: as many as kLoopMaxTPB threads allow.
+static int plan_resident(dpg_system *s) {
+    int dev = 0, nsm = 0, coop = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    if (!coop) return set_err(DPG_ERR_CUDA, "no cooperative launch");
+    const long long n = s->n, per = (n + nsm - 1) / nsm;  // particles an SM
+    auto warps = [](long long threads) { return (int)std::max<long long>(32, (threads + 31) / 32 * 32); };
+    if (per <= kTileP) {
+        dpg_system::Plan &q = s->tile;
+        // at least 4 particles a block: with fewer, more blocks only make the barriers longer
+        q.chunk = (int)std::max<long long>(per, 4);
+        q.lanes = q.chunk * 8 <= kLoopMaxTPB ? 8 : 4;
+        q.threads = warps((long long)q.chunk * q.lanes);
+        q.blocks = (int)((n + q.chunk - 1) / q.chunk);
+        q.smem = tile_bytes(q.chunk);
+        for (void *fn : {tile_fn<kLoopFire>(s), tile_fn<kLoopNve>(s)}) {
+            int occ = 0;
+            // the attribute is the function's, whichever system launches it: the largest block's
+            CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_bytes(kTileP)));
+            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, q.threads, q.smem));
+            if (occ < 1) return set_err(DPG_ERR_CUDA, "the resident loop does not fit an SM");
+        }
+    }
+    dpg_system::Plan &q = s->loop;
+    if (s->mixed) q.lanes = per * 8 <= kLoopMaxTPB ? 8 : 1;
+    else q.lanes = per * 8 <= kLoopMaxTPB ? 8 : (per * 2 <= kLoopMaxTPB ? 2 : 1);
+    q.threads = std::min(kLoopMaxTPB, warps(per * q.lanes));
+    q.smem = sizeof(ForceWarp) * (q.threads / 32);
+    int per_sm = kLoopBlocksPerSM;
+    for (void *fn : {loop_fn<kLoopFire>(s), loop_fn<kLoopNve>(s)}) {
+        int occ = 0;
+        CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(sizeof(ForceWarp) * (kLoopMaxTPB / 32))));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, q.threads, q.smem));
+        per_sm = std::min(per_sm, occ);
+    }
+    if (per_sm < 1) return set_err(DPG_ERR_CUDA, "the resident loop does not fit an SM");
+    const int tile = q.threads / q.lanes;
+    const long long blocks = std::min<long long>((long long)per_sm * nsm, (n + tile - 1) / tile);
+    q.chunk = (int)((n + blocks - 1) / blocks);
+    q.blocks = (int)((n + q.chunk - 1) / q.chunk);
+    return DPG_OK;
+}
+
+// Launches of the resident loop until a flag is raised, each of at most `most`
+// iterations (a fraction of a second).
+static int run_resident(dpg_system *s, int kind) {
+    const bool tile = s->tile.blocks > 0 && s->cap <= kTileSlots;
+    const dpg_system::Plan &q = tile ? s->tile : s->loop;
+    void *fn = tile ? (kind == kLoopFire ? tile_fn<kLoopFire>(s) : tile_fn<kLoopNve>(s))
+                    : (kind == kLoopFire ? loop_fn<kLoopFire>(s) : loop_fn<kLoopNve>(s));
+    long long most = std::max<long long>(256, (1LL << 26) / (s->n + 1024));
+    double dt = s->chunk_dt;
+    int chunk = q.chunk;
+    void *args[] = {(void *)&s->d, (void *)&s->lsync, (void *)&dt, (void *)&chunk, (void *)&most};
+    do {
+        CK(cudaMemsetAsync(s->lsync, 0, sizeof(LoopSync), s->stream));
+        CK(cudaLaunchCooperativeKernel(fn, dim3(q.blocks), dim3(q.threads), args, q.smem, s->stream));
+        TRY(pull_state(s));
+        if (s->hs->flags & kError) return set_err(DPG_ERR_TIMEOUT, "a grid barrier of the resident loop ran out");
+    } while (!s->hs->flags);
+    return DPG_OK;
+}
+
 // Run iterations until the device says done (or halts on overflow).
 // Returns after a host-visible stop; *halted_overflow tells the caller to
 // finish the interrupted iteration.
@@ -1075,6 +1176,17 @@ static int run_loop(dpg_system *s, int kind, int *halted_overflow) {
     TRY(mixed_refresh(s));
     if (s->mixed) s->q_fresh = false;
     else TRY(quant_refresh(s));
+    if (s->mode == kModeResident) {
+        const int rc = s->loop.blocks ? DPG_OK : plan_resident(s);
+        if (rc != DPG_OK) {
+            (void)cudaGetLastError();
+            s->mode = kModeCond;
+        } else {
+            TRY(run_resident(s, kind));
+            if (s->hs->flags & kOverflow) *halted_overflow = 1;
+            return DPG_OK;
+        }
+    }
     if (s->mode == kModeCond) {
         int rc = build_cond_graph(s, kind);
         if (rc != DPG_OK) {
