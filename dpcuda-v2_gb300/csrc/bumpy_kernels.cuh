@@ -33,6 +33,8 @@ struct BumpyExt {
     int *o2n;                // old -> new body slot during a re-sort
     int *vnbr, *vcount;      // vertex neighbour list, column-major [capv][nv]
     float4 *vpk;             // mixed form: packed FP32 vertex offsets (see mixed_pack)
+    uint4 *vq;               // fixed-point vertex positions (see Quant in dpg_device.cuh)
+    float vin2, vout2, vpin2, vpout2;  // filter limits of the two vertex-list cutoffs
     int mixed;               // 1: FP32 vertex pairs (the body DevParams stay FP64)
     long long vlist_built;   // n_rebuilds value at the last vertex-list build
     double tmax2, power_rot;
@@ -55,6 +57,7 @@ struct BumpySys {
 };
 
 constexpr int kWarpsPerBlock = kTPB / 32;
+constexpr int kMoveBodies = 32;  // bodies per block of the move kernels
 
 // calcTorque: include/particles/base/kernels.cuh:237-241
 __device__ __forceinline__ double torque_of(double fx, double fy, double px, double py, double cx,
@@ -83,119 +86,155 @@ __global__ void kb_kick(BumpySys *bs, double dt) {
     body_kick(bs, b, dt);
 }
 
+// what the loops' move kernels keep current with a vertex position (see moved_update)
+__device__ __forceinline__ void vertex_moved(BumpySys *bs, int v, double2 q) {
+    BumpyExt &x = bs->x;
+    if (x.mixed) x.vpk[v] = mixed_pack(bs->b.p, q, x.rv);
+    if (!x.mixed || bs->b.s.fp64_now) x.vq[v] = quant_of(bs->b.p, q, x.rv);
+}
+
 // ---- body + vertex move: kernelUpdateRigidPositions + kernelTranslateAndRotateVertices1
-// (kernels.cu:21-78,152-201), one warp per body.  Returns the squared
-// displacements from the neighbour / cell reference positions (lane 0).
-__device__ __forceinline__ void body_move(BumpySys *bs, int b, int lane, double dt, double &nd2,
-                                          double &cd2) {
+// (kernels.cu:21-78,152-201) of the bodies [b0, b1) by a block.  The body part
+// (kick, displacement, cosine and sine of the increment: some 130 FP64
+// instructions, each of which holds an FP64 pipe for all 32 lanes whatever
+// their number) runs on one thread a body; a warp a body spent them once per
+// body.  The vertices then turn with one thread each.  kMoveBodies bodies at a
+// time; every thread of the block calls it.
+struct MoveMem {
+    double2 p[kMoveBodies], n[kMoveBodies], cs[kMoveBodies];
+};
+// pre(b): what a body does before it moves (thread of the body)
+template <class F>
+__device__ __forceinline__ void bodies_move(BumpySys *bs, int b0, int b1, double dt, MoveMem &m, F pre,
+                                            double &nd2, double &cd2) {
     DevSys &d = bs->b;
     BumpyExt &x = bs->x;
-    double2 p = d.v.pos[b], u = d.v.vel[b];
-    double ang = x.th[b], w = x.w[b];
-    double ddx = u.x * dt, ddy = u.y * dt, dth = w * dt;
-    double nx = p.x + ddx, ny = p.y + ddy;
-    __syncwarp();
-    if (lane == 0) {
-        d.v.pos[b] = make_double2(nx, ny);
-        x.th[b] = ang + dth;
-        x.adelta[b] = dth;
-        double2 a = d.w.pos_n[b], c = d.w.pos_c[b];
-        double a1 = nx - a.x, a2 = ny - a.y, c1 = nx - c.x, c2 = ny - c.y;
-        nd2 = a1 * a1 + a2 * a2;
-        cd2 = c1 * c1 + c2 * c2;
-    }
-    double ca = cos(dth), sa = sin(dth);
-    const int f = x.start[b], nvb = x.nvb[b];
-    for (int k = lane; k < nvb; k += 32) {
-        double2 q = x.vpos[f + k];
-        double rx = q.x - p.x, ry = q.y - p.y;
-        double rxr = rx * ca - ry * sa, ryr = rx * sa + ry * ca;
-        double2 nq = make_double2(nx + rxr, ny + ryr);
-        x.vpos[f + k] = nq;
-        if (x.mixed) x.vpk[f + k] = mixed_pack(d.p, nq, x.rv);
+    for (int base = b0; base < b1; base += kMoveBodies) {
+        const int nbod = min(kMoveBodies, b1 - base);
+        if (threadIdx.x < nbod) {
+            const int b = base + threadIdx.x;
+            pre(b);
+            const double2 p = d.v.pos[b], u = d.v.vel[b];
+            const double ang = x.th[b], w = x.w[b];
+            const double ddx = u.x * dt, ddy = u.y * dt, dth = w * dt;
+            const double nx = p.x + ddx, ny = p.y + ddy;
+            d.v.pos[b] = make_double2(nx, ny);
+            x.th[b] = ang + dth;
+            x.adelta[b] = dth;
+            const double2 a = d.w.pos_n[b], c = d.w.pos_c[b];
+            const double a1 = nx - a.x, a2 = ny - a.y, c1 = nx - c.x, c2 = ny - c.y;
+            nd2 = fmax(nd2, a1 * a1 + a2 * a2);
+            cd2 = fmax(cd2, c1 * c1 + c2 * c2);
+            m.p[threadIdx.x] = p;
+            m.n[threadIdx.x] = make_double2(nx, ny);
+            m.cs[threadIdx.x] = make_double2(cos(dth), sin(dth));
+        }
+        __syncthreads();
+        const int v0 = x.start[base], last = base + nbod - 1, v1 = x.start[last] + x.nvb[last];
+        for (int v = v0 + threadIdx.x; v < v1; v += blockDim.x) {
+            const int k = x.vbody[v] - base;
+            const double2 q = x.vpos[v], p = m.p[k], n = m.n[k], cs = m.cs[k];
+            const double rx = q.x - p.x, ry = q.y - p.y;
+            const double rxr = rx * cs.x - ry * cs.y, ryr = rx * cs.y + ry * cs.x;
+            const double2 nq = make_double2(n.x + rxr, n.y + ryr);
+            x.vpos[v] = nq;
+            vertex_moved(bs, v, nq);
+        }
+        __syncthreads();
     }
 }
 
 __global__ void kb_drift(BumpySys *bs, double dt) {
-    const int lane = threadIdx.x & 31;
-    const int b = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+    __shared__ MoveMem m;
+    const int b0 = blockIdx.x * kMoveBodies, b1 = min(b0 + kMoveBodies, bs->b.p.n);
     double v[2] = {0.0, 0.0};
-    if (b < bs->b.p.n) body_move(bs, b, lane, dt, v[0], v[1]);
+    bodies_move(bs, b0, b1, dt, m, [](int) {}, v[0], v[1]);
     const int ops[2] = {1, 1};
     if (grid_reduce<2>(v, ops, &bs->b)) { bs->b.s.max_nd2 = v[0]; bs->b.s.max_cd2 = v[1]; }
 }
 
 // ---- forces: kernelCalcRigidBumpyForces1 + kernelCalcRigidBumpyParticleForces1
-// (kernels.cu:366-442) fused, one warp per body.  Outputs the body sums (every
-// lane holds the same values).  walls: kernelCalcRigidBumpyWallForces
-// (kernels.cu:348-362) first, as NVE::wall_step calls it before the pairs, so
-// a vertex carries (0 + wall) + pair sum.
-__device__ __forceinline__ void body_forces(const BumpySys *__restrict__ bs, int b, int lane,
-                                            bool walls, double &bfx, double &bfy, double &btq,
-                                            double &bpe) {
+// (kernels.cu:366-442) fused, one warp per body.  The vertex pairs run through
+// the filter and the warp's queue (pair_sums); the body's force, torque and
+// energy are then added over its vertices in vertex order by four lanes, one
+// sum each, skipping the vertices without a term (+0.0 leaves such a sum as it
+// is).  Lanes 0 - 3 return the force x, force y, torque and energy of the body.
+// walls: kernelCalcRigidBumpyWallForces (kernels.cu:348-362) first, as
+// NVE::wall_step calls it before the pairs, so a vertex carries (0 + wall) +
+// pair sum.
+__device__ __forceinline__ PairArgs vertex_args(const BumpySys *bs) {
+    PairArgs f = pair_args(&bs->b);
+    f.pos = bs->x.vpos;
+    f.rad = nullptr;
+    f.rv = bs->x.rv;
+    f.nbr = bs->x.vnbr;
+    f.q = bs->x.vq;
+    f.n = bs->x.nv;
+    return f;
+}
+
+__device__ __forceinline__ double body_forces(const BumpySys *bs, int b, bool walls, ForceWarp &fw) {
     const DevSys &d = bs->b;
     const BumpyExt &x = bs->x;
-    const int nv = x.nv, capv = x.capv;
-    const double bx = d.p.box[0], by = d.p.box[1], e_c = d.p.e_c, n_c = d.p.n_c, rv = x.rv;
+    const int lane = threadIdx.x & 31, capv = x.capv;
+    const double rv = x.rv;
     const double2 c = d.v.pos[b];
     const int f = x.start[b], nvb = x.nvb[b];
     const bool mixed = x.mixed && !d.s.fp64_now;
-    bfx = 0.0; bfy = 0.0; btq = 0.0; bpe = 0.0;
+    const PairArgs fa = vertex_args(bs);
+    double sum = 0.0;
     for (int base = 0; base < nvb; base += 32) {
-        int k = base + lane;
-        double vfx = 0.0, vfy = 0.0, vtq = 0.0, vpe = 0.0;
-        if (k < nvb) {
-            int v = f + k;
-            double2 q = x.vpos[v];
-            int cnt = min(x.vcount[v], capv);
-            double ax = 0.0, ay = 0.0, en = 0.0;
-            if (mixed) {  // FP32 vertex pairs; torque and body sums stay FP64
+        const int k = base + lane, v = f + k;
+        const bool real = k < nvb;
+        const int cnt = real ? min(x.vcount[v], capv) : 0;
+        double t[3] = {0.0, 0.0, 0.0};  // pair sums: force x, force y, energy
+        if (mixed) {                    // FP32 vertex pairs; torque and body sums stay FP64
+            if (real) {
                 const float4 a = x.vpk[v];
+                const float e_c = (float)d.p.e_c, n_c = (float)d.p.n_c;
                 float sx = 0.f, sy = 0.f, se = 0.f;
-                for (int t = 0; t < cnt; t++) {
-                    int u = __ldg(&x.vnbr[(size_t)t * nv + v]);
+                for (int q = 0; q < cnt; q++) {
                     float fx, fy;
-                    se += mixed_pair(d.p, a, x.vpk[u], (float)e_c, (float)n_c, fx, fy);
+                    se += mixed_pair(d.p, a, x.vpk[x.vnbr[(size_t)q * fa.n + v]], e_c, n_c, fx, fy);
                     sx += fx;
                     sy += fy;
                 }
-                ax = (double)sx;
-                ay = (double)sy;
-                en = (double)se;
-            } else {
-                for (int t = 0; t < cnt; t++) {
-                    int u = __ldg(&x.vnbr[(size_t)t * nv + v]);
-                    double2 o = x.vpos[u];
-                    double fx, fy;
-                    double e = disk_pair(q.x, q.y, rv, o.x, o.y, rv, bx, by, e_c, n_c, fx, fy);
-                    ax += fx;
-                    ay += fy;
-                    en += e;
-                }
+                t[0] = (double)sx;
+                t[1] = (double)sy;
+                t[2] = (double)se;
             }
-            if (walls) {
-                double wx, wy;
-                const double we = wall_force(d.p, q, rv, wx, wy);
-                vfx = 0.0 + wx;
-                vfy = 0.0 + wy;
-                vtq = 0.0 + torque_of(wx, wy, q.x, q.y, c.x, c.y);
-                vpe = 0.0 + we;
-            }
-            if (cnt > 0) {
-                vfx = vfx + ax;
-                vfy = vfy + ay;
-                vtq = vtq + torque_of(ax, ay, q.x, q.y, c.x, c.y);
-                vpe = vpe + en;
-            }
+        } else {
+            pair_sums<1, 3>(fa, real ? v : f, cnt, fw, t);
         }
-        int lim = min(32, nvb - base);
-        for (int l = 0; l < lim; l++) {
-            bfx += __shfl_sync(0xffffffffu, vfx, l);
-            bfy += __shfl_sync(0xffffffffu, vfy, l);
-            btq += __shfl_sync(0xffffffffu, vtq, l);
-            bpe += __shfl_sync(0xffffffffu, vpe, l);
+        double vf[4] = {0.0, 0.0, 0.0, 0.0};  // the vertex: force x, force y, torque, energy
+        bool some = t[0] != 0.0 || t[1] != 0.0 || t[2] != 0.0;
+        const double2 q = x.vpos[real ? v : f];
+        if (walls && real) {
+            double wx, wy;
+            const double we = wall_force(d.p, q, rv, wx, wy);
+            vf[0] = 0.0 + wx;
+            vf[1] = 0.0 + wy;
+            vf[2] = 0.0 + torque_of(wx, wy, q.x, q.y, c.x, c.y);
+            vf[3] = 0.0 + we;
+            some = true;
         }
+        if (some) {
+            vf[0] = vf[0] + t[0];
+            vf[1] = vf[1] + t[1];
+            vf[2] = vf[2] + torque_of(t[0], t[1], q.x, q.y, c.x, c.y);
+            vf[3] = vf[3] + t[2];
+        }
+        __syncwarp();
+        // the queue's result rows hold the four terms of 32 vertices
+#pragma unroll
+        for (int e = 0; e < 4; e++) fw.r[0][e * 32 + lane] = vf[e];
+        __syncwarp();
+        unsigned todo = __ballot_sync(0xffffffffu, some);
+        if (lane < 4)
+            for (; todo; todo &= todo - 1) sum += fw.r[0][lane * 32 + __ffs(todo) - 1];
+        __syncwarp();
     }
+    return sum;
 }
 
 // mixed form: packed offsets of every vertex from the current vertex positions
@@ -205,22 +244,34 @@ __global__ void kb_mixed_refresh(BumpySys *bs) {
     bs->x.vpk[v] = mixed_pack(bs->b.p, bs->x.vpos[v], bs->x.rv);
 }
 
+// fixed-point positions of every vertex
+__global__ void kb_vquant(BumpySys *bs) {
+    int v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= bs->x.nv) return;
+    bs->x.vq[v] = quant_of(bs->b.p, bs->x.vpos[v], bs->x.rv);
+}
+
+// the same ahead of a vertex-list build, for the systems whose move kernels do
+// not keep them
+__global__ void kb_vquant_rebuild(BumpySys *bs) {
+    if (bs->b.s.n_rebuilds == bs->x.vlist_built) return;
+    int v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= bs->x.nv) return;
+    bs->x.vq[v] = quant_of(bs->b.p, bs->x.vpos[v], bs->x.rv);
+}
+
 // drop-in calculateForces (+= into the body arrays); walls = 1: calculateWallForces
 // then calculateForces
 __global__ void kb_force_acc(BumpySys *bs, int walls) {
-    const int lane = threadIdx.x & 31;
-    const int b = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+    __shared__ ForceWarp fw[kWarpsPerBlock];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int b = blockIdx.x * kWarpsPerBlock + wid;
     if (b >= bs->b.p.n) return;
-    double fx, fy, tq, pe;
-    body_forces(bs, b, lane, walls != 0, fx, fy, tq, pe);
-    if (lane == 0) {
-        double2 f = bs->b.v.frc[b];
-        f.x += fx;
-        f.y += fy;
-        bs->b.v.frc[b] = f;
-        bs->x.tq[b] += tq;
-        bs->b.w.pe[b] += pe;
-    }
+    const double sum = body_forces(bs, b, walls != 0, fw[wid]);
+    if (lane == 0) bs->b.v.frc[b].x += sum;
+    if (lane == 1) bs->b.v.frc[b].y += sum;
+    if (lane == 2) bs->x.tq[b] += sum;
+    if (lane == 3) bs->b.w.pe[b] += sum;
 }
 
 // zeroForceAndPotentialEnergy (rigid_bumpy.cu:1378-1381); vertex arrays are not kept
@@ -284,48 +335,63 @@ __global__ void kb_observables(BumpySys *bs) {
     }
 }
 
-// ---- vertex neighbour list: kernelUpdateVertexNeighborList (kernels.cu:870-922),
-// warp per body so the walk over the body's neighbour bodies is uniform.
-// Runs only when the body list was rebuilt since the last vertex build.
-__global__ void kb_vlist(BumpySys *bs) {
-    if (bs->b.s.n_rebuilds == bs->x.vlist_built) return;
-    const int lane = threadIdx.x & 31;
-    const int b = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+// ---- vertex neighbour list: kernelUpdateVertexNeighborList (kernels.cu:870-922):
+// vertices within the vertex cutoff, over the body's neighbour bodies (those
+// whose centre is within the body cutoff of the vertex) in list order, vertices
+// ascending.  G lanes per vertex: they share first the bodies, then each
+// body's vertices (16 consecutive bytes a lane), ballots give the hits their
+// places.  The fixed-point filter decides all but ~1e-5 of the tests; in FP64
+// the list of 4096 bodies took up to 940 us.  Returns the row's length.  All
+// lanes of the warp call it (real = false past the last vertex).
+template <int G>
+__device__ __forceinline__ int vlist_row(BumpySys *bs, int v, bool real) {
+    constexpr unsigned kAll = 0xffffffffu, kGroup = (1u << G) - 1u;
     const DevSys &d = bs->b;
     BumpyExt &x = bs->x;
-    int mxc = 0;
-    if (b < d.p.n) {
-        const int nb = d.p.n, nv = x.nv, capv = x.capv;
-        const double bx = d.p.box[0], by = d.p.box[1], c2 = x.vcut2, pc2 = x.vpcut2;
-        const int f = x.start[b], nvb = x.nvb[b];
-        const int ncnt = min(d.w.count[b], d.p.cap);
-        for (int base = 0; base < nvb; base += 32) {
-            int k = base + lane;
-            if (k >= nvb) break;
-            int v = f + k;
-            double2 q = x.vpos[v];
-            int cnt = 0;
-            for (int t = 0; t < ncnt; t++) {
-                int ob = d.v.nbr[(size_t)t * nb + b];
-                double2 oc = d.v.pos[ob];
-                double ex = pbc_dist(q.x, oc.x, bx), ey = pbc_dist(q.y, oc.y, by);
-                if (!(ex * ex + ey * ey < pc2)) continue;
-                int of = x.start[ob], on = x.nvb[ob];
-                for (int u = of; u < of + on; u++) {
-                    double2 o = x.vpos[u];
-                    double gx = pbc_dist(q.x, o.x, bx), gy = pbc_dist(q.y, o.y, by);
-                    if (gx * gx + gy * gy < c2) {
-                        if (cnt < capv) x.vnbr[(size_t)cnt * nv + v] = u;
-                        cnt++;
-                    }
-                }
+    const int lane = threadIdx.x & 31, sub = lane & (G - 1), lead = lane - sub;
+    const int nb = d.p.n, nv = x.nv, capv = x.capv;
+    const int b = real ? x.vbody[v] : 0, vv = real ? v : 0;
+    const int ncnt = real ? min(d.w.count[b], d.p.cap) : 0;
+    const uint4 qv = x.vq[vv];
+    int cnt = 0;
+    for (int t0 = 0; __any_sync(kAll, t0 < ncnt); t0 += G) {
+        const int t = t0 + sub;
+        const int ob = t < ncnt ? d.v.nbr[(size_t)t * nb + b] : 0;
+        const bool near = t < ncnt && within(d.p, x.vpos, vv, d.v.pos, ob, qv, d.v.q[ob], x.vpin2, x.vpout2, x.vpcut2);
+        unsigned bodies = (__ballot_sync(kAll, near) >> lead) & kGroup;
+        const int of_l = near ? x.start[ob] : 0, on_l = near ? x.nvb[ob] : 0;
+        while (__any_sync(kAll, bodies != 0)) {
+            const int src = bodies ? __ffs(bodies) - 1 : 0;
+            const int of = __shfl_sync(kAll, of_l, lead + src);
+            const int on_s = __shfl_sync(kAll, on_l, lead + src), on = bodies ? on_s : 0;
+            bodies &= bodies - 1;
+            for (int u0 = 0; __any_sync(kAll, u0 < on); u0 += G) {
+                const int u = of + u0 + sub;
+                const bool hit = u0 + sub < on &&
+                                 within(d.p, x.vpos, vv, x.vpos, u, qv, x.vq[u], x.vin2, x.vout2, x.vcut2);
+                const unsigned m = (__ballot_sync(kAll, hit) >> lead) & kGroup;
+                const int at = cnt + __popc(m & ((1u << sub) - 1u));
+                if (hit && at < capv) x.vnbr[(size_t)at * nv + v] = u;
+                cnt += __popc(m);
             }
-            x.vcount[v] = cnt;
-            mxc = max(mxc, cnt);
-            if (x.mixed) x.vpk[v] = mixed_pack(d.p, q, x.rv);
         }
     }
-    double val[1] = {(double)mxc};
+    return cnt;
+}
+
+// Runs only when the body list was rebuilt since the last vertex build.
+constexpr int kVlistLanes = 8;
+__global__ void kb_vlist(BumpySys *bs) {
+    if (bs->b.s.n_rebuilds == bs->x.vlist_built) return;
+    BumpyExt &x = bs->x;
+    const int gid = blockIdx.x * blockDim.x + threadIdx.x, v = gid / kVlistLanes;
+    const bool real = v < x.nv;
+    const int cnt = vlist_row<kVlistLanes>(bs, v, real);
+    if (real && gid % kVlistLanes == 0) {
+        x.vcount[v] = cnt;
+        if (x.mixed) x.vpk[v] = mixed_pack(bs->b.p, x.vpos[v], x.rv);
+    }
+    double val[1] = {real ? (double)cnt : 0.0};
     const int ops[1] = {1};
     if (grid_reduce<1>(val, ops, &bs->b)) {
         int m = (int)val[0];
@@ -451,14 +517,10 @@ __global__ void kb_reorder_vertices(BumpySys *bs) {
 // NVE::step first half with the rigid overrides: kick dt/2, move dt
 __global__ void kb_nve_first(BumpySys *bs, double dt_half, double dt) {
     if (halted(&bs->b)) return;
-    const int lane = threadIdx.x & 31;
-    const int b = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+    __shared__ MoveMem m;
+    const int b0 = blockIdx.x * kMoveBodies, b1 = min(b0 + kMoveBodies, bs->b.p.n);
     double v[2] = {0.0, 0.0};
-    if (b < bs->b.p.n) {
-        if (lane == 0) body_kick(bs, b, dt_half);
-        __syncwarp();
-        body_move(bs, b, lane, dt, v[0], v[1]);
-    }
+    bodies_move(bs, b0, b1, dt, m, [&](int b) { body_kick(bs, b, dt_half); }, v[0], v[1]);
     const int ops[2] = {1, 1};
     if (grid_reduce<2>(v, ops, &bs->b)) {
         DevSys *ds = &bs->b;
@@ -470,64 +532,80 @@ __global__ void kb_nve_first(BumpySys *bs, double dt_half, double dt) {
     }
 }
 
+// a body's new force, torque and energy (overwriting) from its sums, and the
+// kick dt/2 that follows in an NVE step
+__device__ __forceinline__ void body_nve_second(BumpySys *bs, int b, double fx, double fy, double tq,
+                                                double pe, double dt_half) {
+    const double g = bs->b.s.damping;
+    if (g != 0.0) {
+        // DampedNVE::step (src/integrator/damped_nve.cu:22-23) with
+        // kernelCalculateRigidDampedForces (kernels.cu:80-87): body
+        // F = 0 - g v, tau = 0 - g omega, then += the vertex sums
+        const double2 u = bs->b.v.vel[b];
+        const double w = bs->x.w[b];
+        bs->b.v.frc[b] = make_double2((0.0 - g * u.x) + fx, (0.0 - g * u.y) + fy);
+        bs->x.tq[b] = (0.0 - g * w) + tq;
+    } else {
+        bs->b.v.frc[b] = make_double2(0.0 + fx, 0.0 + fy);
+        bs->x.tq[b] = 0.0 + tq;
+    }
+    bs->b.w.pe[b] = 0.0 + pe;
+    body_kick(bs, b, dt_half);
+}
+
+// The sums of the bodies [b0, b1), a warp a body, into sm[body - b0][4], at
+// most kWarpsPerBlock bodies; ends with a barrier.  The threads of the first
+// b1 - b0 bodies then update them side by side.
+__device__ __forceinline__ void block_forces(const BumpySys *bs, int b0, int b1, bool walls, ForceWarp *fw,
+                                             double (*sm)[4]) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, b = b0 + wid;
+    if (b < b1) {
+        const double sum = body_forces(bs, b, walls, fw[wid]);
+        if (lane < 4) sm[wid][lane] = sum;
+    }
+    __syncthreads();
+}
+
 // second half: forces (overwrite) + kick dt/2
 __global__ void kb_nve_second(BumpySys *bs, double dt_half) {
     if (halted(&bs->b)) return;
-    const int lane = threadIdx.x & 31;
-    const int b = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-    if (b < bs->b.p.n) {
-        double fx, fy, tq, pe;
-        body_forces(bs, b, lane, bs->b.s.walls != 0, fx, fy, tq, pe);
-        if (lane == 0) {
-            const double g = bs->b.s.damping;
-            if (g != 0.0) {
-                // DampedNVE::step (src/integrator/damped_nve.cu:22-23) with
-                // kernelCalculateRigidDampedForces (kernels.cu:80-87): body
-                // F = 0 - g v, tau = 0 - g omega, then += the vertex sums
-                const double2 u = bs->b.v.vel[b];
-                const double w = bs->x.w[b];
-                bs->b.v.frc[b] = make_double2((0.0 - g * u.x) + fx, (0.0 - g * u.y) + fy);
-                bs->x.tq[b] = (0.0 - g * w) + tq;
-            } else {
-                bs->b.v.frc[b] = make_double2(0.0 + fx, 0.0 + fy);
-                bs->x.tq[b] = 0.0 + tq;
-            }
-            bs->b.w.pe[b] = 0.0 + pe;
-            body_kick(bs, b, dt_half);
-        }
-    }
+    __shared__ ForceWarp fw[kWarpsPerBlock];
+    __shared__ double sm[kWarpsPerBlock][4];
+    const int b0 = blockIdx.x * kWarpsPerBlock, b1 = min(b0 + kWarpsPerBlock, bs->b.p.n), t = threadIdx.x;
+    block_forces(bs, b0, b1, bs->b.s.walls != 0, fw, sm);
+    if (t < b1 - b0) body_nve_second(bs, b0 + t, sm[t][0], sm[t][1], sm[t][2], sm[t][3], dt_half);
     if (grid_last_block(&bs->b)) {
         if (++bs->b.s.nve_steps_done >= bs->b.s.max_steps) bs->b.s.flags |= kDone;
     }
 }
 
 // FIRE move (src/integrator/fire.cu:29-40 with the rigid overrides)
+__device__ __forceinline__ void bodies_fire_move(BumpySys *bs, int b0, int b1, MoveMem &m, double &nd2,
+                                                 double &cd2) {
+    DevSys *ds = &bs->b;
+    const double dt = ds->s.f_dt, alpha = ds->s.f_alpha;
+    const int up = ds->s.fire_uphill;
+    if (up) {
+        double t0 = 0.0, t1 = 0.0;
+        bodies_move(bs, b0, b1, -dt / 2.0, m, [](int) {}, t0, t1);
+    }
+    bodies_move(bs, b0, b1, dt, m, [&](int b) {
+        if (up) {
+            ds->v.vel[b] = make_double2(0.0, 0.0);
+            bs->x.w[b] = 0.0;
+        }
+        body_kick(bs, b, dt / 2.0);
+        body_mix(bs, b, alpha);
+    }, nd2, cd2);
+}
+
 __global__ void kb_fire_move(BumpySys *bs) {
     DevSys *ds = &bs->b;
     if (halted(ds)) return;
-    const int lane = threadIdx.x & 31;
-    const int b = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-    const double dt = ds->s.f_dt, alpha = ds->s.f_alpha;
-    const int up = ds->s.fire_uphill;
+    __shared__ MoveMem m;
+    const int b0 = blockIdx.x * kMoveBodies, b1 = min(b0 + kMoveBodies, ds->p.n);
     double v[2] = {0.0, 0.0};
-    if (b < ds->p.n) {
-        if (up) {
-            double t0, t1;
-            body_move(bs, b, lane, -dt / 2.0, t0, t1);
-            __syncwarp();
-            if (lane == 0) {
-                ds->v.vel[b] = make_double2(0.0, 0.0);
-                bs->x.w[b] = 0.0;
-            }
-        }
-        __syncwarp();
-        if (lane == 0) {
-            body_kick(bs, b, dt / 2.0);
-            body_mix(bs, b, alpha);
-        }
-        __syncwarp();
-        body_move(bs, b, lane, dt, v[0], v[1]);
-    }
+    bodies_fire_move(bs, b0, b1, m, v[0], v[1]);
     const int ops[2] = {1, 1};
     if (grid_reduce<2>(v, ops, ds)) {
         ds->s.max_nd2 = v[0];
@@ -538,46 +616,33 @@ __global__ void kb_fire_move(BumpySys *bs) {
     }
 }
 
-// FIRE force phase (see k_fire_force for the modes); the stop test uses
-// max|F_b| <= fmax_target and max|tau_b| <= tmax_target.
-__global__ void kb_fire_force(BumpySys *bs, int mode, double tmax_target) {
+// a body's new force, torque and energy from its sums and the FIRE kick; adds
+// its terms of the totals: PE, power, max|F|^2, max tau^2
+__device__ __forceinline__ void body_fire_second(BumpySys *bs, int b, double fx, double fy, double tq,
+                                                 double pe, bool kick, double (&v)[4]) {
     DevSys *ds = &bs->b;
-    if (halted(ds)) return;
-    const int lane = threadIdx.x & 31;
-    const int b = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-    double v[4] = {0.0, 0.0, 0.0, 0.0};
-    if (b < ds->p.n) {
-        double fx, fy, tq, pe;
-        body_forces(bs, b, lane, false, fx, fy, tq, pe);
-        if (lane == 0) {
-            double2 f = make_double2(0.0 + fx, 0.0 + fy);
-            ds->v.frc[b] = f;
-            bs->x.tq[b] = 0.0 + tq;
-            ds->w.pe[b] = 0.0 + pe;
-            if (mode != 1) body_kick(bs, b, ds->s.f_dt / 2.0);
-            double2 u = ds->v.vel[b];
-            double w = bs->x.w[b], t = bs->x.tq[b];
-            v[0] = 0.0 + pe;
-            v[1] = f.x * u.x + f.y * u.y + t * w;
-            v[2] = f.x * f.x + f.y * f.y;
-            v[3] = t * t;
-        }
-    }
-    const int ops[4] = {0, 0, 1, 1};
-    if (!grid_reduce<4>(v, ops, ds)) return;
-    DevState &s = ds->s;
+    const double2 f = make_double2(0.0 + fx, 0.0 + fy);
+    ds->v.frc[b] = f;
+    bs->x.tq[b] = 0.0 + tq;
+    ds->w.pe[b] = 0.0 + pe;
+    if (kick) body_kick(bs, b, ds->s.f_dt / 2.0);
+    const double2 u = ds->v.vel[b];
+    const double w = bs->x.w[b], t = 0.0 + tq;
+    v[0] += 0.0 + pe;
+    v[1] += f.x * u.x + f.y * u.y + t * w;
+    v[2] = fmax(v[2], f.x * f.x + f.y * f.y);
+    v[3] = fmax(v[3], t * t);
+}
+
+// End of a FIRE iteration of rigid bodies (see fire_epilogue)
+__device__ __forceinline__ void bumpy_fire_epilogue(BumpySys *bs, const double (&v)[4], double tmax_target) {
+    DevState &s = bs->b.s;
     s.pe = v[0];
     s.power = v[1];
     s.fmax2 = v[2];
     bs->x.tmax2 = v[3];
     double avg = v[0] / s.dof;
-    if (mode == 1) {
-        s.last_avg_pe = avg;
-        fire_decide(s, v[1]);
-        return;
-    }
-    if (mode == 2) return;
-    double diff = fabs(avg / s.last_avg_pe - 1);
+    const bool pe_still = s.pe_diff_target > 0 && fabs(avg / s.last_avg_pe - 1) < s.pe_diff_target;
     s.last_avg_pe = avg;
     long long it = s.iter;
     // mixed form: FP32 vertex pairs until the switch (as k_fire_force), then FP64
@@ -590,7 +655,7 @@ __global__ void kb_fire_force(BumpySys *bs, int mode, double tmax_target) {
             s.fp64_now = 1;
         fp64 = false;
     }
-    if ((fp64 && diff < s.pe_diff_target) || avg < s.pe_target) {
+    if ((fp64 && pe_still) || avg < s.pe_target) {
         s.result_step = it; s.f_converged = 1; s.flags |= kDone; return;
     }
     if (fp64 && s.fmax_target > 0 && sqrt(v[2]) <= s.fmax_target && sqrt(v[3]) <= tmax_target) {
@@ -600,6 +665,34 @@ __global__ void kb_fire_force(BumpySys *bs, int mode, double tmax_target) {
     s.iter = it + 1;
     fire_decide(s, v[1]);
     if (s.f_stopped) { s.result_step = it + 1; s.f_converged = 1; s.flags |= kDone; }
+}
+
+// FIRE force phase (see k_fire_force for the modes); the stop test uses
+// max|F_b| <= fmax_target and max|tau_b| <= tmax_target.
+__global__ void kb_fire_force(BumpySys *bs, int mode, double tmax_target) {
+    DevSys *ds = &bs->b;
+    if (halted(ds)) return;
+    __shared__ ForceWarp fw[kWarpsPerBlock];
+    __shared__ double sm[kWarpsPerBlock][4];
+    const int b0 = blockIdx.x * kWarpsPerBlock, b1 = min(b0 + kWarpsPerBlock, ds->p.n), t = threadIdx.x;
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+    block_forces(bs, b0, b1, false, fw, sm);
+    if (t < b1 - b0) body_fire_second(bs, b0 + t, sm[t][0], sm[t][1], sm[t][2], sm[t][3], mode != 1, v);
+    const int ops[4] = {0, 0, 1, 1};
+    if (!grid_reduce<4>(v, ops, ds)) return;
+    if (mode == 0) {
+        bumpy_fire_epilogue(bs, v, tmax_target);
+        return;
+    }
+    DevState &s = ds->s;
+    s.pe = v[0];
+    s.power = v[1];
+    s.fmax2 = v[2];
+    bs->x.tmax2 = v[3];
+    if (mode == 1) {
+        s.last_avg_pe = v[0] / s.dof;
+        fire_decide(s, v[1]);
+    }
 }
 
 // FIRE power incl. rotation, then the Fire::step decision (single-step API)

@@ -50,6 +50,8 @@ struct dpg_bumpy_system {
     int nlg = 1, ntpb = kTPB;
     int ngrid() const { return std::max(1, (int)(((long long)nb * nlg + ntpb - 1) / ntpb)); }
     void *nlist_fn() const { return nlg == 8 ? (void *)k_nlist_cell<8> : (void *)k_nlist_cell<1>; }
+    int gm() const { return std::max(1, (nb + kMoveBodies - 1) / kMoveBodies); }  // move kernels
+    int gl() const { return (int)(((long long)nv * kVlistLanes + kTPB - 1) / kTPB); }  // vertex list
     int gb(int count) const { return std::max(1, (count + kTPB - 1) / kTPB); }
     int gw(int bodies) const { return std::max(1, (bodies + kWarpsPerBlock - 1) / kWarpsPerBlock); }
     DevSys *ds() const { return &d->b; }
@@ -63,12 +65,12 @@ typedef dpg_bumpy_system BS;
         CK(cudaGetLastError());                                   \
     } while (0)
 
-// mixed form: vertex offsets from the current vertex positions, before a force
-// evaluation that follows host-side or single-operation changes (the loop
-// kernels keep them current themselves)
+// fixed-point vertex positions and, in the mixed form, the vertex offsets from
+// the current vertex positions, before a force evaluation that follows host-side
+// or single-operation changes (the loop kernels keep them current themselves)
 static int vrefresh(BS *s) {
-    if (s->prm.precision != DPG_MIXED) return DPG_OK;
-    kb_mixed_refresh<<<(s->nv + kTPB - 1) / kTPB, kTPB, 0, s->stream>>>(s->d);
+    if (s->prm.precision == DPG_MIXED) kb_mixed_refresh<<<(s->nv + kTPB - 1) / kTPB, kTPB, 0, s->stream>>>(s->d);
+    kb_vquant<<<(s->nv + kTPB - 1) / kTPB, kTPB, 0, s->stream>>>(s->d);
     CK(cudaGetLastError());
     return DPG_OK;
 }
@@ -155,7 +157,7 @@ extern "C" int dpg_bumpy_create(const dpg_bumpy_params *p, void *cuda_stream, dp
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     s->nlg = (long long)s->nb < (long long)nsm * 1024 ? 8 : 1;
     s->ntpb = (long long)s->nb * s->nlg < (long long)nsm * 2 * kTPB ? 64 : kTPB;
-    w.max_blocks = std::max(std::max(s->gb(s->nb), s->gw(s->nb)), s->ngrid());
+    w.max_blocks = std::max(std::max(std::max(s->gb(s->nb), s->gw(s->nb)), s->ngrid()), s->gl());
     A((void **)&w.partials, (size_t)w.max_blocks * 8 * 8);
     A((void **)&x.w, nb * 8); A((void **)&x.th, nb * 8); A((void **)&x.tq, nb * 8); A((void **)&x.I, nb * 8);
     A((void **)&x.nvb, nb * 4); A((void **)&x.start, nb * 4);
@@ -165,6 +167,7 @@ extern "C" int dpg_bumpy_create(const dpg_bumpy_params *p, void *cuda_stream, dp
     A((void **)&x.vmass_t, nv * 8); A((void **)&x.vbody, nv * 4); A((void **)&x.vbody_t, nv * 4);
     A((void **)&x.svidx, nv * 4); A((void **)&x.svidx_t, nv * 4); A((void **)&x.vcount, nv * 4);
     if (p->precision == DPG_MIXED) A((void **)&x.vpk, nv * 16);
+    A((void **)&x.vq, nv * 16);
     A((void **)&x.adelta, nb * 8); A((void **)&x.m1a, nb * 8); A((void **)&x.m2a, nb * 8);
     A((void **)&x.stress_b, nb * 32); A((void **)&x.ccount, nb * 4); A((void **)&x.vccount, nb * 4);
     A((void **)&w.s_pos, nb * 16); A((void **)&w.s_vel, nb * 16); A((void **)&w.s_frc, nb * 16);
@@ -421,7 +424,25 @@ static int enqueue_rebuild(BS *s) {
     } else {
         LAUNCH(k_nlist_all, s->gb(s->nb), kTPB, ds);
     }
-    LAUNCH(kb_vlist, s->gw(s->nb), kTPB, s->d);
+    LAUNCH(kb_vquant_rebuild, s->gb(s->nv), kTPB, s->d);
+    LAUNCH(kb_vlist, s->gl(), kTPB, s->d);
+    return DPG_OK;
+}
+
+// what the device derives from the box: DevParams and the vertex-list limits
+static int push_params(BS *s) {
+    DevParams &p = s->h.b.p;
+    params_update(p);
+    CK(cudaMemcpyAsync(&s->d->b.p, &p, sizeof(DevParams), cudaMemcpyHostToDevice, s->stream));
+    const double big = std::max(p.box[0], p.box[1]);
+    const bool on = p.q_tol < INFINITY;
+    float lim[4];
+    quant_limits(s->vcutoff * s->vcutoff, big, on, lim[0], lim[1]);
+    quant_limits(s->vpcutoff * s->vpcutoff, big, on, lim[2], lim[3]);
+    TRY(put(s, &s->d->x.vin2, lim[0]));
+    TRY(put(s, &s->d->x.vout2, lim[1]));
+    TRY(put(s, &s->d->x.vpin2, lim[2]));
+    TRY(put(s, &s->d->x.vpout2, lim[3]));
     return DPG_OK;
 }
 
@@ -451,7 +472,8 @@ static int resolve_overflow(BS *s) {
         } else {
             TRY(put(s, &s->d->x.vlist_built, s->hs->n_rebuilds - 1));
         }
-        LAUNCH(kb_vlist, s->gw(s->nb), kTPB, s->d);
+        LAUNCH(kb_vquant_rebuild, s->gb(s->nv), kTPB, s->d);
+        LAUNCH(kb_vlist, s->gl(), kTPB, s->d);
     }
     return set_err(DPG_ERR_OVERFLOW, "neighbour capacity did not settle");
 }
@@ -520,8 +542,7 @@ extern "C" int dpg_bumpy_setup_neighbors(dpg_bumpy_handle s, const dpg_neighbor_
     DevParams &p = s->h.b.p;
     p.method = s->method; p.ncd = s->ncd; p.ncells = s->ncells; p.cap = s->cap;
     p.cutoff2 = s->cutoff * s->cutoff; p.cell_size = s->cs; p.nthr2 = s->nthr2; p.cthr2 = s->cthr2;
-    params_update(p);
-    CK(cudaMemcpyAsync(&s->d->b.p, &p, sizeof(DevParams), cudaMemcpyHostToDevice, s->stream));
+    TRY(push_params(s));
     TRY(put(s, &s->d->x.vcut2, s->vcutoff * s->vcutoff));
     TRY(put(s, &s->d->x.vpcut2, s->vpcutoff * s->vpcutoff));
     TRY(pull(s));
@@ -596,7 +617,7 @@ extern "C" int dpg_bumpy_kick(dpg_bumpy_handle s, double dt) {
 
 extern "C" int dpg_bumpy_drift(dpg_bumpy_handle s, double dt) {
     if (!s) return set_err(DPG_ERR_ARG, "null handle");
-    LAUNCH(kb_drift, s->gw(s->nb), kTPB, s->d, dt);
+    LAUNCH(kb_drift, s->gm(), kTPB, s->d, dt);
     return DPG_OK;
 }
 
@@ -634,8 +655,7 @@ extern "C" int dpg_bumpy_scale_box(dpg_bumpy_handle s, double factor) {
     s->h.b.p.box[0] = nl;
     s->h.b.p.box[1] = nl;
     if (s->ncd > 0) { s->cs = nl / s->ncd; s->h.b.p.cell_size = s->cs; }
-    params_update(s->h.b.p);
-    CK(cudaMemcpyAsync(&s->d->b.p, &s->h.b.p, sizeof(DevParams), cudaMemcpyHostToDevice, s->stream));
+    TRY(push_params(s));
     return DPG_OK;
 }
 
@@ -657,8 +677,8 @@ static cudaGraphNode_t addk(cudaGraph_t g, cudaGraphNode_t dep, void *fn, int bl
 
 // kind 0 FIRE, 1 NVE
 static int enqueue_iteration(BS *s, int kind) {
-    if (kind == 0) LAUNCH(kb_fire_move, s->gw(s->nb), kTPB, s->d);
-    else LAUNCH(kb_nve_first, s->gw(s->nb), kTPB, s->d, 0.5 * s->loop_dt, s->loop_dt);
+    if (kind == 0) LAUNCH(kb_fire_move, s->gm(), kTPB, s->d);
+    else LAUNCH(kb_nve_first, s->gm(), kTPB, s->d, 0.5 * s->loop_dt, s->loop_dt);
     TRY(enqueue_rebuild(s));
     if (kind == 0) LAUNCH(kb_fire_force, s->gw(s->nb), kTPB, s->d, 0, s->loop_tmax);
     else LAUNCH(kb_nve_second, s->gw(s->nb), kTPB, s->d, 0.5 * s->loop_dt);
@@ -693,8 +713,8 @@ static int build_graph(BS *s, int kind) {
     int GW = s->gw(s->nb), GB = s->gb(s->nb);
     cudaGraphNode_t last = nullptr;
     if (err == cudaSuccess)
-        last = kind == 0 ? addk(body, nullptr, (void *)kb_fire_move, GW, kTPB, a_b, &err)
-                         : addk(body, nullptr, (void *)kb_nve_first, GW, kTPB, a_n1, &err);
+        last = kind == 0 ? addk(body, nullptr, (void *)kb_fire_move, s->gm(), kTPB, a_b, &err)
+                         : addk(body, nullptr, (void *)kb_nve_first, s->gm(), kTPB, a_n1, &err);
     cudaGraphNodeParams ip = {};
     ip.type = cudaGraphNodeTypeConditional;
     ip.conditional.handle = hrb;
@@ -717,7 +737,8 @@ static int build_graph(BS *s, int kind) {
         } else {
             prev = addk(ib, prev, (void *)k_nlist_all, GB, kTPB, a_d, &err);
         }
-        prev = addk(ib, prev, (void *)kb_vlist, GW, kTPB, a_b, &err);
+        prev = addk(ib, prev, (void *)kb_vquant_rebuild, s->gb(s->nv), kTPB, a_b, &err);
+        prev = addk(ib, prev, (void *)kb_vlist, s->gl(), kTPB, a_b, &err);
         last = kind == 0 ? addk(body, inode, (void *)kb_fire_force, GW, kTPB, a_ff, &err)
                          : addk(body, inode, (void *)kb_nve_second, GW, kTPB, a_n2, &err);
         last = addk(body, last, (void *)k_loop_guard, 1, 1, a_d, &err);
@@ -803,7 +824,7 @@ extern "C" int dpg_bumpy_fire_step(dpg_bumpy_handle s, int *stopped) {
     TRY(need(s));
     TRY(put(s, &s->d->b.s.flags, 0));
     LAUNCH(kb_fire_power_decide, s->gb(s->nb), kTPB, s->d);
-    LAUNCH(kb_fire_move, s->gw(s->nb), kTPB, s->d);
+    LAUNCH(kb_fire_move, s->gm(), kTPB, s->d);
     TRY(enqueue_rebuild(s));
     TRY(resolve_overflow(s));
     TRY(vrefresh(s));
@@ -1025,8 +1046,7 @@ extern "C" int dpg_bumpy_restore_state(dpg_bumpy_handle s) {
     // Particle::setBoxSize: the box only; the cell size keeps its value
     s->h.b.p.box[0] = s->snap_box[0];
     s->h.b.p.box[1] = s->snap_box[1];
-    params_update(s->h.b.p);
-    CK(cudaMemcpyAsync(&s->d->b.p, &s->h.b.p, sizeof(DevParams), cudaMemcpyHostToDevice, s->stream));
+    TRY(push_params(s));
     TRY(rebuild_now(s, 1));
     return vrefresh(s);
 }
@@ -1135,8 +1155,7 @@ extern "C" int dpg_bumpy_set_box(dpg_bumpy_handle s, double bx, double by) {
     s->h.b.p.box[0] = bx;
     s->h.b.p.box[1] = by;
     if (s->ncd > 0) { s->cs = bx / s->ncd; s->h.b.p.cell_size = s->cs; }
-    params_update(s->h.b.p);
-    CK(cudaMemcpyAsync(&s->d->b.p, &s->h.b.p, sizeof(DevParams), cudaMemcpyHostToDevice, s->stream));
+    TRY(push_params(s));
     return DPG_OK;
 }
 

@@ -75,18 +75,19 @@ typedef PairWarp<3> ForceWarp;   // force x, force y, energy
 // what the pair sums read (the caller may keep it in registers)
 struct PairArgs {
     const double2 *pos;
-    const double *rad;
+    const double *rad;   // null: every radius is rv
     const int *nbr;
     const uint4 *q;
     int n;
     double bx, by, e_c, n_c;
     int l4x, l4y;
     float sx, sy, tol;
+    double rv;
 };
 
 __device__ __forceinline__ PairArgs pair_args(const DevSys *ds) {
     return {ds->v.pos, ds->v.rad, ds->v.nbr, ds->v.q, ds->p.n, ds->p.box[0], ds->p.box[1], ds->p.e_c,
-            ds->p.n_c, ds->p.q_l4[0], ds->p.q_l4[1], ds->p.q_s[0], ds->p.q_s[1], ds->p.q_tol};
+            ds->p.n_c, ds->p.q_l4[0], ds->p.q_l4[1], ds->p.q_s[0], ds->p.q_s[1], ds->p.q_tol, 0.0};
 }
 
 // disk_pair for the sums (see pbc_dist_sum)
@@ -204,7 +205,8 @@ __device__ __forceinline__ void pair_sums(const PairArgs &f, int i, int cnt, Pai
                 if (e < w1) {
                     const int j = f.nbr[(size_t)(s0 + (ent & 31)) * f.n + io];
                     double dx, dy, fx, fy;
-                    const double ee = disk_pair_sum(f, f.pos[io], f.rad[io], f.pos[j], f.rad[j], dx, dy, fx, fy);
+                    const double ri = f.rad ? f.rad[io] : f.rv, rj = f.rad ? f.rad[j] : f.rv;
+                    const double ee = disk_pair_sum(f, f.pos[io], ri, f.pos[j], rj, dx, dy, fx, fy);
                     if (K == 3) {
                         w.r[0][e - w0] = fx;
                         w.r[1][e - w0] = fy;
@@ -900,15 +902,19 @@ __device__ __forceinline__ void finish_list_build(DevSys *ds, int cnt) {
 
 // d2 < cutoff2 for particles i and j, decided by the fixed-point distance where
 // it can, by the FP64 test of the reference where it cannot
+__device__ __forceinline__ bool within(const DevParams &p, const double2 *a, int i, const double2 *b, int j,
+                                       uint4 qi, uint4 qj, float in2, float out2, double c2) {
+    const float d2 = quant_d2(p.q_s[0], p.q_s[1], qi, qj);
+    const bool marked = (qi.w | qj.w) != 0;
+    if (!marked && d2 > out2) return false;
+    if (!marked && d2 < in2) return true;
+    const double2 pi = a[i], pj = b[j];
+    const double dx = pbc_dist(pi.x, pj.x, p.box[0]), dy = pbc_dist(pi.y, pj.y, p.box[1]);
+    return dx * dx + dy * dy < c2;
+}
 __device__ __forceinline__ bool within_cutoff(const DevSys *ds, const double2 *pos, int i, int j, uint4 qi,
                                               uint4 qj) {
-    const float d2 = quant_d2(ds->p.q_s[0], ds->p.q_s[1], qi, qj);
-    const bool marked = (qi.w | qj.w) != 0;
-    if (!marked && d2 > ds->p.q_out2) return false;
-    if (!marked && d2 < ds->p.q_in2) return true;
-    const double2 pi = pos[i], pj = pos[j];
-    const double dx = pbc_dist(pi.x, pj.x, ds->p.box[0]), dy = pbc_dist(pi.y, pj.y, ds->p.box[1]);
-    return dx * dx + dy * dy < ds->p.cutoff2;
+    return within(ds->p, pos, i, pos, j, qi, qj, ds->p.q_in2, ds->p.q_out2, ds->p.cutoff2);
 }
 
 // The neighbour row of particle i from the 3x3 cells around its own

@@ -74,3 +74,27 @@ def test_lists_and_sums_match_the_oracle(n, phi, images, unit, lanes):
     assert s.getContactCount() == o.contact_count()
     np.testing.assert_allclose(s.getPressure(), o.pressure(), rtol=1e-12)
     s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,phi,n_small", [(1, 0.5, 20), (33, 0.8, 3), (100, 0.9, 20), (65, 0.9, 33), (40, 1.5, 70)])
+def test_vertex_lists_and_sums_match_the_oracle(n, phi, n_small):
+    import dpcuda_gb300 as dpg
+    from oracle.oracle import BumpyOracle, bumpy_packing
+    st = bumpy_packing(n, phi, 5, n_small=n_small)
+    o = BumpyOracle(n, st["nv"], st["box"], st["e_c"], 2.0, st["rv"], st["seg"], True)
+    o.set_bodies(st["x"], st["y"], st["th"], st["r"], st["nvb"])
+    o.init_vertices()
+    o.set_mass(1.0)
+    o.setup_neighbors(0, 1.5, 0.2, 8.0, 0.5)
+    px, py = o.vertices()
+    b = dpg.RigidBumpy(n, st["nv"], st["box"], st["e_c"], 2.0, st["rv"], st["seg"], True)
+    b.setBodies(st["x"], st["y"], st["th"], st["r"], st["nvb"])
+    b.setVertexPositions(px, py)
+    b.setMass(1.0)
+    b.setupNeighbors("cell", 1.5, 0.2, 8.0, 0.5)
+    g, r = b.getBodies(), o.bodies()
+    for k in ("fx", "fy", "tq", "pe"):
+        np.testing.assert_array_equal(g[k], r[k], err_msg=k)
+    assert b.getVertexNeighborSets() == o.vertex_neighbor_sets()
+    b.close()
