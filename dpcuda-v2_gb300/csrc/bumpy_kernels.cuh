@@ -34,6 +34,8 @@ struct BumpyExt {
     int *vnbr, *vcount;      // vertex neighbour list, column-major [capv][nv]
     float4 *vpk;             // mixed form: packed FP32 vertex offsets (see mixed_pack)
     uint4 *vq;               // fixed-point vertex positions (see Quant in dpg_device.cuh)
+    float4 *vpk_t;           // the other buffers of vpk and vq (NVE in the resident grid)
+    uint4 *vq_t;
     float vin2, vout2, vpin2, vpout2;  // filter limits of the two vertex-list cutoffs
     int mixed;               // 1: FP32 vertex pairs (the body DevParams stay FP64)
     long long vlist_built;   // n_rebuilds value at the last vertex-list build
@@ -86,13 +88,6 @@ __global__ void kb_kick(BumpySys *bs, double dt) {
     body_kick(bs, b, dt);
 }
 
-// what the loops' move kernels keep current with a vertex position (see moved_update)
-__device__ __forceinline__ void vertex_moved(BumpySys *bs, int v, double2 q) {
-    BumpyExt &x = bs->x;
-    if (x.mixed) x.vpk[v] = mixed_pack(bs->b.p, q, x.rv);
-    if (!x.mixed || bs->b.s.fp64_now) x.vq[v] = quant_of(bs->b.p, q, x.rv);
-}
-
 // ---- body + vertex move: kernelUpdateRigidPositions + kernelTranslateAndRotateVertices1
 // (kernels.cu:21-78,152-201) of the bodies [b0, b1) by a block.  The body part
 // (kick, displacement, cosine and sine of the increment: some 130 FP64
@@ -103,10 +98,12 @@ __device__ __forceinline__ void vertex_moved(BumpySys *bs, int v, double2 q) {
 struct MoveMem {
     double2 p[kMoveBodies], n[kMoveBodies], cs[kMoveBodies];
 };
-// pre(b): what a body does before it moves (thread of the body)
+// pre(b): what a body does before it moves (thread of the body); vpos, vpk, vq:
+// where the moved vertices go, with what the pair loops read of them (see
+// moved_update)
 template <class F>
 __device__ __forceinline__ void bodies_move(BumpySys *bs, int b0, int b1, double dt, MoveMem &m, F pre,
-                                            double &nd2, double &cd2) {
+                                            double &nd2, double &cd2, double2 *vpos, float4 *vpk, uint4 *vq) {
     DevSys &d = bs->b;
     BumpyExt &x = bs->x;
     for (int base = b0; base < b1; base += kMoveBodies) {
@@ -137,8 +134,9 @@ __device__ __forceinline__ void bodies_move(BumpySys *bs, int b0, int b1, double
             const double rx = q.x - p.x, ry = q.y - p.y;
             const double rxr = rx * cs.x - ry * cs.y, ryr = rx * cs.y + ry * cs.x;
             const double2 nq = make_double2(n.x + rxr, n.y + ryr);
-            x.vpos[v] = nq;
-            vertex_moved(bs, v, nq);
+            vpos[v] = nq;
+            if (x.mixed) vpk[v] = mixed_pack(d.p, nq, x.rv);
+            if (!x.mixed || d.s.fp64_now) vq[v] = quant_of(d.p, nq, x.rv);
         }
         __syncthreads();
     }
@@ -148,7 +146,7 @@ __global__ void kb_drift(BumpySys *bs, double dt) {
     __shared__ MoveMem m;
     const int b0 = blockIdx.x * kMoveBodies, b1 = min(b0 + kMoveBodies, bs->b.p.n);
     double v[2] = {0.0, 0.0};
-    bodies_move(bs, b0, b1, dt, m, [](int) {}, v[0], v[1]);
+    bodies_move(bs, b0, b1, dt, m, [](int) {}, v[0], v[1], bs->x.vpos, bs->x.vpk, bs->x.vq);
     const int ops[2] = {1, 1};
     if (grid_reduce<2>(v, ops, &bs->b)) { bs->b.s.max_nd2 = v[0]; bs->b.s.max_cd2 = v[1]; }
 }
@@ -403,10 +401,7 @@ __global__ void kb_vlist(BumpySys *bs) {
 
 // ---- re-sort of bodies and their vertex blocks:
 // RigidBumpy::reorderParticleData (rigid_bumpy.cu:1303-1376, kernels.cu:796-868)
-__global__ void kb_reorder_bodies(BumpySys *bs) {
-    if (bs->b.s.rebuild != 2) return;
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= bs->b.p.n) return;
+__device__ __forceinline__ void reorder_body(BumpySys *bs, int s) {
     DevSys &d = bs->b;
     BumpyExt &x = bs->x;
     int o = d.w.perm[s];
@@ -426,6 +421,12 @@ __global__ void kb_reorder_bodies(BumpySys *bs) {
     x.nvb_t[s] = x.nvb[o];
     d.w.cell_of[s] = d.w.cell_raw[o];
     d.w.pos_c[s] = p;
+}
+
+__global__ void kb_reorder_bodies(BumpySys *bs) {
+    if (bs->b.s.rebuild != 2) return;
+    int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < bs->b.p.n) reorder_body(bs, s);
 }
 
 // exclusive scan of the re-sorted vertex counts into the new block starts (one block)
@@ -466,49 +467,41 @@ __global__ void __launch_bounds__(kScanTPB) kb_scan_starts(BumpySys *bs) {
     }
 }
 
-// move every vertex block to its body's new start (warp per new body), then
-// swap current / alternate buffers on the device (last block)
+// move the vertex block of new body s to its new start, one warp
+__device__ __forceinline__ void reorder_vertices(BumpySys *bs, int s, int lane) {
+    BumpyExt &x = bs->x;
+    int o = bs->b.w.perm[s];
+    int of = x.start[o], nf = x.start_t[s], n = x.nvb_t[s];
+    for (int k = lane; k < n; k += 32) {
+        x.vpos_t[nf + k] = x.vpos[of + k];
+        x.vmass_t[nf + k] = x.vmass[of + k];
+        x.svidx_t[nf + k] = x.svidx[of + k];
+        x.vbody_t[nf + k] = s;
+    }
+}
+
+// after a re-sort: the sorted buffers become the current ones
+__device__ __forceinline__ void swap_sorted(BumpySys *bs) {
+    DevView &v = bs->b.v;
+    BumpyExt &x = bs->x;
+    swap_ptr(v.pos, v.pos_t); swap_ptr(v.vel, v.vel_t); swap_ptr(v.frc, v.frc_t);
+    swap_ptr(v.rad, v.rad_t); swap_ptr(v.mass, v.mass_t); swap_ptr(v.sidx, v.sidx_t);
+    swap_ptr(v.m1, v.m1_t); swap_ptr(v.m2, v.m2_t);
+    swap_ptr(x.w, x.w_t); swap_ptr(x.th, x.th_t); swap_ptr(x.tq, x.tq_t); swap_ptr(x.I, x.I_t);
+    swap_ptr(x.nvb, x.nvb_t); swap_ptr(x.start, x.start_t);
+    swap_ptr(x.vpos, x.vpos_t); swap_ptr(x.vmass, x.vmass_t);
+    swap_ptr(x.vbody, x.vbody_t); swap_ptr(x.svidx, x.svidx_t);
+}
+
+// the vertex blocks (warp per new body), then the swap (last block)
 __global__ void kb_reorder_vertices(BumpySys *bs) {
     if (bs->b.s.rebuild != 2) return;
-    const int lane = threadIdx.x & 31;
     const int s = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-    DevSys &d = bs->b;
-    BumpyExt &x = bs->x;
-    if (s < d.p.n) {
-        int o = d.w.perm[s];
-        int of = x.start[o], nf = x.start_t[s], n = x.nvb_t[s];
-        for (int k = lane; k < n; k += 32) {
-            x.vpos_t[nf + k] = x.vpos[of + k];
-            x.vmass_t[nf + k] = x.vmass[of + k];
-            x.svidx_t[nf + k] = x.svidx[of + k];
-            x.vbody_t[nf + k] = s;
-        }
-    }
+    if (s < bs->b.p.n) reorder_vertices(bs, s, threadIdx.x & 31);
     if (grid_last_block(&bs->b)) {
-        DevView &v = d.v;
-        double2 *t2;
-        double *t1;
-        int *ti;
-        t2 = v.pos; v.pos = v.pos_t; v.pos_t = t2;
-        t2 = v.vel; v.vel = v.vel_t; v.vel_t = t2;
-        t2 = v.frc; v.frc = v.frc_t; v.frc_t = t2;
-        t1 = v.rad; v.rad = v.rad_t; v.rad_t = t1;
-        t1 = v.mass; v.mass = v.mass_t; v.mass_t = t1;
-        ti = v.sidx; v.sidx = v.sidx_t; v.sidx_t = ti;
-        t2 = v.m1; v.m1 = v.m1_t; v.m1_t = t2;
-        t2 = v.m2; v.m2 = v.m2_t; v.m2_t = t2;
-        t1 = x.w; x.w = x.w_t; x.w_t = t1;
-        t1 = x.th; x.th = x.th_t; x.th_t = t1;
-        t1 = x.tq; x.tq = x.tq_t; x.tq_t = t1;
-        t1 = x.I; x.I = x.I_t; x.I_t = t1;
-        ti = x.nvb; x.nvb = x.nvb_t; x.nvb_t = ti;
-        ti = x.start; x.start = x.start_t; x.start_t = ti;
-        t2 = x.vpos; x.vpos = x.vpos_t; x.vpos_t = t2;
-        t1 = x.vmass; x.vmass = x.vmass_t; x.vmass_t = t1;
-        ti = x.vbody; x.vbody = x.vbody_t; x.vbody_t = ti;
-        ti = x.svidx; x.svidx = x.svidx_t; x.svidx_t = ti;
-        d.s.max_cd2 = 0.0;
-        d.s.n_cell_rebuilds++;
+        swap_sorted(bs);
+        bs->b.s.max_cd2 = 0.0;
+        bs->b.s.n_cell_rebuilds++;
     }
 }
 
@@ -520,7 +513,8 @@ __global__ void kb_nve_first(BumpySys *bs, double dt_half, double dt) {
     __shared__ MoveMem m;
     const int b0 = blockIdx.x * kMoveBodies, b1 = min(b0 + kMoveBodies, bs->b.p.n);
     double v[2] = {0.0, 0.0};
-    bodies_move(bs, b0, b1, dt, m, [&](int b) { body_kick(bs, b, dt_half); }, v[0], v[1]);
+    bodies_move(bs, b0, b1, dt, m, [&](int b) { body_kick(bs, b, dt_half); }, v[0], v[1],
+                bs->x.vpos, bs->x.vpk, bs->x.vq);
     const int ops[2] = {1, 1};
     if (grid_reduce<2>(v, ops, &bs->b)) {
         DevSys *ds = &bs->b;
@@ -587,7 +581,7 @@ __device__ __forceinline__ void bodies_fire_move(BumpySys *bs, int b0, int b1, M
     const int up = ds->s.fire_uphill;
     if (up) {
         double t0 = 0.0, t1 = 0.0;
-        bodies_move(bs, b0, b1, -dt / 2.0, m, [](int) {}, t0, t1);
+        bodies_move(bs, b0, b1, -dt / 2.0, m, [](int) {}, t0, t1, bs->x.vpos, bs->x.vpk, bs->x.vq);
     }
     bodies_move(bs, b0, b1, dt, m, [&](int b) {
         if (up) {
@@ -596,7 +590,7 @@ __device__ __forceinline__ void bodies_fire_move(BumpySys *bs, int b0, int b1, M
         }
         body_kick(bs, b, dt / 2.0);
         body_mix(bs, b, alpha);
-    }, nd2, cd2);
+    }, nd2, cd2, bs->x.vpos, bs->x.vpk, bs->x.vq);
 }
 
 __global__ void kb_fire_move(BumpySys *bs) {

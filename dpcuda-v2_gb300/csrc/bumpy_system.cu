@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "bumpy_kernels.cuh"
+#include "bumpy_loop.cuh"
 #include "host_common.h"
 
 using namespace dpg;
@@ -39,7 +40,9 @@ struct dpg_bumpy_system {
     std::vector<void *> allocs;
     int *nbr = nullptr, *vnbr = nullptr, *cell_buf = nullptr;
     double *xfer = nullptr;
-    int mode = 2;
+    int mode = 2;  // 3 resident grid, 2 graph, 0 separate launches
+    LoopSync *lsync = nullptr;          // resident grid: barrier state,
+    int lblocks = 0, lchunk = 0, ltpb = 0;  // blocks, bodies a block, threads a block
     cudaGraphExec_t loop_exec[2] = {nullptr, nullptr};
     cudaGraphConditionalHandle h_loop[2] = {0, 0}, h_rb[2] = {0, 0};
     double loop_dt = 0.0, loop_tmax = 0.0;
@@ -138,6 +141,7 @@ extern "C" int dpg_bumpy_create(const dpg_bumpy_params *p, void *cuda_stream, dp
     }
     const char *m = getenv("DPG_LOOP_MODE");
     if (m && (!strcmp(m, "stream") || !strcmp(m, "graph"))) s->mode = 0;
+    else if (!(m && !strcmp(m, "cond"))) s->mode = 3;
     const size_t nb = s->nb, nv = s->nv;
     int rc = DPG_OK;
     auto A = [&](void **pp, size_t b) { if (rc == DPG_OK) rc = balloc(s, pp, b); };
@@ -158,6 +162,7 @@ extern "C" int dpg_bumpy_create(const dpg_bumpy_params *p, void *cuda_stream, dp
     s->nlg = (long long)s->nb < (long long)nsm * 1024 ? 8 : 1;
     s->ntpb = (long long)s->nb * s->nlg < (long long)nsm * 2 * kTPB ? 64 : kTPB;
     w.max_blocks = std::max(std::max(std::max(s->gb(s->nb), s->gw(s->nb)), s->ngrid()), s->gl());
+    w.max_blocks = std::max(w.max_blocks, nsm);
     A((void **)&w.partials, (size_t)w.max_blocks * 8 * 8);
     A((void **)&x.w, nb * 8); A((void **)&x.th, nb * 8); A((void **)&x.tq, nb * 8); A((void **)&x.I, nb * 8);
     A((void **)&x.nvb, nb * 4); A((void **)&x.start, nb * 4);
@@ -168,6 +173,9 @@ extern "C" int dpg_bumpy_create(const dpg_bumpy_params *p, void *cuda_stream, dp
     A((void **)&x.svidx, nv * 4); A((void **)&x.svidx_t, nv * 4); A((void **)&x.vcount, nv * 4);
     if (p->precision == DPG_MIXED) A((void **)&x.vpk, nv * 16);
     A((void **)&x.vq, nv * 16);
+    A((void **)&x.vq_t, nv * 16);
+    if (p->precision == DPG_MIXED) A((void **)&x.vpk_t, nv * 16);
+    A((void **)&s->lsync, sizeof(LoopSync));
     A((void **)&x.adelta, nb * 8); A((void **)&x.m1a, nb * 8); A((void **)&x.m2a, nb * 8);
     A((void **)&x.stress_b, nb * 32); A((void **)&x.ccount, nb * 4); A((void **)&x.vccount, nb * 4);
     A((void **)&w.s_pos, nb * 16); A((void **)&w.s_vel, nb * 16); A((void **)&w.s_frc, nb * 16);
@@ -230,7 +238,7 @@ static int reset_views(BS *s) {
     cur.w_t = h.w_t; cur.th_t = h.th_t; cur.tq_t = h.tq_t; cur.I_t = h.I_t; cur.nvb_t = h.nvb_t;
     cur.start_t = h.start_t; cur.vpos = h.vpos; cur.vpos_t = h.vpos_t; cur.vmass = h.vmass;
     cur.vmass_t = h.vmass_t; cur.vbody = h.vbody; cur.vbody_t = h.vbody_t; cur.svidx = h.svidx;
-    cur.svidx_t = h.svidx_t;
+    cur.svidx_t = h.svidx_t; cur.vq = h.vq; cur.vq_t = h.vq_t; cur.vpk = h.vpk; cur.vpk_t = h.vpk_t;
     CK(cudaMemcpyAsync(&s->d->x, &cur, sizeof(BumpyExt), cudaMemcpyHostToDevice, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     return DPG_OK;
@@ -754,9 +762,58 @@ static int build_graph(BS *s, int kind) {
     return DPG_OK;
 }
 
+// The resident grid: a block an SM, its bodies' forces a warp a body.  Above
+// kLoopBodies bodies a block the loops stay graphs of full-size kernels.
+static int plan_resident(BS *s) {
+    int dev = 0, nsm = 0, coop = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    const int per = (s->nb + nsm - 1) / nsm;
+    if (!coop || per > kLoopBodies) return set_err(DPG_ERR_STATE, "no resident loop for this system");
+    // at least 8 warps for the list builds, at most a warp a body beyond that
+    s->ltpb = std::min(kLoopMaxTPB, std::max(256, 32 * per));
+    for (void *fn : {(void *)kb_loop<0>, (void *)kb_loop<1>}) {
+        int occ = 0;
+        // the attribute is the function's, whichever system launches it: the largest block's
+        CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(sizeof(ForceWarp) * (kLoopMaxTPB / 32))));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, s->ltpb, sizeof(ForceWarp) * (s->ltpb / 32)));
+        if (occ < 1) return set_err(DPG_ERR_CUDA, "the resident loop does not fit an SM");
+    }
+    s->lchunk = per;
+    s->lblocks = (s->nb + per - 1) / per;
+    return DPG_OK;
+}
+
+static int run_resident(BS *s, int kind) {
+    void *fn = kind == 0 ? (void *)kb_loop<0> : (void *)kb_loop<1>;
+    long long most = std::max<long long>(256, (1LL << 24) / (s->nb + 1024));
+    double dt = s->loop_dt, tmax = s->loop_tmax;
+    void *args[] = {(void *)&s->d, (void *)&s->lsync, (void *)&dt, (void *)&tmax, (void *)&s->lchunk, (void *)&most};
+    do {
+        CK(cudaMemsetAsync(s->lsync, 0, sizeof(LoopSync), s->stream));
+        CK(cudaLaunchCooperativeKernel(fn, dim3(s->lblocks), dim3(s->ltpb), args,
+                                       sizeof(ForceWarp) * (s->ltpb / 32), s->stream));
+        TRY(pull(s));
+        if (s->hs->flags & kError) return set_err(DPG_ERR_TIMEOUT, "a grid barrier of the resident loop ran out");
+    } while (!s->hs->flags);
+    return DPG_OK;
+}
+
 static int run_loop(BS *s, int kind, int *ovf) {
     *ovf = 0;
     TRY(vrefresh(s));
+    if (s->mode == 3) {
+        if (!s->lblocks && plan_resident(s) != DPG_OK) {
+            (void)cudaGetLastError();
+            s->mode = 2;
+        } else {
+            TRY(run_resident(s, kind));
+            if (s->hs->flags & kOverflow) *ovf = 1;
+            return DPG_OK;
+        }
+    }
     if (s->mode == 2) {
         if (build_graph(s, kind) != DPG_OK) {
             s->mode = 0;

@@ -16,6 +16,13 @@ namespace {  // kernels have internal linkage: each translation unit owns its co
 
 constexpr int kMixed = 1;  // DevParams.precision of the mixed form (DPG_MIXED)
 
+template <class T>
+__device__ __forceinline__ void swap_ptr(T *&a, T *&b) {
+    T *t = a;
+    a = b;
+    b = t;
+}
+
 __device__ __forceinline__ bool halted(const DevSys *ds) { return ds->s.flags != 0; }
 
 // harmonic (power-law) contact of particle i with j, force on i:
@@ -871,17 +878,14 @@ __global__ void k_reorder(DevSys *ds) {
     }
     if (grid_last_block(ds)) {
         DevView &v = ds->v;
-        double2 *t2;
-        double *t1;
-        int *ti;
-        t2 = v.pos; v.pos = v.pos_t; v.pos_t = t2;
-        t2 = v.vel; v.vel = v.vel_t; v.vel_t = t2;
-        t2 = v.frc; v.frc = v.frc_t; v.frc_t = t2;
-        t1 = v.rad; v.rad = v.rad_t; v.rad_t = t1;
-        t1 = v.mass; v.mass = v.mass_t; v.mass_t = t1;
-        ti = v.sidx; v.sidx = v.sidx_t; v.sidx_t = ti;
-        t2 = v.m1; v.m1 = v.m1_t; v.m1_t = t2;
-        t2 = v.m2; v.m2 = v.m2_t; v.m2_t = t2;
+        swap_ptr(v.pos, v.pos_t);
+        swap_ptr(v.vel, v.vel_t);
+        swap_ptr(v.frc, v.frc_t);
+        swap_ptr(v.rad, v.rad_t);
+        swap_ptr(v.mass, v.mass_t);
+        swap_ptr(v.sidx, v.sidx_t);
+        swap_ptr(v.m1, v.m1_t);
+        swap_ptr(v.m2, v.m2_t);
         ds->s.max_cd2 = 0.0;
         ds->s.n_cell_rebuilds++;
     }

@@ -33,6 +33,7 @@ struct LoopSync {
     unsigned long long ring[4];  // barrier k uses ring[k & 3]: arrivals and flag counts
     int err;                     // a barrier ran out of polls
     int max_count;               // longest neighbour row of the last list build
+    int max_vcount;              // longest vertex row (rigid bodies)
 };
 
 // what a barrier carries besides the arrival count (bits 0 - 15): how many
@@ -117,18 +118,24 @@ __device__ __forceinline__ void cell_scan_block(const int *cnt, int *start, int 
     if (threadIdx.x == 0) start[ncells] = carry;
 }
 
-template <class T>
-__device__ __forceinline__ void swap_ptr(T *&a, T *&b) {
-    T *t = a;
-    a = b;
-    b = t;
-}
-
 // a block's slots and the tiles it walks them in: every thread runs the same
 // number of tiles (G lanes per slot), `i < last` says whether its slot is real
 struct Range {
     int first, last;
 };
+
+// neighbour row of particle i by the all-pairs methods, one thread
+__device__ __forceinline__ int nlist_all_row(const DevSys *ds, int i) {
+    const DevView &v = ds->v;
+    const uint4 qi = v.q[i];
+    int cnt = 0;
+    for (int j = 0; j < ds->p.n; j++) {
+        if (j == i || !within_cutoff(ds, v.pos, i, j, qi, v.q[j])) continue;
+        if (cnt < ds->p.cap) v.nbr[(size_t)cnt * ds->p.n + i] = j;
+        cnt++;
+    }
+    return cnt;
+}
 
 // The rebuild of the cell list (kind 2) and the neighbour list inside the
 // loop: the kernels k_cell_index .. k_nlist_cell as phases between barriers.
@@ -204,13 +211,7 @@ __device__ bool loop_rebuild(DevSys *ds, LoopSync *ls, unsigned &bk, int kind, R
         }
     } else {
         for (int i = r.first + t; i < r.last; i += nt) {
-            const uint4 qi = v.q[i];
-            int cnt = 0;
-            for (int j = 0; j < p.n; j++) {
-                if (j == i || !within_cutoff(ds, v.pos, i, j, qi, v.q[j])) continue;
-                if (cnt < p.cap) v.nbr[(size_t)cnt * p.n + i] = j;
-                cnt++;
-            }
+            const int cnt = nlist_all_row(ds, i);
             mx = max(mx, cnt);
             const double2 x = v.pos[i];
             ds->w.count[i] = cnt;
@@ -257,36 +258,74 @@ __device__ __forceinline__ int rebuild_kind(unsigned long long w) {
     return raised(w, kNeedCell) ? 2 : (raised(w, kNeedList) ? 1 : 0);
 }
 
-// Sums (0, 1) and maximum (2) of the first nwr warps' values in a fixed order;
-// thread 0 gets them.  Every thread of the block calls it.
-__device__ __forceinline__ void reduce3(double (&v)[3], int nwr, double *sm) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (wid < nwr) {
+// Maximum of non-negative numbers without the FP64 pipe: their bits order them.
+// A NaN b is dropped, as fmax does.
+__device__ __forceinline__ double max_pos(double a, double b) {
+    const long long ia = __double_as_longlong(a), ib = __double_as_longlong(b);
+    return ib > ia && ib <= 0x7ff0000000000000LL ? b : a;
+}
+
+// The totals of a FIRE iteration over the grid: v[0], v[1] summed, the other
+// K - 2 maxima; thread 0 gets them.  `nwr`: warps that hold values.  Two sums
+// share each FP64 instruction (lanes 0 - 15 and 16 - 31): an instruction holds
+// the pipe for a whole warp whatever its lanes.  The block partials are added
+// in a fixed order, so every block gets the same bits.  false: the barrier ran
+// out.  Every thread of the block calls it.
+template <int K>
+__device__ __forceinline__ void warp_totals(double &sum, double (&mx)[K - 2]) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            v[0] += __shfl_down_sync(0xffffffffu, v[0], o);
-            v[1] += __shfl_down_sync(0xffffffffu, v[1], o);
-            v[2] = fmax(v[2], __shfl_down_sync(0xffffffffu, v[2], o));
-        }
+    for (int o = 8; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o, 16);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < K - 2; k++) mx[k] = max_pos(mx[k], __shfl_down_sync(0xffffffffu, mx[k], o));
+}
+template <int K>
+__device__ __forceinline__ bool grid_totals(double (&v)[K], int nwr, double *part, LoopSync *ls, unsigned &bk,
+                                            double *sm) {
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nb = gridDim.x;
+    double mx[K - 2], sum;
+    if (wid < nwr) {
+        const bool low = lane < 16;
+        sum = low ? v[0] : v[1];
+        sum += __shfl_xor_sync(0xffffffffu, low ? v[1] : v[0], 16);
+#pragma unroll
+        for (int k = 0; k < K - 2; k++) mx[k] = max_pos(0.0, v[2 + k]);
+        warp_totals<K>(sum, mx);
+        if ((lane & 15) == 0) sm[wid * K + (low ? 0 : 1)] = sum;
         if (lane == 0)
 #pragma unroll
-            for (int k = 0; k < 3; k++) sm[wid * 3 + k] = v[k];
+            for (int k = 0; k < K - 2; k++) sm[wid * K + 2 + k] = mx[k];
     }
     __syncthreads();
-    if (threadIdx.x == 0)
-        for (int b = 1; b < nwr; b++) {
-            v[0] += sm[b * 3];
-            v[1] += sm[b * 3 + 1];
-            v[2] = fmax(v[2], sm[b * 3 + 2]);
+    if (t < K) {
+        double a = sm[t];
+        for (int w = 1; w < nwr; w++) a = t < 2 ? a + sm[w * K + t] : max_pos(a, sm[w * K + t]);
+        part[t * nb + blockIdx.x] = a;
+    }
+    if (!grid_bar(ls, bk, 0)) return false;
+    if (wid == 0) {
+        const double *mine = part + (lane < 16 ? 0 : nb);
+        sum = 0.0;
+        for (int b = lane & 15; b < nb; b += 16) sum += mine[b];
+#pragma unroll
+        for (int k = 0; k < K - 2; k++) {
+            mx[k] = 0.0;
+            for (int b = lane; b < nb; b += 32) mx[k] = max_pos(mx[k], part[(2 + k) * nb + b]);
         }
-    __syncthreads();
+        warp_totals<K>(sum, mx);
+        v[1] = __shfl_sync(0xffffffffu, sum, 16);
+        v[0] = sum;
+#pragma unroll
+        for (int k = 0; k < K - 2; k++) v[2 + k] = mx[k];
+    }
+    return true;
 }
 
 // End of a resident loop: the displacement maxima of the last move (zero where
-// a build followed), then the state and the buffer pointers, written by block 0
-// after every block has handed in its own.
-__device__ __forceinline__ void loop_exit(DevSys *ds, DevSys *L, LoopSync *ls, unsigned &bk, Range r,
-                                          double *red) {
+// a build followed), after every block has handed in its own.  True on thread 0
+// of block 0, which then writes its copy of the system back.
+__device__ __forceinline__ bool loop_exit(DevSys *L, LoopSync *ls, unsigned &bk, Range r, double *red) {
     const int t = threadIdx.x, nb = gridDim.x;
     double m[2] = {0.0, 0.0};
     for (int i = r.first + t; i < r.last; i += blockDim.x) {
@@ -297,13 +336,13 @@ __device__ __forceinline__ void loop_exit(DevSys *ds, DevSys *L, LoopSync *ls, u
     }
     const int ops[2] = {1, 1};
     block_reduce<2>(m, ops, red);
-    double *part = L->w.partials + 4 * nb;  // apart from the sums that a slower block may still read
+    double *part = L->w.partials + 5 * nb;  // apart from the sums that a slower block may still read
     if (t == 0) {
         part[blockIdx.x] = m[0];
         part[nb + blockIdx.x] = m[1];
     }
     const bool all = grid_bar(ls, bk, 0) != 0;
-    if (blockIdx.x != 0) return;
+    if (blockIdx.x != 0) return false;
     m[0] = 0.0;
     m[1] = 0.0;
     if (all)
@@ -317,9 +356,8 @@ __device__ __forceinline__ void loop_exit(DevSys *ds, DevSys *L, LoopSync *ls, u
         L->s.max_cd2 = m[1];
         L->s.rebuild = 0;
         if (!all) L->s.flags |= kError;
-        ds->v = L->v;
-        ds->s = L->s;
     }
+    return t == 0;
 }
 
 // ---- one tile per block: a block's particles stay in its registers -----------
@@ -621,22 +659,8 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
                 tot[1] = f.x * u.x + f.y * u.y;
                 tot[2] = f.x * f.x + f.y * f.y;
             }
-            const int nb = gridDim.x;
-            double *part = w.partials;
-            reduce3(tot, (np + 31) / 32, red);
-            if (t == 0)
-#pragma unroll
-                for (int k = 0; k < 3; k++) part[k * nb + blockIdx.x] = tot[k];
-            ok = grid_bar(ls, bk, 0) != 0;
+            ok = grid_totals<3>(tot, (np + 31) / 32, w.partials, ls, bk, red);
             if (!ok) break;
-#pragma unroll
-            for (int k = 0; k < 3; k++) tot[k] = 0.0;
-            for (int b = t; b < nb; b += blockDim.x) {
-                tot[0] += part[b];
-                tot[1] += part[nb + b];
-                tot[2] = fmax(tot[2], part[2 * nb + b]);
-            }
-            reduce3(tot, min(nw, (nb + 31) / 32), red);
             if (t == 0) fire_epilogue<M>(s, tot);
             __syncthreads();
             if (s.flags || it >= iters) break;
@@ -646,7 +670,10 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
         store_own();
         if (mine) w.pe[own] = pe;
     }
-    loop_exit(ds, &L, ls, bk, r, red);
+    if (loop_exit(&L, ls, bk, r, red)) {
+        ds->v = v;
+        ds->s = s;
+    }
 }
 
 // Pair sums of slot i in the loop: FP64 with the queue, or FP32 (M) with G
@@ -815,30 +842,17 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_loop(DevSys *ds, LoopSync *l
             const int kind = rebuild_kind(bw);
             if (kind) ok = loop_rebuild<M>(&L, ls, bk, kind, r);
         } else {
-            // totals: block partials, then every block sums them in block order
-            const int ops[3] = {0, 0, 1};
-            block_reduce<3>(tot, ops, red);
-            const int nb = gridDim.x;
-            double *part = w.partials;
-            if (t == 0)
-#pragma unroll
-                for (int k = 0; k < 3; k++) part[k * nb + blockIdx.x] = tot[k];
-            ok = grid_bar(ls, bk, 0) != 0;
+            ok = grid_totals<3>(tot, nt / 32, w.partials, ls, bk, red);
             if (!ok) break;
-#pragma unroll
-            for (int k = 0; k < 3; k++) tot[k] = 0.0;
-            for (int b = t; b < nb; b += nt) {
-                tot[0] += part[b];
-                tot[1] += part[nb + b];
-                tot[2] = fmax(tot[2], part[2 * nb + b]);
-            }
-            block_reduce<3>(tot, ops, red);
             if (t == 0) fire_epilogue<M>(s, tot);
             __syncthreads();
             if (s.flags || it >= iters) break;
         }
     }
-    loop_exit(ds, &L, ls, bk, r, red);
+    if (loop_exit(&L, ls, bk, r, red)) {
+        ds->v = v;
+        ds->s = s;
+    }
 }
 
 }  // namespace
