@@ -22,6 +22,7 @@ namespace {  // kernels have internal linkage: each translation unit owns its co
 
 struct BumpyExt {
     int nv, capv, rotation, max_vcount;
+    int max_nvb;             // most vertices of a body
     double rv, vcut2, vpcut2;
     double *w, *th, *tq, *I;  // angular velocity, angle, torque, moment of inertia
     int *nvb, *start;
@@ -336,60 +337,75 @@ __global__ void kb_observables(BumpySys *bs) {
 // ---- vertex neighbour list: kernelUpdateVertexNeighborList (kernels.cu:870-922):
 // vertices within the vertex cutoff, over the body's neighbour bodies (those
 // whose centre is within the body cutoff of the vertex) in list order, vertices
-// ascending.  G lanes per vertex: they share first the bodies, then each
-// body's vertices (16 consecutive bytes a lane), ballots give the hits their
-// places.  The fixed-point filter decides all but ~1e-5 of the tests; in FP64
-// the list of 4096 bodies took up to 940 us.  Returns the row's length.  All
-// lanes of the warp call it (real = false past the last vertex).
-template <int G>
-__device__ __forceinline__ int vlist_row(BumpySys *bs, int v, bool real) {
-    constexpr unsigned kAll = 0xffffffffu, kGroup = (1u << G) - 1u;
+// ascending.  A warp takes 32 vertices of a body, one a lane.  For each listed
+// body its lanes first load 32 of that body's vertices side by side and drop
+// those out of reach of every vertex of their own body (triangle inequality
+// over the body's centre); the few that are left go round the warp by shuffles.
+// The fixed-point filter decides all but ~1e-5 of the tests.  `rows`: the
+// warp's listed bodies [t0, t1); cnt: the row's length so far; write: entries
+// are stored.  All lanes of the warp call it with the same body.
+__device__ __forceinline__ void vlist_scan(BumpySys *bs, int b, int v, bool real, uint4 qv, float reach, int t0,
+                                           int t1, bool write, int &cnt) {
+    constexpr unsigned kAll = 0xffffffffu;
     const DevSys &d = bs->b;
     BumpyExt &x = bs->x;
-    const int lane = threadIdx.x & 31, sub = lane & (G - 1), lead = lane - sub;
-    const int nb = d.p.n, nv = x.nv, capv = x.capv;
-    const int b = real ? x.vbody[v] : 0, vv = real ? v : 0;
-    const int ncnt = real ? min(d.w.count[b], d.p.cap) : 0;
-    const uint4 qv = x.vq[vv];
-    int cnt = 0;
-    for (int t0 = 0; __any_sync(kAll, t0 < ncnt); t0 += G) {
-        const int t = t0 + sub;
-        const int ob = t < ncnt ? d.v.nbr[(size_t)t * nb + b] : 0;
-        const bool near = t < ncnt && within(d.p, x.vpos, vv, d.v.pos, ob, qv, d.v.q[ob], x.vpin2, x.vpout2, x.vpcut2);
-        unsigned bodies = (__ballot_sync(kAll, near) >> lead) & kGroup;
-        const int of_l = near ? x.start[ob] : 0, on_l = near ? x.nvb[ob] : 0;
-        while (__any_sync(kAll, bodies != 0)) {
-            const int src = bodies ? __ffs(bodies) - 1 : 0;
-            const int of = __shfl_sync(kAll, of_l, lead + src);
-            const int on_s = __shfl_sync(kAll, on_l, lead + src), on = bodies ? on_s : 0;
-            bodies &= bodies - 1;
-            for (int u0 = 0; __any_sync(kAll, u0 < on); u0 += G) {
-                const int u = of + u0 + sub;
-                const bool hit = u0 + sub < on &&
-                                 within(d.p, x.vpos, vv, x.vpos, u, qv, x.vq[u], x.vin2, x.vout2, x.vcut2);
-                const unsigned m = (__ballot_sync(kAll, hit) >> lead) & kGroup;
-                const int at = cnt + __popc(m & ((1u << sub) - 1u));
-                if (hit && at < capv) x.vnbr[(size_t)at * nv + v] = u;
-                cnt += __popc(m);
+    const DevParams &p = d.p;
+    const int lane = threadIdx.x & 31, nb = p.n, nv = x.nv, capv = x.capv;
+    const uint4 qb = d.v.q[b];
+    for (int t = t0; t < t1; t++) {
+        const int ob = d.v.nbr[(size_t)t * nb + b];
+        const bool near = real && within(p, x.vpos, v, d.v.pos, ob, qv, d.v.q[ob], x.vpin2, x.vpout2, x.vpcut2);
+        if (!__any_sync(kAll, near)) continue;
+        const int of = x.start[ob], on = x.nvb[ob];
+        for (int u0 = 0; u0 < on; u0 += 32) {
+            const bool there = u0 + lane < on;
+            const uint4 qu = x.vq[of + (there ? u0 + lane : 0)];
+            const bool close = there && ((qu.w | qb.w) != 0 || !(quant_d2(p.q_s[0], p.q_s[1], qu, qb) > reach * reach));
+            for (unsigned todo = __ballot_sync(kAll, close); todo; todo &= todo - 1) {
+                const int src = __ffs(todo) - 1, u = of + u0 + src;
+                const uint4 qo = make_uint4(__shfl_sync(kAll, qu.x, src), __shfl_sync(kAll, qu.y, src), 0u,
+                                            __shfl_sync(kAll, qu.w, src));
+                if (near && within(p, x.vpos, v, x.vpos, u, qv, qo, x.vin2, x.vout2, x.vcut2)) {
+                    if (write && cnt < capv) x.vnbr[(size_t)cnt * nv + v] = u;
+                    cnt++;
+                }
             }
         }
     }
-    return cnt;
 }
 
-// Runs only when the body list was rebuilt since the last vertex build.
-constexpr int kVlistLanes = 8;
+// how far from its centre a vertex of another body can be and still be in the
+// row of one of the warp's vertices (real lanes)
+__device__ __forceinline__ float vlist_reach(const BumpySys *bs, uint4 qb, uint4 qv, bool real) {
+    const DevParams &p = bs->b.p;
+    const float d = real ? sqrtf(quant_d2(p.q_s[0], p.q_s[1], qv, qb)) : 0.f;
+    const float most = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(d)));
+    if (__any_sync(0xffffffffu, real && qv.w != 0)) return INFINITY;
+    return (most + sqrtf(bs->x.vout2)) * 1.00001f + 2.f * p.q_tol;
+}
+
+// Runs only when the body list was rebuilt since the last vertex build; a warp
+// a body.
 __global__ void kb_vlist(BumpySys *bs) {
     if (bs->b.s.n_rebuilds == bs->x.vlist_built) return;
     BumpyExt &x = bs->x;
-    const int gid = blockIdx.x * blockDim.x + threadIdx.x, v = gid / kVlistLanes;
-    const bool real = v < x.nv;
-    const int cnt = vlist_row<kVlistLanes>(bs, v, real);
-    if (real && gid % kVlistLanes == 0) {
-        x.vcount[v] = cnt;
-        if (x.mixed) x.vpk[v] = mixed_pack(bs->b.p, x.vpos[v], x.rv);
+    const int lane = threadIdx.x & 31, b = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+    int mx = 0;
+    if (b < bs->b.p.n) {
+        const int f = x.start[b], nvb = x.nvb[b], rows = min(bs->b.w.count[b], bs->b.p.cap);
+        for (int base = 0; base < nvb; base += 32) {
+            const bool real = base + lane < nvb;
+            const int v = f + (real ? base + lane : 0);
+            const uint4 qv = x.vq[v];
+            int cnt = 0;
+            vlist_scan(bs, b, v, real, qv, vlist_reach(bs, bs->b.v.q[b], qv, real), 0, rows, true, cnt);
+            if (!real) continue;
+            x.vcount[v] = cnt;
+            if (x.mixed) x.vpk[v] = mixed_pack(bs->b.p, x.vpos[v], x.rv);
+            mx = max(mx, cnt);
+        }
     }
-    double val[1] = {real ? (double)cnt : 0.0};
+    double val[1] = {(double)mx};
     const int ops[1] = {1};
     if (grid_reduce<1>(val, ops, &bs->b)) {
         int m = (int)val[0];

@@ -42,7 +42,8 @@ struct dpg_bumpy_system {
     double *xfer = nullptr;
     int mode = 2;  // 3 resident grid, 2 graph, 0 separate launches
     LoopSync *lsync = nullptr;          // resident grid: barrier state,
-    int lblocks = 0, lchunk = 0, ltpb = 0;  // blocks, bodies a block, threads a block
+    int lblocks = 0, lchunk = 0;        // blocks, bodies a block
+    int max_nvb = 0;                    // most vertices of a body
     cudaGraphExec_t loop_exec[2] = {nullptr, nullptr};
     cudaGraphConditionalHandle h_loop[2] = {0, 0}, h_rb[2] = {0, 0};
     double loop_dt = 0.0, loop_tmax = 0.0;
@@ -54,7 +55,6 @@ struct dpg_bumpy_system {
     int ngrid() const { return std::max(1, (int)(((long long)nb * nlg + ntpb - 1) / ntpb)); }
     void *nlist_fn() const { return nlg == 8 ? (void *)k_nlist_cell<8> : (void *)k_nlist_cell<1>; }
     int gm() const { return std::max(1, (nb + kMoveBodies - 1) / kMoveBodies); }  // move kernels
-    int gl() const { return (int)(((long long)nv * kVlistLanes + kTPB - 1) / kTPB); }  // vertex list
     int gb(int count) const { return std::max(1, (count + kTPB - 1) / kTPB); }
     int gw(int bodies) const { return std::max(1, (bodies + kWarpsPerBlock - 1) / kWarpsPerBlock); }
     DevSys *ds() const { return &d->b; }
@@ -161,7 +161,7 @@ extern "C" int dpg_bumpy_create(const dpg_bumpy_params *p, void *cuda_stream, dp
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     s->nlg = (long long)s->nb < (long long)nsm * 1024 ? 8 : 1;
     s->ntpb = (long long)s->nb * s->nlg < (long long)nsm * 2 * kTPB ? 64 : kTPB;
-    w.max_blocks = std::max(std::max(std::max(s->gb(s->nb), s->gw(s->nb)), s->ngrid()), s->gl());
+    w.max_blocks = std::max(std::max(s->gb(s->nb), s->gw(s->nb)), s->ngrid());
     w.max_blocks = std::max(w.max_blocks, nsm);
     A((void **)&w.partials, (size_t)w.max_blocks * 8 * 8);
     A((void **)&x.w, nb * 8); A((void **)&x.th, nb * 8); A((void **)&x.tq, nb * 8); A((void **)&x.I, nb * 8);
@@ -255,6 +255,8 @@ extern "C" int dpg_bumpy_set_bodies(dpg_bumpy_handle s, const double *x, const d
     }
     if (tot != s->nv) return set_err(DPG_ERR_ARG, "vertex counts sum to %lld, expected %d", tot, s->nv);
     TRY(reset_views(s));
+    s->max_nvb = *std::max_element(nvb, nvb + s->nb);
+    TRY(put(s, &s->d->x.max_nvb, s->max_nvb));
     // bodies are still in input order here (no cell sort yet): plain copies
     std::vector<double> zeros(s->nb, 0.0);
     std::vector<double2> buf(s->nb);
@@ -433,7 +435,7 @@ static int enqueue_rebuild(BS *s) {
         LAUNCH(k_nlist_all, s->gb(s->nb), kTPB, ds);
     }
     LAUNCH(kb_vquant_rebuild, s->gb(s->nv), kTPB, s->d);
-    LAUNCH(kb_vlist, s->gl(), kTPB, s->d);
+    LAUNCH(kb_vlist, s->gw(s->nb), kTPB, s->d);
     return DPG_OK;
 }
 
@@ -481,7 +483,7 @@ static int resolve_overflow(BS *s) {
             TRY(put(s, &s->d->x.vlist_built, s->hs->n_rebuilds - 1));
         }
         LAUNCH(kb_vquant_rebuild, s->gb(s->nv), kTPB, s->d);
-        LAUNCH(kb_vlist, s->gl(), kTPB, s->d);
+        LAUNCH(kb_vlist, s->gw(s->nb), kTPB, s->d);
     }
     return set_err(DPG_ERR_OVERFLOW, "neighbour capacity did not settle");
 }
@@ -746,7 +748,7 @@ static int build_graph(BS *s, int kind) {
             prev = addk(ib, prev, (void *)k_nlist_all, GB, kTPB, a_d, &err);
         }
         prev = addk(ib, prev, (void *)kb_vquant_rebuild, s->gb(s->nv), kTPB, a_b, &err);
-        prev = addk(ib, prev, (void *)kb_vlist, s->gl(), kTPB, a_b, &err);
+        prev = addk(ib, prev, (void *)kb_vlist, s->gw(s->nb), kTPB, a_b, &err);
         last = kind == 0 ? addk(body, inode, (void *)kb_fire_force, GW, kTPB, a_ff, &err)
                          : addk(body, inode, (void *)kb_nve_second, GW, kTPB, a_n2, &err);
         last = addk(body, last, (void *)k_loop_guard, 1, 1, a_d, &err);
@@ -762,8 +764,9 @@ static int build_graph(BS *s, int kind) {
     return DPG_OK;
 }
 
-// The resident grid: a block an SM, its bodies' forces a warp a body.  Above
-// kLoopBodies bodies a block the loops stay graphs of full-size kernels.
+// The resident grid: a block an SM.  It holds at most kLoopBodies bodies,
+// kBodyVerts vertices and list rows of kVertSlots; larger systems run the
+// loops as graphs of full-size kernels.
 static int plan_resident(BS *s) {
     int dev = 0, nsm = 0, coop = 0;
     CK(cudaGetDevice(&dev));
@@ -771,14 +774,10 @@ static int plan_resident(BS *s) {
     CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     const int per = (s->nb + nsm - 1) / nsm;
     if (!coop || per > kLoopBodies) return set_err(DPG_ERR_STATE, "no resident loop for this system");
-    // at least 8 warps for the list builds, at most a warp a body beyond that
-    s->ltpb = std::min(kLoopMaxTPB, std::max(256, 32 * per));
     for (void *fn : {(void *)kb_loop<0>, (void *)kb_loop<1>}) {
         int occ = 0;
-        // the attribute is the function's, whichever system launches it: the largest block's
-        CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(sizeof(ForceWarp) * (kLoopMaxTPB / 32))));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, s->ltpb, sizeof(ForceWarp) * (s->ltpb / 32)));
+        CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BodyMem)));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kLoopMaxTPB, sizeof(BodyMem)));
         if (occ < 1) return set_err(DPG_ERR_CUDA, "the resident loop does not fit an SM");
     }
     s->lchunk = per;
@@ -786,15 +785,20 @@ static int plan_resident(BS *s) {
     return DPG_OK;
 }
 
+static bool resident_holds(const BS *s) {
+    return s->capv <= kVertSlots && (long long)s->lchunk * s->max_nvb <= kBodyVerts;
+}
+
 static int run_resident(BS *s, int kind) {
     void *fn = kind == 0 ? (void *)kb_loop<0> : (void *)kb_loop<1>;
     long long most = std::max<long long>(256, (1LL << 24) / (s->nb + 1024));
     double dt = s->loop_dt, tmax = s->loop_tmax;
     void *args[] = {(void *)&s->d, (void *)&s->lsync, (void *)&dt, (void *)&tmax, (void *)&s->lchunk, (void *)&most};
+    // 8 warps for the roles and the list builds, more where the vertices fill them
+    const int threads = (long long)s->lchunk * s->max_nvb > 256 ? kLoopMaxTPB : 256;
     do {
         CK(cudaMemsetAsync(s->lsync, 0, sizeof(LoopSync), s->stream));
-        CK(cudaLaunchCooperativeKernel(fn, dim3(s->lblocks), dim3(s->ltpb), args,
-                                       sizeof(ForceWarp) * (s->ltpb / 32), s->stream));
+        CK(cudaLaunchCooperativeKernel(fn, dim3(s->lblocks), dim3(threads), args, sizeof(BodyMem), s->stream));
         TRY(pull(s));
         if (s->hs->flags & kError) return set_err(DPG_ERR_TIMEOUT, "a grid barrier of the resident loop ran out");
     } while (!s->hs->flags);
@@ -804,17 +808,16 @@ static int run_resident(BS *s, int kind) {
 static int run_loop(BS *s, int kind, int *ovf) {
     *ovf = 0;
     TRY(vrefresh(s));
-    if (s->mode == 3) {
-        if (!s->lblocks && plan_resident(s) != DPG_OK) {
-            (void)cudaGetLastError();
-            s->mode = 2;
-        } else {
-            TRY(run_resident(s, kind));
-            if (s->hs->flags & kOverflow) *ovf = 1;
-            return DPG_OK;
-        }
+    if (s->mode == 3 && !s->lblocks && plan_resident(s) != DPG_OK) {
+        (void)cudaGetLastError();
+        s->mode = 2;
     }
-    if (s->mode == 2) {
+    if (s->mode == 3 && resident_holds(s)) {
+        TRY(run_resident(s, kind));
+        if (s->hs->flags & kOverflow) *ovf = 1;
+        return DPG_OK;
+    }
+    if (s->mode >= 2) {
         if (build_graph(s, kind) != DPG_OK) {
             s->mode = 0;
         } else {

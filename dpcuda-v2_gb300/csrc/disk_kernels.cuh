@@ -97,6 +97,33 @@ __device__ __forceinline__ PairArgs pair_args(const DevSys *ds) {
             ds->p.n_c, ds->p.q_l4[0], ds->p.q_l4[1], ds->p.q_s[0], ds->p.q_s[1], ds->p.q_tol, 0.0};
 }
 
+// The terms of a contact from its displacement, for radius sum rs, its square
+// and its reciprocal rounded to nearest (0: none kept; the quotient is the same
+// either way).  sure: the fixed-point distance has already decided that the two
+// touch.  disk_pair's arithmetic.
+__device__ __forceinline__ double contact_terms(double dx, double dy, double rs, double rs2, double inv,
+                                                bool sure, double e_c, double n_c, double &fx, double &fy) {
+    const double d2 = dx * dx + dy * dy;
+    fx = 0.0;
+    fy = 0.0;
+    if (!sure && d2 >= rs2) return 0.0;
+    const double d = sqrt(d2);
+    // (no quotient near the end of the range: |d| above 2^-300, 1e-15 < rs < 1e16)
+    const bool quick = inv != 0.0 && (unsigned)__double2hiint(d) > 0x2d300000u;
+    const double ov = 1.0 - (quick ? div_by(d, rs, inv) : d / rs);
+    double ovp = ov, energy;
+    if (n_c == 2.0) {  // pow(ov, 1) == ov, and x / 4 == x * 0.25 exactly
+        energy = e_c == 1.0 ? ov * ov * 0.25 : e_c * ov * ovp * 0.25;
+    } else {
+        ovp = pow(ov, n_c - 1);
+        energy = e_c * ov * ovp / (2.0 * n_c);
+    }
+    const double fm = (e_c == 1.0 ? ovp : e_c * ovp) / (rs * d);
+    fx = fm * dx;
+    fy = fm * dy;
+    return energy;
+}
+
 // disk_pair for the sums (see pbc_dist_sum)
 __device__ __forceinline__ double disk_pair_sum(const PairArgs &f, double2 pi, double ri, double2 pj,
                                                 double rj, double &dx, double &dy, double &fx,

@@ -429,7 +429,8 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
     long long it = 0;
 
     double2 x = {0.0, 0.0}, u = {0.0, 0.0}, f = {0.0, 0.0}, xn = {0.0, 0.0}, xc = {0.0, 0.0};
-    double mass = 1.0, rad = 0.0, pe = 0.0, dtm = 0.0, dtm_of = -1.0;
+    double mass = 1.0, rad = 0.0, pe = 0.0, dtm = 0.0, dtm_of = 0.0;
+    bool dtm_known = false;
     int gcnt = 0;  // row length of the group's particle
     auto load_own = [&]() {
         if (mine) {
@@ -437,7 +438,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
             xn = w.pos_n[own]; xc = w.pos_c[own];
             mass = v.mass[own]; rad = v.rad[own];
         }
-        dtm_of = -1.0;
+        dtm_known = false;
         gcnt = g < np ? min(w.count[r.first + g], p.cap) : 0;
         for (int k = sub; k < gcnt; k += G) {
             const int j = v.nbr[(size_t)k * n + r.first + g];
@@ -454,9 +455,10 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
     };
     // (h / mass), kept while h is the same
     auto kick_factor = [&](double h) {
-        if (h != dtm_of) {
+        if (!dtm_known || h != dtm_of) {
             dtm = h / mass;
             dtm_of = h;
+            dtm_known = true;
         }
         return dtm;
     };
