@@ -352,22 +352,38 @@ __device__ __forceinline__ void vlist_scan(BumpySys *bs, int b, int v, bool real
     const DevParams &p = d.p;
     const int lane = threadIdx.x & 31, nb = p.n, nv = x.nv, capv = x.capv;
     const uint4 qb = d.v.q[b];
-    for (int t = t0; t < t1; t++) {
-        const int ob = d.v.nbr[(size_t)t * nb + b];
-        const bool near = real && within(p, x.vpos, v, d.v.pos, ob, qv, d.v.q[ob], x.vpin2, x.vpout2, x.vpcut2);
-        if (!__any_sync(kAll, near)) continue;
-        const int of = x.start[ob], on = x.nvb[ob];
-        for (int u0 = 0; u0 < on; u0 += 32) {
-            const bool there = u0 + lane < on;
-            const uint4 qu = x.vq[of + (there ? u0 + lane : 0)];
-            const bool close = there && ((qu.w | qb.w) != 0 || !(quant_d2(p.q_s[0], p.q_s[1], qu, qb) > reach * reach));
-            for (unsigned todo = __ballot_sync(kAll, close); todo; todo &= todo - 1) {
-                const int src = __ffs(todo) - 1, u = of + u0 + src;
-                const uint4 qo = make_uint4(__shfl_sync(kAll, qu.x, src), __shfl_sync(kAll, qu.y, src), 0u,
-                                            __shfl_sync(kAll, qu.w, src));
-                if (near && within(p, x.vpos, v, x.vpos, u, qv, qo, x.vin2, x.vout2, x.vcut2)) {
-                    if (write && cnt < capv) x.vnbr[(size_t)cnt * nv + v] = u;
-                    cnt++;
+    for (int r0 = t0; r0 < t1; r0 += 32) {
+        // the listed bodies, one a lane: all their loads in flight together, and
+        // the next body's vertices while this one's are tested
+        const int rows = min(32, t1 - r0);
+        const int ob_l = lane < rows ? d.v.nbr[(size_t)(r0 + lane) * nb + b] : 0;
+        const uint4 q_l = d.v.q[ob_l];
+        const int of_l = x.start[ob_l], on_l = x.nvb[ob_l];
+        auto vertex_of = [&](int r) {
+            const int of = __shfl_sync(kAll, of_l, r), on = __shfl_sync(kAll, on_l, r);
+            return x.vq[of + (lane < on ? lane : 0)];
+        };
+        uint4 next = vertex_of(0);
+        for (int r = 0; r < rows; r++) {
+            const int ob = __shfl_sync(kAll, ob_l, r), of = __shfl_sync(kAll, of_l, r), on = __shfl_sync(kAll, on_l, r);
+            const uint4 qo = make_uint4(__shfl_sync(kAll, q_l.x, r), __shfl_sync(kAll, q_l.y, r), 0u,
+                                        __shfl_sync(kAll, q_l.w, r));
+            uint4 qu = next;
+            if (r + 1 < rows) next = vertex_of(r + 1);
+            const bool near = real && within(p, x.vpos, v, d.v.pos, ob, qv, qo, x.vpin2, x.vpout2, x.vpcut2);
+            if (!__any_sync(kAll, near)) continue;
+            for (int u0 = 0; u0 < on; u0 += 32) {
+                const bool there = u0 + lane < on;
+                if (u0) qu = x.vq[of + (there ? u0 + lane : 0)];
+                const bool close = there && ((qu.w | qb.w) != 0 || !(quant_d2(p.q_s[0], p.q_s[1], qu, qb) > reach * reach));
+                for (unsigned todo = __ballot_sync(kAll, close); todo; todo &= todo - 1) {
+                    const int src = __ffs(todo) - 1, u = of + u0 + src;
+                    const uint4 qw = make_uint4(__shfl_sync(kAll, qu.x, src), __shfl_sync(kAll, qu.y, src), 0u,
+                                                __shfl_sync(kAll, qu.w, src));
+                    if (near && within(p, x.vpos, v, x.vpos, u, qv, qw, x.vin2, x.vout2, x.vcut2)) {
+                        if (write && cnt < capv) x.vnbr[(size_t)cnt * nv + v] = u;
+                        cnt++;
+                    }
                 }
             }
         }
@@ -651,20 +667,12 @@ __device__ __forceinline__ void bumpy_fire_epilogue(BumpySys *bs, const double (
     s.power = v[1];
     s.fmax2 = v[2];
     bs->x.tmax2 = v[3];
-    double avg = v[0] / s.dof;
-    const bool pe_still = s.pe_diff_target > 0 && fabs(avg / s.last_avg_pe - 1) < s.pe_diff_target;
-    s.last_avg_pe = avg;
+    double avg;
+    const bool pe_still = fire_energy(s, avg);
     long long it = s.iter;
     // mixed form: FP32 vertex pairs until the switch (as k_fire_force), then FP64
-    bool fp64 = true;
-    if (bs->x.mixed && !s.fp64_now) {
-        double g2 = fmax(v[2], v[3]);
-        if (g2 < 0.81 * s.best_f2) { s.best_f2 = g2; s.best_it = it; }
-        const double gm = sqrt(g2);
-        if (gm <= s.switch_fmax || s.f_nbad > 5 || (gm < 100.0 * s.switch_fmax && it - s.best_it > 2000))
-            s.fp64_now = 1;
-        fp64 = false;
-    }
+    const bool fp64 = !bs->x.mixed || s.fp64_now;
+    if (!fp64) fire_switch(s, max_pos(v[2], v[3]));
     if ((fp64 && pe_still) || avg < s.pe_target) {
         s.result_step = it; s.f_converged = 1; s.flags |= kDone; return;
     }

@@ -148,9 +148,10 @@ __device__ __forceinline__ bool bumpy_rebuild(BumpySys *bs, LoopSync *ls, unsign
 //  - the vertex pairs that the filter lets through form one queue per block,
 //    evaluated on full warps; only the vertices that have a term compute a
 //    torque and enter the body sums (in vertex order, one thread a sum).
-constexpr int kBodyVerts = 2048;  // vertices per block at most
-constexpr int kVertQueue = 2048;  // queued vertex pairs evaluated at a time
+constexpr int kBodyVerts = 1536;  // vertices per block at most
 constexpr int kVertSlots = 32;    // vertex-list capacity at most
+constexpr int kVertRows = 6144;   // list entries kept on chip (more are read from memory)
+constexpr int kVertQueue = 2048;  // queued vertex pairs evaluated at a time
 
 struct BodyMem {
     double2 vpos[kBodyVerts];           // current vertex positions
@@ -159,14 +160,43 @@ struct BodyMem {
     double2 p[kLoopBodies], n[kLoopBodies], cs[kLoopBodies];  // a move: from, to, cosine and sine
     double sum[4][kLoopBodies];         // force x, force y, torque, energy
     double xa[4][kLoopBodies], xb[4][kLoopBodies];  // exchanged between the roles
-    int ej[kVertQueue];                 // queue: other vertex,
-    unsigned ent[kVertQueue];           //        vertex << 6 | sure << 5 | slot
-    int off[kBodyVerts + 1];            // first queue entry of each term vertex
-    unsigned short tv[kBodyVerts];      // its vertex
+    // the vertex rows of the block as one list: entry e belongs to vertex k for
+    // row[k] <= e < row[k + 1]
+    int row[kBodyVerts + 1];
+    int other[kVertRows];               // the other vertex
+    unsigned short of[kVertRows];       // k
+    // a force pass: which entries touch (bit e), which certainly do, and how
+    // many touch before each word: the queue position of entry e is rank(e)
+    unsigned touch[kBodyVerts + 1], sure[kBodyVerts];
+    int count[kBodyVerts], before[kBodyVerts + 1];
+    unsigned short ent[kVertQueue];     // entry at each queue position
+    unsigned vmask[kBodyVerts / 32];    // vertices that have a term
+    unsigned short tv[kBodyVerts];      // the term vertices
     int first[kLoopBodies + 1];         // first term vertex of each body
     int vfirst[kLoopBodies + 1];        // first vertex of each body (block-local)
     unsigned char vb[kBodyVerts];       // body of each vertex (block-local)
+    __device__ __forceinline__ int rank(int e) const {
+        return before[e >> 5] + __popc(touch[e >> 5] & ((1u << (e & 31)) - 1u));
+    }
 };
+
+// vertex and other vertex of entry e: from the chip, or by a search of the rows
+// and a load
+__device__ __forceinline__ void entry_of(const BodyMem &m, const BumpySys &L, int nv, int v0, int e, int &k, int &j) {
+    if (m.row[nv] <= kVertRows) {
+        k = m.of[e];
+        j = m.other[e];
+        return;
+    }
+    int lo = 0, hi = nv;  // row[lo] <= e < row[hi]
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (m.row[mid] <= e) lo = mid;
+        else hi = mid;
+    }
+    k = lo;
+    j = L.x.vnbr[(size_t)(e - m.row[k]) * L.x.nv + v0 + k];
+}
 
 // vertex contact: disk_pair_sum with one radius sum, its square and its reciprocal
 struct VertConst {
@@ -178,50 +208,6 @@ __device__ __forceinline__ double vertex_pair(const PairArgs &f, const VertConst
     return contact_terms(dx, dy, c.rs, c.rs2, c.inv, sure, f.e_c, f.n_c, fx, fy);
 }
 
-// The queue in windows, for a block with more contacts than the queue holds
-// (far above any packing): the entries are found again from the lists, each
-// window's terms added to the term vertices in order.
-__device__ __noinline__ void vertex_windows(BodyMem &m, const BumpySys &L, const PairArgs &fa,
-                                            const VertConst &vc, int terms, int entries, int v0) {
-    const int t = threadIdx.x, nt = blockDim.x;
-    for (int q = t; q < terms; q += nt) m.term[0][q] = m.term[1][q] = m.term[3][q] = 0.0;
-    for (int w0 = 0; w0 < entries; w0 += kVertQueue) {
-        const int w1 = min(entries, w0 + kVertQueue);
-        __syncthreads();
-        for (int q = t; q < terms; q += nt) {
-            if (m.off[q + 1] <= w0 || m.off[q] >= w1) continue;
-            const int k = m.tv[q], vg = v0 + k, cnt = min(L.x.vcount[vg], L.x.capv);
-            const uint4 qi = L.x.vq[vg];
-            int at = m.off[q];
-            for (int c = 0; c < cnt; c++) {
-                const int j = L.x.vnbr[(size_t)c * fa.n + vg];
-                if (!quant_contact(fa.sx, fa.sy, fa.tol, qi, L.x.vq[j])) continue;
-                if (at >= w0 && at < w1) {
-                    m.ent[at - w0] = (unsigned)k << 6 | (unsigned)c;
-                    m.ej[at - w0] = j;
-                }
-                at++;
-            }
-        }
-        __syncthreads();
-        for (int e = t; e < w1 - w0; e += nt) {
-            double fx, fy;
-            const double ee = vertex_pair(fa, vc, false, m.vpos[m.ent[e] >> 6], fa.pos[m.ej[e]], fx, fy);
-            m.res[0][e] = fx;
-            m.res[1][e] = fy;
-            m.res[2][e] = ee;
-        }
-        __syncthreads();
-        for (int q = t; q < terms; q += nt)
-            for (int e = max(m.off[q], w0); e < min(m.off[q + 1], w1); e++) {
-                m.term[0][q] += m.res[0][e - w0];
-                m.term[1][q] += m.res[1][e - w0];
-                m.term[3][q] += m.res[2][e - w0];
-            }
-    }
-    __syncthreads();
-}
-
 template <int KIND>
 __global__ void __launch_bounds__(kLoopMaxTPB, 1) kb_loop(BumpySys *bs, LoopSync *ls, double dt, double tmax,
                                                          int chunk, long long iters) {
@@ -229,7 +215,6 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) kb_loop(BumpySys *bs, LoopSync
     BodyMem &m = *reinterpret_cast<BodyMem *>(loop_smem);
     __shared__ BumpySys L;
     __shared__ double red[32 * 4];
-    __shared__ int wtot[kLoopMaxTPB / 32];
     const int t = threadIdx.x, nt = blockDim.x, lane = t & 31, wid = t >> 5, nw = nt >> 5;
     if (t == 0) L = *bs;
     __syncthreads();
@@ -275,9 +260,19 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) kb_loop(BumpySys *bs, LoopSync
         for (int k = t; k < nv; k += nt) {
             m.vpos[k] = x.vpos[v0 + k];
             m.vb[k] = (unsigned char)(x.vbody[v0 + k] - r.first);
+            m.count[k] = min(x.vcount[v0 + k], x.capv);
         }
         if (t < np) m.vfirst[t] = x.start[r.first + t] - v0;
         if (t == 0) m.vfirst[np] = nv;
+        __syncthreads();
+        cell_scan_block(m.count, m.row, nv);
+        __syncthreads();
+        if (m.row[nv] <= kVertRows)
+            for (int k = t; k < nv; k += nt)
+                for (int q = 0; q < m.count[k]; q++) {
+                    m.other[m.row[k] + q] = x.vnbr[(size_t)q * x.nv + v0 + k];
+                    m.of[m.row[k] + q] = (unsigned short)k;
+                }
         __syncthreads();
     };
     auto store_own = [&]() {
@@ -396,131 +391,149 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) kb_loop(BumpySys *bs, LoopSync
         const bool walls = KIND == 1 && s.walls != 0;
         const bool fp32 = x.mixed && !s.fp64_now;
         const PairArgs fa = vertex_args(&L);
-        int entries = 0, terms = 0;  // queue entries and term vertices before this tile
-        for (int k0 = 0; k0 < nv; k0 += nt) {
-            const int k = k0 + t, vg = v0 + k;
-            const bool real = k < nv;
-            const int cnt = real ? min(x.vcount[vg], x.capv) : 0;
-            unsigned bits = 0, sure = 0;
-            double ax = 0.0, ay = 0.0, en = 0.0;
+        const int rows = nv > 0 ? m.row[nv] : 0, words = (rows + 31) / 32;
+        const float e_cf = (float)p.e_c, n_cf = (float)p.n_c;
+        // which entries touch: a word a warp, four words in flight
+        for (int w0 = wid; w0 < words; w0 += 4 * nw) {
+            int k[4], j[4];
+            bool on[4];
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                const int e = (w0 + c * nw) * 32 + lane;
+                on[c] = e < rows;
+                k[c] = 0;
+                j[c] = v0;
+                if (on[c]) entry_of(m, L, nv, v0, e, k[c], j[c]);
+            }
+            int hit[4] = {0, 0, 0, 0};
             if (fp32) {
-                if (real) {
-                    const float4 pa = x.vpk[vg];
-                    const float e_c = (float)p.e_c, n_c = (float)p.n_c;
-                    float sx = 0.f, sy = 0.f, se = 0.f;
-                    for (int q = 0; q < cnt; q++) {
-                        float fx, fy;
-                        se += mixed_pair(p, pa, x.vpk[x.vnbr[(size_t)q * fa.n + vg]], e_c, n_c, fx, fy);
-                        sx += fx;
-                        sy += fy;
-                    }
-                    ax = (double)sx;
-                    ay = (double)sy;
-                    en = (double)se;
+                float4 o[4];
+#pragma unroll
+                for (int c = 0; c < 4; c++) o[c] = x.vpk[j[c]];
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    float fx, fy;
+                    const float e = mixed_pair(p, x.vpk[v0 + k[c]], o[c], e_cf, n_cf, fx, fy);
+                    hit[c] = on[c] && (e != 0.f || fx != 0.f || fy != 0.f);
                 }
             } else {
-                const uint4 qi = x.vq[real ? vg : v0];
-                for (int q0 = 0; q0 < cnt; q0 += 4) {
-                    int j[4];
-                    uint4 qj[4];
+                uint4 o[4];
 #pragma unroll
-                    for (int c = 0; c < 4; c++) j[c] = q0 + c < cnt ? x.vnbr[(size_t)(q0 + c) * fa.n + vg] : vg;
+                for (int c = 0; c < 4; c++) o[c] = x.vq[j[c]];
 #pragma unroll
-                    for (int c = 0; c < 4; c++) qj[c] = x.vq[j[c]];
-#pragma unroll
-                    for (int c = 0; c < 4; c++) {
-                        if (q0 + c >= cnt) break;
-                        const int hit = quant_contact(fa.sx, fa.sy, fa.tol, qi, qj[c]);
-                        if (hit) {
-                            bits |= 1u << (q0 + c);
-                            asm volatile("prefetch.global.L1 [%0];" ::"l"(x.vpos + j[c]));
-                        }
-                        if (hit == 2) sure |= 1u << (q0 + c);
-                    }
+                for (int c = 0; c < 4; c++) {
+                    if (on[c]) hit[c] = quant_contact(fa.sx, fa.sy, fa.tol, x.vq[v0 + k[c]], o[c]);
+                    if (hit[c]) asm volatile("prefetch.global.L1 [%0];" ::"l"(x.vpos + j[c]));
                 }
             }
-            // places in the queue and among the term vertices: one block scan of both
-            const bool some = real && (walls || bits != 0 || ax != 0.0 || ay != 0.0 || en != 0.0);
-            const int c = __popc(bits);
-            int incl = c | (some ? 1 << 16 : 0);
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += y;
-            }
-            if (lane == 31) wtot[wid] = incl;
-            __syncthreads();
-            const int w_l = lane < nw ? wtot[lane] : 0;
-            const int before = (int)__reduce_add_sync(0xffffffffu, (unsigned)(lane < wid ? w_l : 0));
-            const int tile = (int)__reduce_add_sync(0xffffffffu, (unsigned)w_l);
-            const int ex = incl + before - (c | (some ? 1 << 16 : 0));
-            const int off = entries + (ex & 0xffff), rank = terms + (ex >> 16);
-            if (real && m.vfirst[m.vb[k]] == k) m.first[m.vb[k]] = rank;
-            if (some) {
-                m.tv[rank] = (unsigned short)k;
-                m.off[rank] = off;
-                if (fp32) {
-                    m.term[0][rank] = ax;
-                    m.term[1][rank] = ay;
-                    m.term[3][rank] = en;
+            for (int c = 0; c < 4; c++) {
+                if (w0 + c * nw >= words) break;
+                const unsigned any = __ballot_sync(0xffffffffu, hit[c] != 0), both = __ballot_sync(0xffffffffu, hit[c] == 2);
+                if (lane == 0) {
+                    m.touch[w0 + c * nw] = any;
+                    m.sure[w0 + c * nw] = both;
+                    m.count[w0 + c * nw] = __popc(any);
                 }
             }
-            // entries past the queue's end are queued again window by window below
-            int at = off;
-            for (unsigned b = bits; b; b &= b - 1, at++) {
-                const int q = __ffs(b) - 1;
-                if (at >= kVertQueue) break;
-                m.ent[at] = (unsigned)k << 6 | (sure >> q & 1u) << 5 | (unsigned)q;
-                m.ej[at] = x.vnbr[(size_t)q * fa.n + vg];
-            }
-            entries += tile & 0xffff;
-            terms += tile >> 16;
-            __syncthreads();  // wtot is rewritten by the next tile
-        }
-        if (t == 0) {
-            m.off[terms] = entries;
-            m.first[np] = terms;
         }
         __syncthreads();
-        if (entries > kVertQueue) {  // the same on every thread: too many at once
-            vertex_windows(m, L, fa, vc, terms, entries, v0);
-        } else if (!fp32) {
-            for (int e = t; e < entries; e += nt) {
-                const unsigned ent = m.ent[e];
-                double fx, fy;
-                const double ee = vertex_pair(fa, vc, ent >> 5 & 1u, m.vpos[ent >> 6], fa.pos[m.ej[e]], fx, fy);
-                m.res[0][e] = fx;
-                m.res[1][e] = fy;
-                m.res[2][e] = ee;
+        cell_scan_block(m.count, m.before, words);
+        if (t == 0 && (rows & 31) == 0) m.touch[words] = 0;  // rank(rows) reads this word
+        __syncthreads();
+        const int entries = m.before[words];
+        // the vertices that have a term
+        const int vwords = (nv + 31) / 32;
+        for (int w = wid; w < vwords; w += nw) {
+            const int k = w * 32 + lane;
+            const bool some = k < nv && (walls || m.rank(m.row[k + 1]) > m.rank(m.row[k]));
+            const unsigned b = __ballot_sync(0xffffffffu, some);
+            if (lane == 0) m.vmask[w] = b;
+        }
+        // evaluate the queue, a window at a time (one, but far above any packing)
+        for (int q0 = 0; q0 < entries || q0 == 0; q0 += kVertQueue) {
+            const int q1 = min(entries, q0 + kVertQueue);
+            for (int w = wid; w < words; w += nw) {
+                const int at = m.before[w] + __popc(m.touch[w] & ((1u << lane) - 1u)) - q0;
+                if ((m.touch[w] >> lane & 1u) && at >= 0 && at < kVertQueue) m.ent[at] = (unsigned short)(w * 32 + lane);
             }
             __syncthreads();
-        }
-        for (int q = t; q < terms; q += nt) {
-            double ax = 0.0, ay = 0.0, en = 0.0;
-            if (fp32 || entries > kVertQueue) {
-                ax = m.term[0][q]; ay = m.term[1][q]; en = m.term[3][q];
-            } else {
-                for (int e = m.off[q]; e < m.off[q + 1]; e++) {
-                    ax += m.res[0][e];
-                    ay += m.res[1][e];
-                    en += m.res[2][e];
+            if (q0 == 0) {  // the term vertices, their bodies' first
+                for (int w = wid; w < vwords; w += nw) {
+                    const int pre = (int)__reduce_add_sync(0xffffffffu, (unsigned)((lane < w ? __popc(m.vmask[lane]) : 0) +
+                                                                                  (lane + 32 < w ? __popc(m.vmask[lane + 32]) : 0)));
+                    const int k = w * 32 + lane, at = pre + __popc(m.vmask[w] & ((1u << lane) - 1u));
+                    if (m.vmask[w] >> lane & 1u) m.tv[at] = (unsigned short)k;
+                    if (k < nv && m.vfirst[m.vb[k]] == k) m.first[m.vb[k]] = at;
+                    if (k == nv - 1) m.first[np] = at + (m.vmask[w] >> lane & 1u);
                 }
             }
-            const int k = m.tv[q], b = m.vb[k];
-            const double2 c = m.n[b], pv = m.vpos[k];
-            double t0 = torque_of(ax, ay, pv.x, pv.y, c.x, c.y);
-            if (walls) {
-                double wx, wy;
-                const double we = wall_force(p, pv, rv, wx, wy);
-                t0 = (0.0 + torque_of(wx, wy, pv.x, pv.y, c.x, c.y)) + t0;
-                ax = (0.0 + wx) + ax;
-                ay = (0.0 + wy) + ay;
-                en = (0.0 + we) + en;
+            for (int q = t; q < q1 - q0; q += nt) {
+                const int e = m.ent[q];
+                int k, j;
+                entry_of(m, L, nv, v0, e, k, j);
+                if (fp32) {
+                    float *rf = reinterpret_cast<float *>(&m.res[0][0]);
+                    float fx, fy;
+                    rf[2 * kVertQueue + q] = mixed_pair(p, x.vpk[v0 + k], x.vpk[j], e_cf, n_cf, fx, fy);
+                    rf[q] = fx;
+                    rf[kVertQueue + q] = fy;
+                } else {
+                    double fx, fy;
+                    const double ee = vertex_pair(fa, vc, m.sure[e >> 5] >> (e & 31) & 1u, m.vpos[k], fa.pos[j], fx, fy);
+                    m.res[0][q] = fx;
+                    m.res[1][q] = fy;
+                    m.res[2][q] = ee;
+                }
             }
-            m.term[0][q] = ax;
-            m.term[1][q] = ay;
-            m.term[2][q] = t0;
-            m.term[3][q] = en;
+            __syncthreads();
+            const int terms = np > 0 ? m.first[np] : 0;
+            for (int q = t; q < terms; q += nt) {
+                const int k = m.tv[q], a0 = m.rank(m.row[k]), a1 = m.rank(m.row[k + 1]);
+                const int b0 = max(a0, q0), b1 = min(a1, q1);
+                double ax = 0.0, ay = 0.0, en = 0.0;
+                if (fp32) {
+                    const float *rf = reinterpret_cast<const float *>(&m.res[0][0]);
+                    float sx = 0.f, sy = 0.f, se = 0.f;
+                    if (a0 < q0 && b0 < b1) {  // carried over from the window before
+                        sx = (float)m.term[0][q]; sy = (float)m.term[1][q]; se = (float)m.term[3][q];
+                    }
+                    for (int e = b0; e < b1; e++) {
+                        sx += rf[e - q0];
+                        sy += rf[kVertQueue + e - q0];
+                        se += rf[2 * kVertQueue + e - q0];
+                    }
+                    ax = (double)sx; ay = (double)sy; en = (double)se;
+                } else {
+                    if (a0 < q0 && b0 < b1) { ax = m.term[0][q]; ay = m.term[1][q]; en = m.term[3][q]; }
+                    for (int e = b0; e < b1; e++) {
+                        ax += m.res[0][e - q0];
+                        ay += m.res[1][e - q0];
+                        en += m.res[2][e - q0];
+                    }
+                }
+                if (a1 > q1) {  // goes on in the next window
+                    if (b0 < b1) { m.term[0][q] = ax; m.term[1][q] = ay; m.term[3][q] = en; }
+                    continue;
+                }
+                if (a1 <= q0 && q0 > 0) continue;  // done in an earlier window
+                const int b = m.vb[k];
+                const double2 c = m.n[b], pv = m.vpos[k];
+                double t0 = torque_of(ax, ay, pv.x, pv.y, c.x, c.y);
+                if (walls) {
+                    double wx, wy;
+                    const double we = wall_force(p, pv, rv, wx, wy);
+                    t0 = (0.0 + torque_of(wx, wy, pv.x, pv.y, c.x, c.y)) + t0;
+                    ax = (0.0 + wx) + ax;
+                    ay = (0.0 + wy) + ay;
+                    en = (0.0 + we) + en;
+                }
+                m.term[0][q] = ax;
+                m.term[1][q] = ay;
+                m.term[2][q] = t0;
+                m.term[3][q] = en;
+            }
+            if (q1 < entries) __syncthreads();
         }
         __syncthreads();
         if (mine) {

@@ -162,7 +162,7 @@ extern "C" int dpg_bumpy_create(const dpg_bumpy_params *p, void *cuda_stream, dp
     s->nlg = (long long)s->nb < (long long)nsm * 1024 ? 8 : 1;
     s->ntpb = (long long)s->nb * s->nlg < (long long)nsm * 2 * kTPB ? 64 : kTPB;
     w.max_blocks = std::max(std::max(s->gb(s->nb), s->gw(s->nb)), s->ngrid());
-    w.max_blocks = std::max(w.max_blocks, nsm);
+    w.max_blocks = std::max(w.max_blocks, kLoopBlocksMax);
     A((void **)&w.partials, (size_t)w.max_blocks * 8 * 8);
     A((void **)&x.w, nb * 8); A((void **)&x.th, nb * 8); A((void **)&x.tq, nb * 8); A((void **)&x.I, nb * 8);
     A((void **)&x.nvb, nb * 4); A((void **)&x.start, nb * 4);
@@ -772,6 +772,7 @@ static int plan_resident(BS *s) {
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    nsm = std::min(nsm, kLoopBlocksMax);
     const int per = (s->nb + nsm - 1) / nsm;
     if (!coop || per > kLoopBodies) return set_err(DPG_ERR_STATE, "no resident loop for this system");
     for (void *fn : {(void *)kb_loop<0>, (void *)kb_loop<1>}) {

@@ -1223,6 +1223,32 @@ __global__ void k_fire_move(DevSys *ds) {
     }
 }
 
+// Mean energy of a FIRE iteration (s.pe) and whether it has stopped changing.
+// Without energy targets no test reads it, and the FP64 division stays off the
+// iteration's serial path (0: below no target).
+__device__ __forceinline__ bool fire_energy(DevState &s, double &avg) {
+    avg = 0.0;
+    if (!(s.pe_target > 0) && !(s.pe_diff_target > 0)) return false;
+    avg = s.pe / s.dof;
+    const bool still = s.pe_diff_target > 0 && fabs(avg / s.last_avg_pe - 1) < s.pe_diff_target;
+    s.last_avg_pe = avg;
+    return still;
+}
+
+// Mixed form: FP32 pairs until max|F| reaches switch_fmax, FIRE keeps going
+// uphill, or max|F| stops falling within 100x of switch_fmax (FP32 noise
+// floor); FP64 pairs after.  f2: max|F|^2 of the iteration.
+__device__ __forceinline__ void fire_switch(DevState &s, double f2) {
+    if (f2 < 0.81 * s.best_f2) { s.best_f2 = f2; s.best_it = s.iter; }
+    bool go = s.f_nbad > 5;
+    // far above 100 switch_fmax the root is not needed to tell
+    if (!go && f2 < 1.001e4 * s.switch_fmax * s.switch_fmax) {
+        const double fm = sqrt(f2);
+        go = fm <= s.switch_fmax || (fm < 100.0 * s.switch_fmax && s.iter - s.best_it > 2000);
+    }
+    if (go) s.fp64_now = 1;
+}
+
 // End of a FIRE iteration, from its totals (PE, power, max|F|^2): the
 // minimizeFire convergence tests (src/routines/minimization.cu:96-106) and the
 // next step's Fire::step decision.
@@ -1231,23 +1257,12 @@ __device__ __forceinline__ void fire_epilogue(DevState &s, const double (&v)[3])
     s.pe = v[0];
     s.power = v[1];
     s.fmax2 = v[2];
-    double avg = v[0] / s.dof;
-    // (no target: no test, and no FP64 division on the iteration's serial path)
-    const bool pe_still = s.pe_diff_target > 0 && fabs(avg / s.last_avg_pe - 1) < s.pe_diff_target;
-    s.last_avg_pe = avg;
+    double avg;
+    const bool pe_still = fire_energy(s, avg);
     long long it = s.iter;
-    // mixed form: FP32 pairs until max|F| reaches switch_fmax, FIRE keeps going
-    // uphill, or max|F| stops falling within 100x of switch_fmax (FP32 noise
-    // floor); FP64 pairs after, and only an FP64 state may pass the PE-change
-    // and max|F| tests
-    bool fp64 = true;
-    if (M && !s.fp64_now) {
-        if (v[2] < 0.81 * s.best_f2) { s.best_f2 = v[2]; s.best_it = it; }
-        const double fm = sqrt(v[2]);
-        if (fm <= s.switch_fmax || s.f_nbad > 5 || (fm < 100.0 * s.switch_fmax && it - s.best_it > 2000))
-            s.fp64_now = 1;
-        fp64 = false;
-    }
+    // only an FP64 state may pass the PE-change and max|F| tests
+    const bool fp64 = !M || s.fp64_now;
+    if (!fp64) fire_switch(s, v[2]);
     if ((fp64 && pe_still) || avg < s.pe_target) {
         s.result_step = it; s.f_converged = 1; s.flags |= kDone; return;
     }

@@ -27,6 +27,7 @@ namespace dpg {
 namespace {
 
 constexpr int kLoopMaxTPB = 512;
+constexpr int kLoopBlocksMax = 160;  // blocks of a FIRE loop at most
 constexpr long long kBarPolls = 1LL << 22;  // ~1 s of polls
 
 struct LoopSync {
@@ -258,13 +259,6 @@ __device__ __forceinline__ int rebuild_kind(unsigned long long w) {
     return raised(w, kNeedCell) ? 2 : (raised(w, kNeedList) ? 1 : 0);
 }
 
-// Maximum of non-negative numbers without the FP64 pipe: their bits order them.
-// A NaN b is dropped, as fmax does.
-__device__ __forceinline__ double max_pos(double a, double b) {
-    const long long ia = __double_as_longlong(a), ib = __double_as_longlong(b);
-    return ib > ia && ib <= 0x7ff0000000000000LL ? b : a;
-}
-
 // The totals of a FIRE iteration over the grid: v[0], v[1] summed, the other
 // K - 2 maxima; thread 0 gets them.  `nwr`: warps that hold values.  Two sums
 // share each FP64 instruction (lanes 0 - 15 and 16 - 31): an instruction holds
@@ -305,13 +299,25 @@ __device__ __forceinline__ bool grid_totals(double (&v)[K], int nwr, double *par
     }
     if (!grid_bar(ls, bk, 0)) return false;
     if (wid == 0) {
+        // all loads in flight at once (one trip to L2), then added in order
         const double *mine = part + (lane < 16 ? 0 : nb);
-        sum = 0.0;
-        for (int b = lane & 15; b < nb; b += 16) sum += mine[b];
+        constexpr int U = (kLoopBlocksMax + 15) / 16;
+        double a[U], c[K - 2][U / 2];
+#pragma unroll
+        for (int q = 0; q < U; q++) a[q] = (lane & 15) + 16 * q < nb ? mine[(lane & 15) + 16 * q] : 0.0;
+#pragma unroll
+        for (int k = 0; k < K - 2; k++)
+#pragma unroll
+            for (int q = 0; q < U / 2; q++) c[k][q] = lane + 32 * q < nb ? part[(2 + k) * nb + lane + 32 * q] : 0.0;
+        sum = a[0];
+#pragma unroll
+        for (int q = 1; q < U; q++)
+            if (16 * q < nb) sum += a[q];
 #pragma unroll
         for (int k = 0; k < K - 2; k++) {
             mx[k] = 0.0;
-            for (int b = lane; b < nb; b += 32) mx[k] = max_pos(mx[k], part[(2 + k) * nb + b]);
+#pragma unroll
+            for (int q = 0; q < U / 2; q++) mx[k] = max_pos(mx[k], c[k][q]);
         }
         warp_totals<K>(sum, mx);
         v[1] = __shfl_sync(0xffffffffu, sum, 16);

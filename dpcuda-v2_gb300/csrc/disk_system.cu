@@ -152,7 +152,6 @@ struct dpg_system {
 // The loops run as one resident grid up to kLoopMaxN particles, as a graph of
 // full-size kernels above (see plan_resident).
 constexpr int kLoopMaxN = 1 << 17;
-constexpr int kLoopBlocksPerSM = 2;
 
 static int dalloc(dpg_system *s, void **p, size_t bytes) {
     CK(cudaMalloc(p, bytes > 0 ? bytes : 16));
@@ -312,7 +311,7 @@ extern "C" int dpg_create(const dpg_params *p, void *cuda_stream, dpg_handle *ou
     const int fg8 = std::max(1, (int)(((long long)s->n * 8 + s->ftpb - 1) / s->ftpb));
     w.max_blocks = std::max(std::max(s->grid(s->n), s->grid_full(s->n)), std::max(s->fgrid(), fg8));
     w.max_blocks = std::max(std::max(w.max_blocks, s->ngrid()), (s->n + kStressTPB - 1) / kStressTPB);
-    w.max_blocks = std::max(w.max_blocks, kLoopBlocksPerSM * nsm);
+    w.max_blocks = std::max(w.max_blocks, kLoopBlocksMax);
     A((void **)&w.partials, (size_t)w.max_blocks * 8 * 8);
     A((void **)&w.s_pos, n * 16); A((void **)&w.s_vel, n * 16); A((void **)&w.s_frc, n * 16);
     A((void **)&w.s_rad, n * 8); A((void **)&w.s_mass, n * 8); A((void **)&w.s_sidx, n * 4);
@@ -1101,14 +1100,14 @@ static void *loop_fn(const dpg_system *s) {
 // kTileP of them on each SM, rows of at most kTileSlots neighbours.  k_loop
 // walks any number of tiles through memory.  Few particles leave most of the
 // FP64 pipes idle unless they are spread over every SM, so both take a block an
-// SM and as few warps as cover its particles (k_loop a second block an SM where
-// it fits).  Lanes per neighbour row: as many as kLoopMaxTPB threads allow.
+// SM and as few warps as cover its particles.  Lanes per neighbour row: as many as kLoopMaxTPB threads allow.
 static int plan_resident(dpg_system *s) {
     int dev = 0, nsm = 0, coop = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     if (!coop) return set_err(DPG_ERR_CUDA, "no cooperative launch");
+    nsm = std::min(nsm, kLoopBlocksMax);
     const long long n = s->n, per = (n + nsm - 1) / nsm;  // particles an SM
     auto warps = [](long long threads) { return (int)std::max<long long>(32, (threads + 31) / 32 * 32); };
     if (per <= kTileP) {
@@ -1132,17 +1131,15 @@ static int plan_resident(dpg_system *s) {
     else q.lanes = per * 8 <= kLoopMaxTPB ? 8 : (per * 2 <= kLoopMaxTPB ? 2 : 1);
     q.threads = std::min(kLoopMaxTPB, warps(per * q.lanes));
     q.smem = sizeof(ForceWarp) * (q.threads / 32);
-    int per_sm = kLoopBlocksPerSM;
     for (void *fn : {loop_fn<kLoopFire>(s), loop_fn<kLoopNve>(s)}) {
         int occ = 0;
         CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)(sizeof(ForceWarp) * (kLoopMaxTPB / 32))));
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, q.threads, q.smem));
-        per_sm = std::min(per_sm, occ);
+        if (occ < 1) return set_err(DPG_ERR_CUDA, "the resident loop does not fit an SM");
     }
-    if (per_sm < 1) return set_err(DPG_ERR_CUDA, "the resident loop does not fit an SM");
     const int tile = q.threads / q.lanes;
-    const long long blocks = std::min<long long>((long long)per_sm * nsm, (n + tile - 1) / tile);
+    const long long blocks = std::min<long long>(nsm, (n + tile - 1) / tile);
     q.chunk = (int)((n + blocks - 1) / blocks);
     q.blocks = (int)((n + q.chunk - 1) / q.chunk);
     return DPG_OK;
