@@ -44,10 +44,12 @@ struct dpg_ensemble_system {
     bool split_force = false;    // grid form: FP32 and refinement force kernels apart
     long long launches = 0;      // kernel launches and graph launches issued for this ensemble
     // resident form: one stream per size class, the block -> system lists
-    cudaStream_t rs_stream[8] = {};
-    cudaEvent_t rs_fork = nullptr, rs_join[8] = {};
-    int rs_fit[8] = {};          // clusters of each class the GPU holds at once (0: not yet asked)
-    int rs_rot[8] = {};          // rotation of each class's systems between launches
+    static constexpr int kShapes = 13;
+    cudaStream_t rs_stream[kShapes] = {};
+    cudaEvent_t rs_fork = nullptr, rs_join[kShapes] = {};
+    int rs_fit[kShapes] = {};    // clusters of each class the GPU holds at once (0: not yet asked)
+    int rs_rot[kShapes] = {};    // rotation of each class's systems between launches
+    bool rs_wide = true;         // the wide table of shapes (see kRClasses)
     int *d_rs_blocks = nullptr;
 };
 
@@ -70,7 +72,7 @@ static int ealloc(ES *s, void **p, size_t bytes) {
 extern "C" int dpg_ensemble_destroy(dpg_ensemble s) {
     if (!s) return DPG_OK;
     if (s->stream) cudaStreamSynchronize(s->stream);
-    for (int c = 0; c < 8; c++) {
+    for (int c = 0; c < dpg_ensemble_system::kShapes; c++) {
         if (s->rs_stream[c]) cudaStreamDestroy(s->rs_stream[c]);
         if (s->rs_join[c]) cudaEventDestroy(s->rs_join[c]);
     }
@@ -465,42 +467,49 @@ static int run(ES *s, long long guard_limit) {
 }
 
 // ---- the resident form --------------------------------------------------------
-typedef void (*res_kernel_fn)(EDev *, const int *, int, long long, unsigned long long);
-// Size classes (threads per block, particles per lane group, blocks per
-// cluster, lanes per particle): a system goes to the first class that holds it.
+typedef void (*res_kernel_fn)(EDev *, const int *, int, int, long long, unsigned long long);
+// Shapes (warps per block, particles per warp and pass, passes, blocks per
+// cluster): a system goes to the first shape of its table that holds it.  The
+// wide table spreads a system over many blocks and lanes, which shortens its
+// iterations; the dense one packs it into few, which takes fewer instructions
+// in all and lets more systems share the GPU.  No result depends on the shape.
+// Per iteration wide / dense, one system of 100 disks 3.5 / 4.2 us, of 900 5.4 /
+// 7.6; many systems, dense against the former shapes: 400 x 100 disks 8.7 / 13.8,
+// 300 x 400 17.7 / 21.6 (wide: 15.8, 72).
 struct RClass {
-    int nt, ppt, c, g;
+    int w, p, r, c;
     res_kernel_fn fn;
-    int per_block() const { return nt / g * ppt; }
-    int capacity() const { return nt / g * ppt * c; }
+    int per_block() const { return w * p * r; }
+    int capacity() const { return per_block() * c; }
 };
-// Measured on one GB300 (double-word FIRE iterations of 4 / 48 systems):
-// lanes per particle and larger blocks for the small systems (N = 128: 5.4 vs
-// 9.4 us per iteration with 4 particles per thread), clusters of 8 blocks for
-// the largest (N = 4096 alone: 18.8 vs 30.0 us on 4 blocks of 4 particles per
-// thread), 2 particles per thread where many large systems share the GPU
-// (N = 2048, 48 systems: 24.9 vs 30.6 us).
-// The last class holds up to 16384 disks: 8-block clusters of 512 threads x 4
-// particles (2048 disks and ~146 KB of shared memory a block).
-constexpr int kNClass = 8;
-#define RC(NT, PPT, C, G) {NT, PPT, C, G, e_res<NT, PPT, C, G>}
-static const RClass kRClasses[kNClass] = {RC(256, 1, 1, 4), RC(256, 1, 1, 2), RC(256, 1, 1, 1),
-                                          RC(512, 1, 1, 1), RC(512, 1, 2, 1), RC(256, 2, 4, 1),
-                                          RC(256, 2, 8, 1), RC(512, 4, 8, 1)};
+constexpr int kNClass = 13;
+#define RC(W, P, R, C) {W, P, R, C, e_res<W, P, R, ((C) > 1)>}
+static const RClass kRClasses[kNClass] = {
+    RC(16, 8, 1, 1),  RC(16, 8, 1, 2),  RC(16, 8, 1, 4), RC(16, 8, 1, 8), RC(16, 32, 1, 4), RC(16, 32, 1, 8),
+    RC(16, 32, 4, 8), RC(4, 32, 1, 1),  RC(8, 32, 1, 1), RC(8, 32, 2, 1), RC(8, 32, 2, 2),  RC(8, 32, 2, 4),
+    RC(8, 32, 2, 8)};
 #undef RC
+constexpr int kNTable = 7;
+static const int kResWide[kNTable] = {0, 1, 2, 3, 4, 5, 6}, kResDense[kNTable] = {7, 8, 9, 10, 11, 12, 6};
 
-static int res_class_of(int n) {
-    for (int c = 0; c < kNClass; c++)
-        if (n <= kRClasses[c].capacity()) return c;
+static int res_class_in(const int *table, int n) {
+    for (int k = 0; k < kNTable; k++)
+        if (n <= kRClasses[table[k]].capacity()) return table[k];
     return -1;
 }
+static int res_class_of(const ES *s, int n) {
+    return res_class_in(s->rs_wide ? kResWide : kResDense, n);
+}
 
-// largest cell count of the systems of class c
-static int res_ncmax(const ES *s, int c) {
-    int m = 1;
+// largest cell count and system of class c
+static void res_most(const ES *s, int c, int *ncmax, int *nmax) {
+    *ncmax = 1;
+    *nmax = 1;
     for (const auto &y : s->sys)
-        if (res_class_of(y.n) == c) m = std::max(m, y.ncd * y.ncd);
-    return m;
+        if (res_class_of(s, y.n) == c) {
+            *ncmax = std::max(*ncmax, y.ncd * y.ncd);
+            *nmax = std::max(*nmax, y.n);
+        }
 }
 
 static int res_smem_limit() {
@@ -510,24 +519,41 @@ static int res_smem_limit() {
     return v;
 }
 
-// the resident form holds every system: sizes and shared memory within limits
-static bool res_fits(const ES *s) {
-    if (s->max_n > kResMaxN) return false;
-    const size_t lim = (size_t)res_smem_limit();
+// dynamic shared memory there is for a block: the rest is static
+constexpr int kResStatic = 1904;
+static_assert(sizeof(ESys) + sizeof(RCtl) + 32 <= kResStatic, "static shared memory of e_res");
+static size_t res_smem_room() { return (size_t)std::max(0, res_smem_limit() - kResStatic); }
+
+static bool res_table_fits(const ES *s) {
     for (int c = 0; c < kNClass; c++) {
-        const size_t b = res_smem_bytes(kRClasses[c].per_block(), kRClasses[c].capacity(), res_ncmax(s, c));
-        if (b + 4096 > lim) return false;  // room for the kernel's static shared memory
+        int ncmax, nmax;
+        res_most(s, c, &ncmax, &nmax);
+        if (res_smem_bytes(kRClasses[c].per_block(), kRClasses[c].w, nmax, ncmax, 0) > res_smem_room()) return false;
     }
     return true;
 }
 
+// the resident form holds every system: sizes and shared memory within limits.
+// Chooses the table: the wide one while its blocks (one an SM) leave an eighth
+// of the SMs for what clusters cannot use, the dense one beyond, where systems
+// would have to take turns, unless only the wide one's smaller blocks fit.
+static bool res_fits(ES *s) {
+    if (s->max_n > kResMaxN) return false;
+    int dev = 0, nsm = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    long long blocks = 0;
+    for (const auto &y : s->sys) blocks += kRClasses[res_class_in(kResWide, y.n)].c;
+    s->rs_wide = blocks <= nsm / 8 * 7;
+    if (!s->rs_wide && !res_table_fits(s)) s->rs_wide = true;
+    return res_table_fits(s);
+}
 
 // one cluster of K.c blocks per system, nb systems
 static cudaLaunchConfig_t res_config(const RClass &K, int nb, size_t smem, cudaStream_t st,
                                      cudaLaunchAttribute *attr) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(nb * K.c);
-    cfg.blockDim = dim3(K.nt);
+    cfg.blockDim = dim3(32 * K.w);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -551,18 +577,20 @@ static int launch_resident(ES *s, long long budget, unsigned long long slice_ns,
     for (int k = 0; k < s->S; k++) {
         const ESys &y = s->sys[k];
         if (y.phase == kIdle) continue;
-        order[res_class_of(y.n)].push_back(k);
+        order[res_class_of(s, y.n)].push_back(k);
     }
     std::vector<int> flat;
     int first[kNClass];
     size_t smem[kNClass];
-    int ncmax[kNClass];
+    int ncmax[kNClass], lcap[kNClass];
     for (int c = 0; c < kNClass; c++) {
         first[c] = (int)flat.size();
         if (order[c].empty()) continue;
         const RClass &K = kRClasses[c];
-        ncmax[c] = res_ncmax(s, c);
-        smem[c] = res_smem_bytes(K.per_block(), K.capacity(), ncmax[c]);
+        int nmax;
+        res_most(s, c, &ncmax[c], &nmax);
+        lcap[c] = res_list_entries(K.per_block(), K.w, ncmax[c], res_smem_room());
+        smem[c] = res_smem_bytes(K.per_block(), K.w, nmax, ncmax[c], lcap[c]);
         CK(cudaFuncSetAttribute((const void *)K.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[c]));
         if (!s->rs_fit[c]) {
             cudaLaunchAttribute attr[1];
@@ -605,7 +633,7 @@ static int launch_resident(ES *s, long long budget, unsigned long long slice_ns,
         const cudaLaunchConfig_t cfg = res_config(K, nb, smem[c], s->rs_stream[c], attr);
         const int *blocks = s->d_rs_blocks + first[c];
         EDev *dev = s->d;
-        CK(cudaLaunchKernelEx(&cfg, kern, dev, blocks, ncmax[c], budget, slice_ns));
+        CK(cudaLaunchKernelEx(&cfg, kern, dev, blocks, ncmax[c], lcap[c], budget, slice_ns));
         s->launches++;
         CK(cudaEventRecord(s->rs_join[c], s->rs_stream[c]));
         CK(cudaStreamWaitEvent(s->stream, s->rs_join[c], 0));
@@ -639,6 +667,7 @@ static int run_resident(ES *s, long long guard_limit) {
     const unsigned long long kSlice = 200ull * 1000 * 1000;  // 0.2 s
     const long long kChunk = 1LL << 24;
     std::vector<long long> base(s->S, -1);
+    if (!res_fits(s)) return set_err(DPG_ERR_ARG, "resident form: the systems do not fit");
     long long last_sum = -1;
     for (int launches = 0; launches < (1 << 22); launches++) {
         EDev cur;
@@ -675,7 +704,7 @@ static int run_resident(ES *s, long long guard_limit) {
 // disks the grid form ran 3.5e8 particle-iterations/s against the persistent
 // form's 3.0e8 (512-thread blocks).  dpg_ensemble_autotune measures and may
 // choose any of them.
-static int form_of(const ES *s) {
+static int form_of(ES *s) {
     if (s->form != DPG_FORM_AUTO) return s->form;
     return res_fits(s) ? DPG_FORM_RESIDENT : DPG_FORM_GRID;
 }
