@@ -474,8 +474,9 @@ typedef void (*res_kernel_fn)(EDev *, const int *, int, int, long long, unsigned
 // iterations; the dense one packs it into few, which takes fewer instructions
 // in all and lets more systems share the GPU.  No result depends on the shape.
 // Per iteration wide / dense, one system of 100 disks 3.5 / 4.2 us, of 900 5.4 /
-// 7.6; many systems, dense against the former shapes: 400 x 100 disks 8.7 / 13.8,
-// 300 x 400 17.7 / 21.6 (wide: 15.8, 72).
+// 7.6; many (systems x disks), dense against the former shapes: 400 x 100 8.7 /
+// 13.8, 300 x 400 17.7 / 21.6, 160 x 900 26 / 41, 60 x 1500 18 / 21, 40 x 3000
+// 32 / 44 (wide: 15.8, 72, 95, 26, 41).
 struct RClass {
     int w, p, r, c;
     res_kernel_fn fn;
@@ -566,12 +567,13 @@ static cudaLaunchConfig_t res_config(const RClass &K, int nb, size_t smem, cudaS
 }
 
 // Launch every class that has live systems, each on its own stream (forked
-// from and joined back into the ensemble's stream).  slice_ns bounds a launch.
-// A launch carries at most as many systems of a class as the GPU holds
+// from and joined back into the ensemble's stream).  slice_ns bounds a launch,
+// turn_ns one in which systems take turns.  A launch carries at most as many systems of a class as the GPU holds
 // clusters of it at once (cudaOccupancyMaxActiveClusters): more would run as a
 // second wave after the first wave's time slice, on a mostly idle GPU.  The
 // class's systems take turns, rotating between launches.
-static int launch_resident(ES *s, long long budget, unsigned long long slice_ns, int *launched) {
+static int launch_resident(ES *s, long long budget, unsigned long long slice_ns, unsigned long long turn_ns,
+                           int *launched) {
     *launched = 0;
     std::vector<int> order[kNClass];
     for (int k = 0; k < s->S; k++) {
@@ -612,6 +614,7 @@ static int launch_resident(ES *s, long long budget, unsigned long long slice_ns,
             std::rotate(order[c].begin(), order[c].begin() + rot, order[c].end());
             order[c].resize(s->rs_fit[c]);
             s->rs_rot[c] = (int)(((long long)rot + s->rs_fit[c]) % nb);
+            slice_ns = turn_ns;
         }
         flat.insert(flat.end(), order[c].begin(), order[c].end());
     }
@@ -661,10 +664,14 @@ static int grow_lists(ES *s, const EDev &cur) {
 // for at most kSlice of device time per block (so the classes' launches end
 // together and the host sees progress); termination is the device state
 // machine's (every minimisation has a step cap, jamming a compression cap);
+// Where a class has more systems than fit, they take turns of 0.5 ms at first,
+// growing to stay a fifteenth of the time spent: whole runs one after the other
+// would leave the last ones on a mostly idle GPU.
 // the host stops with an error when some system's FIRE passes in this run
 // exceed guard_limit or a launch makes no progress.
 static int run_resident(ES *s, long long guard_limit) {
     const unsigned long long kSlice = 200ull * 1000 * 1000;  // 0.2 s
+    double turn = 0.5e6;
     const long long kChunk = 1LL << 24;
     std::vector<long long> base(s->S, -1);
     if (!res_fits(s)) return set_err(DPG_ERR_ARG, "resident form: the systems do not fit");
@@ -690,7 +697,8 @@ static int run_resident(ES *s, long long guard_limit) {
         if (sum == last_sum) return set_err(DPG_ERR_STATE, "resident launch made no progress");
         last_sum = sum;
         int nl = 0;
-        TRY(launch_resident(s, kChunk, kSlice, &nl));
+        TRY(launch_resident(s, kChunk, kSlice, (unsigned long long)turn, &nl));
+        turn = std::min(1.07 * turn, (double)kSlice);
         if (!nl) return DPG_OK;
     }
     return set_err(DPG_ERR_STATE, "ensemble loop did not finish");
