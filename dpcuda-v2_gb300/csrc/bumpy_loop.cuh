@@ -165,9 +165,9 @@ struct BodyMem {
     int row[kBodyVerts + 1];
     int other[kVertRows];               // the other vertex
     unsigned short of[kVertRows];       // k
-    // a force pass: which entries touch (bit e), which certainly do, and how
-    // many touch before each word: the queue position of entry e is rank(e)
-    unsigned touch[kBodyVerts + 1], sure[kBodyVerts];
+    // a force pass: which entries may touch (bit e), and how many before each
+    // word: the queue position of entry e is rank(e)
+    unsigned touch[kBodyVerts + 1];
     int count[kBodyVerts], before[kBodyVerts + 1];
     unsigned short ent[kVertQueue];     // entry at each queue position
     unsigned vmask[kBodyVerts / 32];    // vertices that have a term
@@ -198,14 +198,14 @@ __device__ __forceinline__ void entry_of(const BodyMem &m, const BumpySys &L, in
     j = L.x.vnbr[(size_t)(e - m.row[k]) * L.x.nv + v0 + k];
 }
 
-// vertex contact: disk_pair_sum with one radius sum, its square and its reciprocal
+// vertex contact: disk_pair_sum with one radius sum and its reciprocal
 struct VertConst {
-    double rs, rs2, inv;
+    double rs, inv;
 };
-__device__ __forceinline__ double vertex_pair(const PairArgs &f, const VertConst &c, bool sure, double2 a,
-                                              double2 b, double &fx, double &fy) {
+__device__ __forceinline__ double vertex_pair(const PairArgs &f, const VertConst &c, double2 a, double2 b,
+                                              double &fx, double &fy) {
     const double dx = pbc_dist_sum(a.x, b.x, f.bx, f.l4x), dy = pbc_dist_sum(a.y, b.y, f.by, f.l4y);
-    return contact_terms(dx, dy, c.rs, c.rs2, c.inv, sure, f.e_c, f.n_c, fx, fy);
+    return contact_terms<true>(dx, dy, c.rs, c.inv, f.e_c, f.n_c, fx, fy);
 }
 
 template <int KIND>
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) kb_loop(BumpySys *bs, LoopSync
     long long it = 0;
     const double dt_half = 0.5 * dt;
     const double rv = x.rv;
-    const VertConst vc = {rv + rv, (rv + rv) * (rv + rv), 1.0 / (rv + rv)};
+    const VertConst vc = {rv + rv, 1.0 / (rv + rv)};
     int v0 = 0, nv = 0;  // the block's first vertex and their number
 
     double a = 0.0, u = 0.0, f = 0.0, mass = 1.0, xn = 0.0, xc = 0.0, da = 0.0, pe = 0.0;
@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) kb_loop(BumpySys *bs, LoopSync
                 j[c] = v0;
                 if (on[c]) entry_of(m, L, nv, v0, e, k[c], j[c]);
             }
-            int hit[4] = {0, 0, 0, 0};
+            bool hit[4] = {false, false, false, false};
             if (fp32) {
                 float4 o[4];
 #pragma unroll
@@ -422,17 +422,16 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) kb_loop(BumpySys *bs, LoopSync
                 for (int c = 0; c < 4; c++) o[c] = x.vq[j[c]];
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
-                    if (on[c]) hit[c] = quant_contact(fa.sx, fa.sy, fa.tol, x.vq[v0 + k[c]], o[c]);
+                    hit[c] = on[c] && quant_touch(fa.sx, fa.sy, fa.tol, x.vq[v0 + k[c]], o[c]);
                     if (hit[c]) asm volatile("prefetch.global.L1 [%0];" ::"l"(x.vpos + j[c]));
                 }
             }
 #pragma unroll
             for (int c = 0; c < 4; c++) {
                 if (w0 + c * nw >= words) break;
-                const unsigned any = __ballot_sync(0xffffffffu, hit[c] != 0), both = __ballot_sync(0xffffffffu, hit[c] == 2);
+                const unsigned any = __ballot_sync(0xffffffffu, hit[c]);
                 if (lane == 0) {
                     m.touch[w0 + c * nw] = any;
-                    m.sure[w0 + c * nw] = both;
                     m.count[w0 + c * nw] = __popc(any);
                 }
             }
@@ -480,7 +479,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) kb_loop(BumpySys *bs, LoopSync
                     rf[kVertQueue + q] = fy;
                 } else {
                     double fx, fy;
-                    const double ee = vertex_pair(fa, vc, m.sure[e >> 5] >> (e & 31) & 1u, m.vpos[k], fa.pos[j], fx, fy);
+                    const double ee = vertex_pair(fa, vc, m.vpos[k], fa.pos[j], fx, fy);
                     m.res[0][q] = fx;
                     m.res[1][q] = fy;
                     m.res[2][q] = ee;

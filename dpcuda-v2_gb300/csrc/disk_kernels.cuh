@@ -56,9 +56,8 @@ __device__ __forceinline__ double disk_pair(double xi, double yi, double ri, dou
 // sum of its pair terms in neighbour-slot order.  Pairs that do not touch add
 // +0.0, which leaves a sum that started at +0.0 unchanged, so only the
 // contacts need FP64 work.  Bound: the FP64 pipe (2 lanes a clock on each SM;
-// a contact is ~45 FP64 instructions, one square root and two divisions among
-// them), where an instruction costs the same with one active lane as with 32.
-// So a warp (32 / G particles, G lanes each) works in three steps: G lanes test
+// a contact is ~30 FP64 instructions), where an instruction costs the same with
+// one active lane as with 32.  So a warp (32 / G particles, G lanes each) works in three steps: G lanes test
 // a particle's slots by the fixed-point filter; the surviving pairs of all its
 // particles are queued in shared memory, ordered by particle and slot, and
 // evaluated 32 at a time, whoever they belong to; each particle then adds its
@@ -97,28 +96,44 @@ __device__ __forceinline__ PairArgs pair_args(const DevSys *ds) {
             ds->p.n_c, ds->p.q_l4[0], ds->p.q_l4[1], ds->p.q_s[0], ds->p.q_s[1], ds->p.q_tol, 0.0};
 }
 
-// The terms of a contact from its displacement, for radius sum rs, its square
-// and its reciprocal rounded to nearest (0: none kept; the quotient is the same
-// either way).  sure: the fixed-point distance has already decided that the two
-// touch.  disk_pair's arithmetic.
-__device__ __forceinline__ double contact_terms(double dx, double dy, double rs, double rs2, double inv,
-                                                bool sure, double e_c, double n_c, double &fx, double &fy) {
+// The terms of a contact from its displacement for radius sum rs; inv: near
+// 1 / rs where the caller keeps one (KEPT).  disk_pair's arithmetic and its bits, on 30 FP64
+// instructions instead of 46 (displacement included) for harmonic contacts: an
+// NVE step of 1048576 disks 362 -> 325 us, of 4096 bodies 60 -> 53 us.
+template <bool KEPT>
+__device__ __forceinline__ double contact_terms(double dx, double dy, double rs, double inv, double e_c,
+                                                double n_c, double &fx, double &fy) {
     const double d2 = dx * dx + dy * dy;
     fx = 0.0;
     fy = 0.0;
-    if (!sure && d2 >= rs2) return 0.0;
+    // constants compared as integers: FP64 compares take the FP64 pipe
+    const bool square = __double2hiint(n_c) == 0x40000000 && __double2loint(n_c) == 0;
+    const bool unit = __double2hiint(e_c) == 0x3ff00000 && __double2loint(e_c) == 0;
+    if (square && middling(d2) && middling(rs) && middling(e_c)) {
+        double y;
+        const double d = root_near(d2, y);
+        if (!KEPT) inv = rcp_near(rs);
+        const double ov = 1.0 - div_near(d, rs, inv);
+        // an overlap above 2^-40 needs no test
+        if (__double2hiint(ov) < 0x3d700000 && d2 >= rs * rs) return 0.0;
+        const double a = unit ? ov : e_c * ov;  // pow(ov, 1) == ov
+        const double fm = div_near(a, rs * d, inv * y);
+        fx = fm * dx;
+        fy = fm * dy;
+        return a * ov * 0.25;  // x / 4 == x * 0.25 exactly
+    }
+    if (d2 >= rs * rs) return 0.0;
     const double d = sqrt(d2);
-    // (no quotient near the end of the range: |d| above 2^-300, 1e-15 < rs < 1e16)
-    const bool quick = inv != 0.0 && (unsigned)__double2hiint(d) > 0x2d300000u;
-    const double ov = 1.0 - (quick ? div_by(d, rs, inv) : d / rs);
-    double ovp = ov, energy;
-    if (n_c == 2.0) {  // pow(ov, 1) == ov, and x / 4 == x * 0.25 exactly
-        energy = e_c == 1.0 ? ov * ov * 0.25 : e_c * ov * ovp * 0.25;
+    const double ov = 1.0 - (d / rs);
+    double ovp, energy;
+    if (square) {
+        ovp = ov;
+        energy = e_c * ov * ovp * 0.25;
     } else {
         ovp = pow(ov, n_c - 1);
         energy = e_c * ov * ovp / (2.0 * n_c);
     }
-    const double fm = (e_c == 1.0 ? ovp : e_c * ovp) / (rs * d);
+    const double fm = e_c * ovp / (rs * d);
     fx = fm * dx;
     fy = fm * dy;
     return energy;
@@ -130,25 +145,7 @@ __device__ __forceinline__ double disk_pair_sum(const PairArgs &f, double2 pi, d
                                                 double &fy) {
     dx = pbc_dist_sum(pi.x, pj.x, f.bx, f.l4x);
     dy = pbc_dist_sum(pi.y, pj.y, f.by, f.l4y);
-    const double rs = ri + rj;
-    const double d2 = dx * dx + dy * dy;
-    fx = 0.0;
-    fy = 0.0;
-    if (d2 >= rs * rs) return 0.0;
-    const double d = sqrt(d2);
-    const double ov = 1.0 - (d / rs);
-    double ovp, energy;
-    if (f.n_c == 2.0) {  // pow(ov, 1) == ov, and x / 4 == x * 0.25 exactly
-        ovp = ov;
-        energy = f.e_c * ov * ovp * 0.25;
-    } else {
-        ovp = pow(ov, f.n_c - 1);
-        energy = f.e_c * ov * ovp / (2.0 * f.n_c);
-    }
-    const double fm = f.e_c * ovp / (rs * d);
-    fx = fm * dx;
-    fy = fm * dy;
-    return energy;
+    return contact_terms<false>(dx, dy, ri + rj, 0.0, f.e_c, f.n_c, fx, fy);
 }
 
 // Slots s0 .. s0 + kSlotChunk - 1 of the particle's list that may touch it, as
