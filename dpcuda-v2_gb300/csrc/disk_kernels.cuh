@@ -65,7 +65,7 @@ __device__ __forceinline__ double disk_pair(double xi, double yi, double ri, dou
 // for bit, for every G.  A loop over slots instead runs as many FP64 rounds as
 // the longest list of the warp has entries (~12 against ~4 queue rounds at 6.5
 // neighbours and 3.3 contacts a particle).
-// Measured at 2^20 disks of 3.3 contacts: k_nve_second 1219 -> 453 us; at 16384
+// Measured at 2^20 disks of 3.3 contacts: k_nve_second 1219 -> 365 us; at 16384
 // (2 lanes) k_fire_force 46 -> 32 us; k_stress of 131071 disks 262 -> 126 us.
 constexpr int kSlotChunk = 16;   // slots filtered before the queue is worked off
 constexpr int kPairWin = 160;    // queue entries evaluated before they are added up:
@@ -397,6 +397,19 @@ __device__ __forceinline__ void moved_update(DevSys *ds, int i, double2 p) {
     const double r = ds->v.rad[i];
     if (ds->p.precision == kMixed) ds->v.pk[i] = mixed_pack(ds->p, p, r);
     if (ds->p.precision != kMixed || ds->s.fp64_now) ds->v.q[i] = quant_of(ds->p, p, r);
+}
+
+// Squared displacements since the last neighbour and cell lists, which have the
+// same start as a rule (compared as integers).  The moves are bound by their
+// FP64 instructions: with this, unit masses tested and maxima taken as integers
+// some 20 instead of 50; k_nve_first of 2^20 disks 97 -> 53 us.
+__device__ __forceinline__ void moved2(double2 p, double2 a, double2 c, double (&v)[2]) {
+    const double dx = p.x - a.x, dy = p.y - a.y;
+    v[0] = v[1] = dx * dx + dy * dy;
+    if (__double_as_longlong(a.x) != __double_as_longlong(c.x) || __double_as_longlong(a.y) != __double_as_longlong(c.y)) {
+        const double cx = p.x - c.x, cy = p.y - c.y;
+        v[1] = cx * cx + cy * cy;
+    }
 }
 
 // mixed form: offsets of every particle from the current positions
@@ -1076,7 +1089,7 @@ __global__ void k_nve_first(DevSys *ds, double dt_half, double dt) {
     if (i < ds->p.n) {
         double2 *vel = ds->v.vel, *pos = ds->v.pos;
         double2 u = vel[i], f = ds->v.frc[i], p = pos[i];
-        double dtm = dt_half / ds->v.mass[i];
+        const double dtm = over_mass(dt_half, ds->v.mass[i]);
         u.x = u.x + f.x * dtm;
         u.y = u.y + f.y * dtm;
         vel[i] = u;
@@ -1084,13 +1097,9 @@ __global__ void k_nve_first(DevSys *ds, double dt_half, double dt) {
         p.y = p.y + u.y * dt;
         pos[i] = p;
         moved_update(ds, i, p);
-        double2 a = ds->w.pos_n[i], c = ds->w.pos_c[i];
-        double dxn = p.x - a.x, dyn = p.y - a.y, dxc = p.x - c.x, dyc = p.y - c.y;
-        v[0] = dxn * dxn + dyn * dyn;
-        v[1] = dxc * dxc + dyc * dyc;
+        moved2(p, ds->w.pos_n[i], ds->w.pos_c[i], v);
     }
-    const int ops[2] = {1, 1};
-    if (grid_reduce<2>(v, ops, ds)) {
+    if (grid_max<2>(v, ds)) {
         ds->s.max_nd2 = v[0];
         ds->s.max_cd2 = v[1];
         int rb = rebuild_decision(ds, v[0], v[1]);
@@ -1140,7 +1149,7 @@ __global__ void k_nve_second(DevSys *ds, double dt_half) {
         const double2 f = nve_force(ds, i, u, ax, ay, en, pe);
         ds->v.frc[i] = f;
         ds->w.pe[i] = pe;
-        double dtm = dt_half / ds->v.mass[i];
+        const double dtm = over_mass(dt_half, ds->v.mass[i]);
         u.x = u.x + f.x * dtm;
         u.y = u.y + f.y * dtm;
         vel[i] = u;
@@ -1196,7 +1205,7 @@ __global__ void k_fire_move(DevSys *ds) {
             p.y = p.y + u.y * back;
             u = make_double2(0.0, 0.0);
         }
-        double dtm = (dt / 2.0) / ds->v.mass[i];
+        const double dtm = over_mass(dt / 2.0, ds->v.mass[i]);
         u.x = u.x + f.x * dtm;
         u.y = u.y + f.y * dtm;
         u = fire_mix(u, f, alpha);
@@ -1205,13 +1214,9 @@ __global__ void k_fire_move(DevSys *ds) {
         p.y = p.y + u.y * dt;
         pos[i] = p;
         moved_update(ds, i, p);
-        double2 a = ds->w.pos_n[i], c = ds->w.pos_c[i];
-        double dxn = p.x - a.x, dyn = p.y - a.y, dxc = p.x - c.x, dyc = p.y - c.y;
-        v[0] = dxn * dxn + dyn * dyn;
-        v[1] = dxc * dxc + dyc * dyc;
+        moved2(p, ds->w.pos_n[i], ds->w.pos_c[i], v);
     }
-    const int ops[2] = {1, 1};
-    if (grid_reduce<2>(v, ops, ds)) {
+    if (grid_max<2>(v, ds)) {
         ds->s.max_nd2 = v[0];
         ds->s.max_cd2 = v[1];
         int rb = rebuild_decision(ds, v[0], v[1]);
@@ -1291,7 +1296,7 @@ __global__ void k_fire_force(DevSys *ds, int mode) {
         double2 *vel = ds->v.vel;
         double2 u = vel[i];
         if (mode != 1) {
-            double dtm = (ds->s.f_dt / 2.0) / ds->v.mass[i];
+            const double dtm = over_mass(ds->s.f_dt / 2.0, ds->v.mass[i]);
             u.x = u.x + f.x * dtm;
             u.y = u.y + f.y * dtm;
             vel[i] = u;

@@ -462,7 +462,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
     // (h / mass), kept while h is the same
     auto kick_factor = [&](double h) {
         if (!dtm_known || h != dtm_of) {
-            dtm = h / mass;
+            dtm = over_mass(h, mass);
             dtm_of = h;
             dtm_known = true;
         }
@@ -754,7 +754,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_loop(DevSys *ds, LoopSync *l
     if (KIND == 1) {
         unsigned long long fl = 0;
         for (int i = r.first + t; i < r.last; i += nt)
-            drift_to_other(i, v.vel[i], v.frc[i], dt_half / v.mass[i], fl);
+            drift_to_other(i, v.vel[i], v.frc[i], over_mass(dt_half, v.mass[i]), fl);
         const unsigned long long bw = grid_bar(ls, bk, block_flags(fl));
         ok = bw != 0;
         if (ok) {
@@ -778,7 +778,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_loop(DevSys *ds, LoopSync *l
                     x.y = x.y + u.y * back;
                     u = make_double2(0.0, 0.0);
                 }
-                const double dtm = (fdt / 2.0) / v.mass[i];
+                const double dtm = over_mass(fdt / 2.0, v.mass[i]);
                 u.x = u.x + f.x * dtm;
                 u.y = u.y + f.y * dtm;
                 u = fire_mix(u, f, alpha);
@@ -819,7 +819,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_loop(DevSys *ds, LoopSync *l
                 const double2 frc = nve_force(&L, i, u, ax, ay, en, pe);
                 v.frc[i] = frc;
                 w.pe[i] = pe;
-                const double dtm = dt_half / v.mass[i];
+                const double dtm = over_mass(dt_half, v.mass[i]);
                 u.x = u.x + frc.x * dtm;
                 u.y = u.y + frc.y * dtm;
                 if (last) v.vel[i] = u;
@@ -828,7 +828,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_loop(DevSys *ds, LoopSync *l
                 const double2 frc = make_double2(0.0 + ax, 0.0 + ay);
                 v.frc[i] = frc;
                 w.pe[i] = 0.0 + en;
-                const double dtm = (s.f_dt / 2.0) / v.mass[i];
+                const double dtm = over_mass(s.f_dt / 2.0, v.mass[i]);
                 u.x = u.x + frc.x * dtm;
                 u.y = u.y + frc.y * dtm;
                 v.vel[i] = u;

@@ -59,3 +59,50 @@ def test_contacts_are_the_oracles(dpg, e_c, n_c, scale):
             np.testing.assert_allclose(got[k], want[k], rtol=1e-14, atol=0, err_msg=k)
     s.close()
     o.close()
+
+
+@pytest.mark.parametrize("n", [1, 33, 700])
+@pytest.mark.parametrize("mass", ["unit", "random", "power", "tiny"])
+def test_kicks_are_the_oracles(dpg, n, mass):
+    """dt / m by unit masses, by the quick quotient and beyond its range (1e-70)."""
+    from oracle.oracle import DiskOracle, disk_packing, fill_normal
+    st = disk_packing(n, 0.5 if n > 1 else 0.1, 40 + n)
+    g = np.random.default_rng(n)
+    m = {"unit": np.ones(n), "random": g.uniform(0.3, 3.0, n), "power": 2.0 ** g.integers(-3, 4, n),
+         "tiny": np.full(n, 1e-70)}[mass]
+    vx, vy = fill_normal(n, 0.0, 1e-2, 1, n), fill_normal(n, 0.0, 1e-2, 1 + n, n)
+    if mass == "tiny":  # no overlaps: a kick of anything but zero would leave the box
+        st = dict(st, r=st["r"] * 1e-3)
+    o = DiskOracle(n, st["box"])
+    o.set_arrays(x=st["x"], y=st["y"], vx=vx, vy=vy, r=st["r"], m=m)
+    o.setup_neighbors(0, 1.7 / 1.4, 0.2, 8.0, 0.5)
+    s = dpg.Disk(n, st["box"])
+    s.setState(st["x"], st["y"], vx, vy, st["r"], m)
+    s.setupNeighbors("cell", 1.7 / 1.4, 0.2, 8.0, 0.5)
+    s.nveSteps(1e-2, 20)
+    o.nve_steps(1e-2, 20)
+    got, want = s.getState(), o.get_arrays()
+    for k in ("x", "y", "vx", "vy", "fx", "fy", "pe"):
+        np.testing.assert_array_equal(got[k], want[k], err_msg=k)
+    s.close()
+    o.close()
+
+
+@pytest.mark.parametrize("e_c", [2.0 ** -24, 2.0 ** 24])
+@pytest.mark.parametrize("n,phi", [(2, 0.3), (31, 0.84), (700, 0.84), (700, 1.2), (5000, 0.84)])
+def test_quick_fp32_contacts_are_the_general_ones(dpg, e_c, n, phi):
+    """A contact constant of 2^-24 or 2^24 lies outside the quick FP32 operations'
+    range and scales every term exactly: with 1 the forces must be the same bits."""
+    from oracle.oracle import disk_packing
+    st = disk_packing(n, phi, 60 + n)
+    out = []
+    for c in (1.0, e_c):
+        s = dpg.Disk(n, st["box"], c, 2.0, precision=dpg.MIXED)
+        s.setState(st["x"], st["y"], None, None, st["r"], st["m"])
+        s.setupNeighbors("cell", 1.7 / 1.4, 0.2, 8.0, 0.5)
+        s.zeroForceAndPotentialEnergy()
+        s.calculateForces()
+        out.append(s.getState())
+        s.close()
+    for k in ("fx", "fy", "pe"):
+        np.testing.assert_array_equal(out[1][k], e_c * out[0][k], err_msg=k)
