@@ -21,12 +21,15 @@
 // barrier does not complete sets LoopSync.err and leaves, and so does every
 // other block at its own limit.
 #pragma once
+#include <cooperative_groups.h>
+
 #include "disk_kernels.cuh"
 
 namespace dpg {
 namespace {
 
 constexpr int kLoopMaxTPB = 512;
+constexpr int kClusterMax = 16;      // blocks of a cluster at most
 constexpr int kLoopBlocksMax = 160;  // blocks of a FIRE loop at most
 constexpr long long kBarPolls = 1LL << 22;  // ~1 s of polls
 
@@ -49,8 +52,27 @@ __device__ __forceinline__ bool raised(unsigned long long v, unsigned long long 
 // out.  Barrier k + 2's word is cleared by block 0 once barrier k is complete:
 // every block has then left barrier k - 2, the word's last use, and reaches
 // k + 2 only after block 0's arrival at k + 1.
+// A grid of one thread-block cluster uses the cluster's barrier, the flags going
+// to every block's shared memory before it (two sets in turn: a block that
+// writes one again has passed a barrier that its readers entered later).
 __device__ __forceinline__ unsigned long long grid_bar(LoopSync *ls, unsigned &k, unsigned long long flags) {
-    __shared__ unsigned long long done;
+    __shared__ unsigned long long done, said[2][kClusterMax];
+    const auto cluster = cooperative_groups::this_cluster();
+    if (cluster.num_blocks() > 1) {
+        const int nb = (int)cluster.num_blocks(), t = threadIdx.x;
+        flags = __shfl_sync(0xffffffffu, flags, 0);
+        if (t < nb) *cluster.map_shared_rank(&said[k & 1][cluster.block_rank()], t) = 1ULL + flags;
+        cluster.sync();
+        if (t < 32) {
+            unsigned long long v = t < nb ? said[k & 1][t] : 0;
+#pragma unroll
+            for (int o = kClusterMax / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (t == 0) done = v;
+        }
+        __syncthreads();
+        k++;
+        return done;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
         unsigned long long *w = &ls->ring[k & 3], v;
@@ -419,6 +441,8 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
     const int g = t / G, sub = t & (G - 1), lead = lane - sub;
     if (t == 0) L = *ds;
     __syncthreads();
+    // every block of a cluster runs before its shared memory is written to
+    if (cooperative_groups::this_cluster().num_blocks() > 1) cooperative_groups::this_cluster().sync();
     const DevParams &p = L.p;
     DevView &v = L.v;
     DevState &s = L.s;

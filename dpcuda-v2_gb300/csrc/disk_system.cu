@@ -92,6 +92,7 @@ struct dpg_system {
     struct Plan {
         int lanes = 1, threads = 0, blocks = 0, chunk = 0;
         size_t smem = 0;
+        bool cluster = false;  // launched as one thread-block cluster
     } tile, loop;
     cudaGraphExec_t loop_exec[kLoopCount] = {nullptr, nullptr};
     cudaGraphConditionalHandle h_loop[kLoopCount] = {0, 0}, h_rb[kLoopCount] = {0, 0};
@@ -152,6 +153,13 @@ struct dpg_system {
 // The loops run as one resident grid up to kLoopMaxN particles, as a graph of
 // full-size kernels above (see plan_resident).
 constexpr int kLoopMaxN = 1 << 17;
+// Up to kClusterN particles k_tile runs on one cluster of at most 16 blocks,
+// whose barrier is shorter than the grid's through L2; more particles want more
+// SMs.  NVE step / FIRE iteration, cluster against grid: 64 disks 7.4 / 12.7
+// against 8.0 / 13.8 us, 256 7.6 / 12.6 against 8.0 / 13.7, 512 8.1 / 13.1
+// against 8.2 / 14.2, 1024 10.0 / 15.5 against 8.6 / 14.4; 8 blocks are no faster
+// at 8 - 128 and slower from 256 on.
+constexpr int kClusterN = 512;
 
 static int dalloc(dpg_system *s, void **p, size_t bytes) {
     CK(cudaMalloc(p, bytes > 0 ? bytes : 16));
@@ -1096,6 +1104,47 @@ static void *loop_fn(const dpg_system *s) {
     }
 }
 
+static cudaLaunchConfig_t cluster_config(const dpg_system::Plan &q, cudaStream_t st, cudaLaunchAttribute *attr) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(q.blocks);
+    cfg.blockDim = dim3(q.threads);
+    cfg.dynamicSmemBytes = q.smem;
+    cfg.stream = st;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = q.blocks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// k_tile's grid as one cluster, where the GPU can hold it
+static void plan_cluster(dpg_system *s) {
+    dpg_system::Plan q = s->tile;
+    const long long n = s->n;
+    q.chunk = (int)std::max<long long>((n + kClusterMax - 1) / kClusterMax, 4);
+    q.blocks = (int)((n + q.chunk - 1) / q.chunk);
+    if (q.blocks < 2 || q.chunk > kTileP) return;
+    q.lanes = q.chunk * 8 <= kLoopMaxTPB ? 8 : 4;
+    q.threads = std::max(32, (q.chunk * q.lanes + 31) / 32 * 32);
+    q.smem = tile_bytes(q.chunk);
+    q.cluster = true;
+    const dpg_system::Plan old = s->tile;
+    s->tile = q;
+    for (void *fn : {tile_fn<kLoopFire>(s), tile_fn<kLoopNve>(s)}) {
+        cudaLaunchAttribute attr[1];
+        const cudaLaunchConfig_t cfg = cluster_config(q, s->stream, attr);
+        int fit = 0;
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_bytes(kTileP)) != cudaSuccess ||
+            cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&fit, fn, &cfg) != cudaSuccess || fit < 1) {
+            (void)cudaGetLastError();
+            s->tile = old;
+            return;
+        }
+    }
+}
+
 // Two resident kernels.  k_tile holds a block's particles in registers: up to
 // kTileP of them on each SM, rows of at most kTileSlots neighbours.  k_loop
 // walks any number of tiles through memory.  Few particles leave most of the
@@ -1125,6 +1174,7 @@ static int plan_resident(dpg_system *s) {
             CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, q.threads, q.smem));
             if (occ < 1) return set_err(DPG_ERR_CUDA, "the resident loop does not fit an SM");
         }
+        if (n <= kClusterN) plan_cluster(s);
     }
     dpg_system::Plan &q = s->loop;
     if (s->mixed) q.lanes = per * 8 <= kLoopMaxTPB ? 8 : 1;
@@ -1158,7 +1208,13 @@ static int run_resident(dpg_system *s, int kind) {
     void *args[] = {(void *)&s->d, (void *)&s->lsync, (void *)&dt, (void *)&chunk, (void *)&most};
     do {
         CK(cudaMemsetAsync(s->lsync, 0, sizeof(LoopSync), s->stream));
-        CK(cudaLaunchCooperativeKernel(fn, dim3(q.blocks), dim3(q.threads), args, q.smem, s->stream));
+        if (q.cluster) {
+            cudaLaunchAttribute attr[1];
+            const cudaLaunchConfig_t cfg = cluster_config(q, s->stream, attr);
+            CK(cudaLaunchKernelExC(&cfg, fn, args));
+        } else {
+            CK(cudaLaunchCooperativeKernel(fn, dim3(q.blocks), dim3(q.threads), args, q.smem, s->stream));
+        }
         TRY(pull_state(s));
         if (s->hs->flags & kError) return set_err(DPG_ERR_TIMEOUT, "a grid barrier of the resident loop ran out");
     } while (!s->hs->flags);
