@@ -469,11 +469,22 @@ __global__ void k_drift(DevSys *ds, double dt) {
 
 // kernelMixVelocitiesAndForces (per-particle FIRE mix): src/particles/base/kernels.cu:91-112
 __device__ __forceinline__ double2 fire_mix(double2 v, double2 f, double alpha) {
-    double fn = sqrt(f.x * f.x + f.y * f.y);
-    double vn = sqrt(v.x * v.x + v.y * v.y);
+    const double f2 = f.x * f.x + f.y * f.y, v2 = v.x * v.x + v.y * v.y;
+    const bool nf = __double_as_longlong(f2) == 0, nv = __double_as_longlong(v2) == 0;
     double mix = 0.0;
-    if (fn > 1e-16) {
-        mix = vn / fn * alpha;
+    if ((nf || middling(f2)) && (nv || middling(v2))) {
+        double yf, yv;
+        const double fn = nf ? 0.0 : root_near(f2, yf);
+        // |F| > 1e-16 by the high word, exactly where that is the same
+        const int h = __double2hiint(fn);
+        if (h > 0x3c9cd2b2 || (h == 0x3c9cd2b2 && fn > 1e-16)) {
+            const double vn = root_near(v2, yv);
+            mix = nv ? 0.0 : div_near(vn, fn, yf) * alpha;
+        } else {
+            v.x = 0.0; v.y = 0.0;
+        }
+    } else if (const double fn = sqrt(f2); fn > 1e-16) {
+        mix = sqrt(v2) / fn * alpha;
     } else {
         v.x = 0.0; v.y = 0.0; mix = 0.0;
     }
@@ -1114,7 +1125,7 @@ __device__ __forceinline__ double2 nve_force(const DevSys *ds, int i, double2 u,
                                              double en, double &pe) {
     double2 f;
     const double g = ds->s.damping;
-    pe = 0.0 + en;
+    pe = en;  // 0 + en: a sum that starts at +0 is never -0
     if (ds->s.walls) {
         // NVE::wall_step (src/integrator/nve.cu:33-35): zero, wall forces,
         // then += the pair sum unless the particle has no neighbours
@@ -1123,13 +1134,13 @@ __device__ __forceinline__ double2 nve_force(const DevSys *ds, int i, double2 u,
         f = make_double2(0.0 + wx, 0.0 + wy);
         pe = 0.0 + ew;
         if (ds->w.count[i] != 0) { f.x += ax; f.y += ay; pe += en; }
-    } else if (g != 0.0) {
+    } else if (__double_as_longlong(g) << 1 != 0) {  // g != 0
         // DampedNVE::step (src/integrator/damped_nve.cu:22-23): F = 0 - g v,
         // then += the pair sum unless the particle has no neighbours
         f = make_double2(0.0 - g * u.x, 0.0 - g * u.y);
         if (ds->w.count[i] != 0) { f.x += ax; f.y += ay; }
     } else {
-        f = make_double2(0.0 + ax, 0.0 + ay);
+        f = make_double2(ax, ay);
     }
     return f;
 }

@@ -5,8 +5,8 @@
 //
 // What bounds the graph loop at 10^2 - 10^5 disks is neither memory nor
 // arithmetic but its nodes: ~25 us of an iteration's 32 - 40 us pass between
-// the kernels (measured: NVE of 1024 disks 38.6 us a step as a graph, 8.7 us
-// here; of 10007 mixed 36 -> 7; FIRE of 16384 disks 71 -> 22 us an iteration).
+// the kernels (measured: NVE of 1024 disks 38.6 us a step as a graph, 7.3 us
+// here; of 10007 mixed 36 -> 7; FIRE of 16384 disks 71 -> 20 us an iteration).
 // Here an NVE step costs one barrier (the kick that ends a step,
 // the next step's kick and its drift run in the same pass, into the other of
 // two position buffers) and a FIRE iteration two (its power decides the next
@@ -263,7 +263,25 @@ __device__ bool loop_rebuild(DevSys *ds, LoopSync *ls, unsigned &bk, int kind, R
     return true;
 }
 
+// 3 d2 > thr for d2 >= 0, decided on the high words (lim: that of thr / 3) but
+// for d2 next to the limit
+__device__ __forceinline__ bool beyond(double d2, int lim, double thr) {
+    const int h = __double2hiint(d2);
+    if (h < lim - 1) return false;
+    if (h > lim + 1 && h < 0x7ff00000) return true;
+    return 3.0 * d2 > thr;
+}
+
 // per-particle displacements since the list builds as barrier flags
+__device__ __forceinline__ unsigned long long move_flags(const DevParams &p, int lim_n, int lim_c, double nd2,
+                                                         double cd2) {
+    unsigned long long f = 0;
+    if (p.method == 0 && beyond(cd2, lim_c, p.cthr2)) f |= kNeedCell;
+    if (p.method != 2 && beyond(nd2, lim_n, p.nthr2)) f |= kNeedList;
+    return f;
+}
+
+// the same without kept limits
 __device__ __forceinline__ unsigned long long move_flags(const DevParams &p, double nd2, double cd2) {
     unsigned long long f = 0;
     if (p.method == 0 && 3.0 * cd2 > p.cthr2) f |= kNeedCell;
@@ -397,7 +415,7 @@ constexpr int kTileStride = kTileSlots + 1;
 struct TileMem {
     double *rl;           // [np][kTileStride] radius of each listed neighbour
     double *res;          // [3][qw] terms of the queued pairs
-    double *sum;          // [3][np] pair sums (FP32 pairs)
+    double *sum;          // [3][np] pair sums
     int *idx;             // [np][kTileStride] listed neighbours
     int *off;             // [np + 1] first queue entry of each particle
     unsigned short *ent;  // [qw] particle << 5 | slot
@@ -429,7 +447,12 @@ __device__ __forceinline__ TileMem tile_mem(unsigned char *base, int np) {
 // those that touch.  The contacts of the whole block form one queue (pair_sums
 // with a block for a warp), so the FP64 instructions run on full warps, and the
 // per-particle update runs on np / 32 warps whatever the lanes per neighbour
-// row.  Same arithmetic and order of sums as k_loop.
+// row.  A particle's three sums run on three threads, which for few particles
+// shares each addition among them; limits, kick factors and zeros are compared
+// as integers and a kick's or a mix's quotient is a quick one: with few warps a
+// block, every FP64 instruction of the update is ~64 clocks of the step (NVE of
+// 1024 disks 8.2 -> 7.3 us, FIRE of 16384 20.6 -> 19.6).  Same arithmetic and
+// order of sums as k_loop.
 template <int KIND, int G, bool M>
 __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *ls, double dt, int chunk,
                                                         long long iters) {
@@ -454,11 +477,15 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
     const int np = r.last - r.first, own = r.first + t;
     const bool mine = t < np;
     const double dt_half = 0.5 * dt;
+    const int lim_n = __double2hiint(p.nthr2 / 3.0), lim_c = __double2hiint(p.cthr2 / 3.0);
+    // the sums' threads: component t / np of particle t % np
+    const int sum_k = np > 0 ? t / np : 3, sum_g = np > 0 ? t % np : 0;
     unsigned bk = 0;
     bool ok = true, stored = false;
     long long it = 0;
 
     double2 x = {0.0, 0.0}, u = {0.0, 0.0}, f = {0.0, 0.0}, xn = {0.0, 0.0}, xc = {0.0, 0.0};
+    float rf = 0.f;
     double mass = 1.0, rad = 0.0, pe = 0.0, dtm = 0.0, dtm_of = 0.0;
     bool dtm_known = false;
     int gcnt = 0;  // row length of the group's particle
@@ -467,6 +494,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
             x = v.pos[own]; u = v.vel[own]; f = v.frc[own];
             xn = w.pos_n[own]; xc = w.pos_c[own];
             mass = v.mass[own]; rad = v.rad[own];
+            rf = (float)rad;
         }
         dtm_known = false;
         gcnt = g < np ? min(w.count[r.first + g], p.cap) : 0;
@@ -485,7 +513,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
     };
     // (h / mass), kept while h is the same
     auto kick_factor = [&](double h) {
-        if (!dtm_known || h != dtm_of) {
+        if (!dtm_known || __double_as_longlong(h) != __double_as_longlong(dtm_of)) {
             dtm = over_mass(h, mass);
             dtm_of = h;
             dtm_known = true;
@@ -496,9 +524,10 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
     auto publish = [&](double2 *pos, float4 *pk, uint4 *q) -> unsigned long long {
         pos[own] = x;
         if (M) pk[own] = mixed_pack(p, x, rad);
-        if (!M || (KIND == 0 && s.fp64_now)) q[own] = quant_of(p, x, rad);
-        const double dxn = x.x - xn.x, dyn = x.y - xn.y, dxc = x.x - xc.x, dyc = x.y - xc.y;
-        return move_flags(p, dxn * dxn + dyn * dyn, dxc * dxc + dyc * dyc);
+        if (!M || (KIND == 0 && s.fp64_now)) q[own] = quant_of(p, x, rf);
+        double d2[2];
+        moved2(x, xn, xc, d2);
+        return move_flags(p, lim_n, lim_c, d2[0], d2[1]);
     };
     auto nve_first = [&]() -> unsigned long long {
         if (!mine) return 0;
@@ -590,11 +619,8 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
                 m.sum[chunk + g] = ay;
                 m.sum[2 * chunk + g] = en;
             }
-            __syncthreads();
-            if (mine)
-#pragma unroll
-                for (int k = 0; k < 3; k++) acc[k] = m.sum[k * chunk + t];
         } else {
+            double sum = 0.0;
             const uint4 qi = v.q[g < np ? r.first + g : r.first];
             unsigned bits = 0;
             for (int k0 = 0; k0 < most; k0 += 4 * G) {
@@ -653,15 +679,19 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
                     m.res[2 * m.qw + e] = ee;
                 }
                 __syncthreads();
-                if (mine) {
-                    const int b0 = max(m.off[t], w0) - w0, b1 = min(m.off[t + 1], w1) - w0;
-                    for (int b = b0; b < b1; b++)
-#pragma unroll
-                        for (int k = 0; k < 3; k++) acc[k] += m.res[k * m.qw + b];
+                if (sum_k < 3) {
+                    const int b0 = max(m.off[sum_g], w0) - w0, b1 = min(m.off[sum_g + 1], w1) - w0;
+                    const double *res = m.res + sum_k * m.qw;
+                    for (int b = b0; b < b1; b++) sum += res[b];
                 }
                 if (w1 < total) __syncthreads();
             }
+            if (sum_k < 3) m.sum[sum_k * chunk + sum_g] = sum;
         }
+        __syncthreads();
+        if (mine)
+#pragma unroll
+            for (int k = 0; k < 3; k++) acc[k] = m.sum[k * chunk + t];
         // ---- kick (k_fire_force, k_nve_second)
         const bool last = KIND == 1 && (it + 1 >= iters || s.nve_steps_done + 1 >= s.max_steps);
         it++;
@@ -682,8 +712,8 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
         } else {
             double tot[3] = {0.0, 0.0, 0.0};
             if (mine) {
-                f = make_double2(0.0 + acc[0], 0.0 + acc[1]);
-                pe = 0.0 + acc[2];
+                f = make_double2(acc[0], acc[1]);
+                pe = acc[2];
                 const double h = kick_factor(s.f_dt / 2.0);
                 u.x = u.x + f.x * h;
                 u.y = u.y + f.y * h;
@@ -749,6 +779,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_loop(DevSys *ds, LoopSync *l
     bool ok = true;
     long long it = 0;
     const double dt_half = 0.5 * dt;
+    const int lim_n = __double2hiint(p.nthr2 / 3.0), lim_c = __double2hiint(p.cthr2 / 3.0);
 
     // NVE: the first half of a step, from the current into the other buffers
     auto drift_to_other = [&](int i, double2 u, double2 f, double dtm, unsigned long long &fl) {
@@ -762,9 +793,9 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_loop(DevSys *ds, LoopSync *l
         const double rad = v.rad[i];
         if (M) v.pk_t[i] = mixed_pack(p, x, rad);
         else v.q_t[i] = quant_of(p, x, rad);
-        const double2 a = w.pos_n[i], c = w.pos_c[i];
-        const double dxn = x.x - a.x, dyn = x.y - a.y, dxc = x.x - c.x, dyc = x.y - c.y;
-        fl |= move_flags(p, dxn * dxn + dyn * dyn, dxc * dxc + dyc * dyc);
+        double d2[2];
+        moved2(x, w.pos_n[i], w.pos_c[i], d2);
+        fl |= move_flags(p, lim_n, lim_c, d2[0], d2[1]);
     };
     auto swap_moved = [&]() {
         if (t == 0) {
@@ -813,9 +844,9 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_loop(DevSys *ds, LoopSync *l
                 const double rad = v.rad[i];
                 if (M) v.pk[i] = mixed_pack(p, x, rad);
                 if (!M || s.fp64_now) v.q[i] = quant_of(p, x, rad);
-                const double2 a = w.pos_n[i], c = w.pos_c[i];
-                const double dxn = x.x - a.x, dyn = x.y - a.y, dxc = x.x - c.x, dyc = x.y - c.y;
-                fl |= move_flags(p, dxn * dxn + dyn * dyn, dxc * dxc + dyc * dyc);
+                double d2[2];
+                moved2(x, w.pos_n[i], w.pos_c[i], d2);
+                fl |= move_flags(p, lim_n, lim_c, d2[0], d2[1]);
             }
             const unsigned long long bw = grid_bar(ls, bk, block_flags(fl));
             ok = bw != 0;
@@ -849,14 +880,14 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_loop(DevSys *ds, LoopSync *l
                 if (last) v.vel[i] = u;
                 else drift_to_other(i, u, frc, dtm, fl);
             } else {
-                const double2 frc = make_double2(0.0 + ax, 0.0 + ay);
+                const double2 frc = make_double2(ax, ay);
                 v.frc[i] = frc;
-                w.pe[i] = 0.0 + en;
+                w.pe[i] = en;
                 const double dtm = over_mass(s.f_dt / 2.0, v.mass[i]);
                 u.x = u.x + frc.x * dtm;
                 u.y = u.y + frc.y * dtm;
                 v.vel[i] = u;
-                tot[0] += 0.0 + en;
+                tot[0] += en;
                 tot[1] += frc.x * u.x + frc.y * u.y;
                 tot[2] = fmax(tot[2], frc.x * frc.x + frc.y * frc.y);
             }
