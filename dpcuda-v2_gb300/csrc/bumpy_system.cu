@@ -311,20 +311,20 @@ extern "C" int dpg_bumpy_get_bodies(dpg_bumpy_handle s, double *x, double *y, do
     for (int k = 0; k < 3; k++) {
         if (!xy[k][0] && !xy[k][1]) continue;
         LAUNCH(k_get_xy, s->gb(s->nb), kTPB, &s->d->b, k, d0, d1);
-        if (xy[k][0]) CK(cudaMemcpyAsync(xy[k][0], d0, nb8, cudaMemcpyDeviceToHost, s->stream));
-        if (xy[k][1]) CK(cudaMemcpyAsync(xy[k][1], d1, nb8, cudaMemcpyDeviceToHost, s->stream));
+        if (xy[k][0]) CK(copy_out(xy[k][0], d0, nb8, s->stream));
+        if (xy[k][1]) CK(copy_out(xy[k][1], d1, nb8, s->stream));
         CK(cudaStreamSynchronize(s->stream));
     }
     double *sc[4] = {angle, omega, torque, inertia};
     for (int k = 0; k < 4; k++) {
         if (!sc[k]) continue;
         LAUNCH(kb_get_body_scalar, s->gb(s->nb), kTPB, s->d, k, d0);
-        CK(cudaMemcpyAsync(sc[k], d0, nb8, cudaMemcpyDeviceToHost, s->stream));
+        CK(copy_out(sc[k], d0, nb8, s->stream));
         CK(cudaStreamSynchronize(s->stream));
     }
     if (pe) {
         LAUNCH(k_get_pe, s->gb(s->nb), kTPB, &s->d->b, d0);
-        CK(cudaMemcpyAsync(pe, d0, nb8, cudaMemcpyDeviceToHost, s->stream));
+        CK(copy_out(pe, d0, nb8, s->stream));
         CK(cudaStreamSynchronize(s->stream));
     }
     return DPG_OK;
@@ -335,8 +335,8 @@ extern "C" int dpg_bumpy_get_vertices(dpg_bumpy_handle s, double *px, double *py
     size_t n = std::max(s->nb, s->nv);
     double *d0 = s->xfer, *d1 = s->xfer + n;
     LAUNCH(kb_get_vertices, s->gb(s->nv), kTPB, s->d, d0, d1);
-    if (px) CK(cudaMemcpyAsync(px, d0, 8 * (size_t)s->nv, cudaMemcpyDeviceToHost, s->stream));
-    if (py) CK(cudaMemcpyAsync(py, d1, 8 * (size_t)s->nv, cudaMemcpyDeviceToHost, s->stream));
+    if (px) CK(copy_out(px, d0, 8 * (size_t)s->nv, s->stream));
+    if (py) CK(copy_out(py, d1, 8 * (size_t)s->nv, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     return DPG_OK;
 }

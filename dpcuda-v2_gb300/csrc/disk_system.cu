@@ -468,8 +468,8 @@ extern "C" int dpg_get_state(dpg_handle s, double *x, double *y, double *vx, dou
         } else {
             double *sx = s->xfer, *sy = s->xfer + s->n;
             LAUNCH(k_get_xy, s->grid(s->n), s->tpb, s->d, k, ox ? sx : nullptr, oy ? sy : nullptr);
-            if (ox) CK(cudaMemcpyAsync(ox, sx, nb, cudaMemcpyDeviceToHost, s->stream));
-            if (oy) CK(cudaMemcpyAsync(oy, sy, nb, cudaMemcpyDeviceToHost, s->stream));
+            if (ox) CK(copy_out(ox, sx, nb, s->stream));
+            if (oy) CK(copy_out(oy, sy, nb, s->stream));
             CK(cudaStreamSynchronize(s->stream));
         }
     }
@@ -477,7 +477,7 @@ extern "C" int dpg_get_state(dpg_handle s, double *x, double *y, double *vx, dou
         double *dst = where == DPG_DEVICE ? pe : s->xfer;
         LAUNCH(k_get_pe, s->grid(s->n), s->tpb, s->d, dst);
         if (where == DPG_HOST) {
-            CK(cudaMemcpyAsync(pe, dst, nb, cudaMemcpyDeviceToHost, s->stream));
+            CK(copy_out(pe, dst, nb, s->stream));
             CK(cudaStreamSynchronize(s->stream));
         }
     }

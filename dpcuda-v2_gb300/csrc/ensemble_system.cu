@@ -258,7 +258,7 @@ extern "C" int dpg_ensemble_get_state(dpg_ensemble s, double *x, double *y, doub
     LAUNCH(e_get, (s->T + 255) / 256, 256, s->d, x ? s->xfer : nullptr, y ? s->xfer + n : nullptr,
            fx ? s->xfer + 2 * n : nullptr, fy ? s->xfer + 3 * n : nullptr, s->d_src);
     for (int k = 0; k < 4; k++)
-        if (dst[k]) CK(cudaMemcpyAsync(dst[k], s->xfer + k * n, 8 * n, cudaMemcpyDeviceToHost, s->stream));
+        if (dst[k]) CK(copy_out(dst[k], s->xfer + k * n, 8 * n, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     return DPG_OK;
 }
