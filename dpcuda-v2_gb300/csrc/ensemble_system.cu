@@ -44,12 +44,12 @@ struct dpg_ensemble_system {
     bool split_force = false;    // grid form: FP32 and refinement force kernels apart
     long long launches = 0;      // kernel launches and graph launches issued for this ensemble
     // resident form: one stream per size class, the block -> system lists
-    static constexpr int kShapes = 13;
+    static constexpr int kShapes = 17;
     cudaStream_t rs_stream[kShapes] = {};
     cudaEvent_t rs_fork = nullptr, rs_join[kShapes] = {};
     int rs_fit[kShapes] = {};    // clusters of each class the GPU holds at once (0: not yet asked)
     int rs_rot[kShapes] = {};    // rotation of each class's systems between launches
-    bool rs_wide = true;         // the wide table of shapes (see kRClasses)
+    int rs_table = 0;            // the table of shapes (see kResTables)
     int *d_rs_blocks = nullptr;
 };
 
@@ -471,27 +471,27 @@ typedef void (*res_kernel_fn)(EDev *, const int *, int, int, long long, unsigned
 // Shapes (warps per block, particles per warp and pass, passes, blocks per
 // cluster): a system goes to the first shape of its table that holds it.  The
 // wide table spreads a system over many blocks and lanes, which shortens its
-// iterations; the dense one packs it into few, which takes fewer instructions
-// in all and lets more systems share the GPU.  No result depends on the shape.
-// Per iteration wide / dense, one system of 100 disks 3.5 / 4.2 us, of 900 5.4 /
-// 7.6; many (systems x disks), dense against the former shapes: 400 x 100 8.7 /
-// 13.8, 300 x 400 17.7 / 21.6, 160 x 900 26 / 41, 60 x 1500 18 / 21, 40 x 3000
-// 32 / 44 (wide: 15.8, 72, 95, 26, 41).
+// iterations; the later ones pack it into fewer SMs, so that more systems run
+// side by side.  No result depends on the shape.
 struct RClass {
     int w, p, r, c;
     res_kernel_fn fn;
     int per_block() const { return w * p * r; }
     int capacity() const { return per_block() * c; }
 };
-constexpr int kNClass = 13;
+constexpr int kNClass = 17;
 #define RC(W, P, R, C) {W, P, R, C, e_res<W, P, R, ((C) > 1)>}
 static const RClass kRClasses[kNClass] = {
     RC(16, 8, 1, 1),  RC(16, 8, 1, 2),  RC(16, 8, 1, 4), RC(16, 8, 1, 8), RC(16, 32, 1, 4), RC(16, 32, 1, 8),
     RC(16, 32, 4, 8), RC(4, 32, 1, 1),  RC(8, 32, 1, 1), RC(8, 32, 2, 1), RC(8, 32, 2, 2),  RC(8, 32, 2, 4),
-    RC(8, 32, 2, 8)};
+    RC(8, 32, 2, 8),  RC(8, 16, 1, 1),  RC(16, 16, 1, 1), RC(16, 32, 1, 1), RC(16, 32, 1, 2)};
 #undef RC
-constexpr int kNTable = 7;
-static const int kResWide[kNTable] = {0, 1, 2, 3, 4, 5, 6}, kResDense[kNTable] = {7, 8, 9, 10, 11, 12, 6};
+constexpr int kNTable = 7, kNTables = 5;
+static const int kResTables[kNTables][kNTable] = {{0, 1, 2, 3, 4, 5, 6},      // wide
+                                                  {0, 14, 15, 16, 4, 5, 6},   // a block of 16 warps
+                                                  {13, 8, 15, 16, 4, 5, 6},   // half a block for the small
+                                                  {7, 8, 15, 16, 4, 5, 6},    // a quarter
+                                                  {7, 8, 9, 10, 11, 12, 6}};  // dense
 
 static int res_class_in(const int *table, int n) {
     for (int k = 0; k < kNTable; k++)
@@ -499,7 +499,7 @@ static int res_class_in(const int *table, int n) {
     return -1;
 }
 static int res_class_of(const ES *s, int n) {
-    return res_class_in(s->rs_wide ? kResWide : kResDense, n);
+    return res_class_in(kResTables[s->rs_table], n);
 }
 
 // largest cell count and system of class c
@@ -534,18 +534,35 @@ static bool res_table_fits(const ES *s) {
     return true;
 }
 
-// the resident form holds every system: sizes and shared memory within limits.
-// Chooses the table: the wide one while its blocks (one an SM) leave an eighth
-// of the SMs for what clusters cannot use, the dense one beyond, where systems
-// would have to take turns, unless only the wide one's smaller blocks fit.
-static bool res_fits(ES *s) {
-    if (s->max_n > kResMaxN) return false;
+// The table: the first whose blocks find room at once, by the SMs they take (a
+// block of 16 warps one, of 8 half of one, a third at 80 registers); the wide one
+// has to leave an eighth of them for what clusters cannot use; else the dense
+// one.  Only live systems count: what is left of a batch spreads out again.
+// Iterations of the batch in 0.1 s, former shapes -> dense table alone -> these:
+// 300 systems of 64 - 128 disks 3.5e6 -> 3.4e6 -> 4.1e6, 150 of 257 - 512 2.1e6 ->
+// 1.8e6 -> 2.3e6; of 129 - 256 3.9e6 in all.
+static void res_choose(ES *s, bool live) {
     int dev = 0, nsm = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    long long blocks = 0;
-    for (const auto &y : s->sys) blocks += kRClasses[res_class_in(kResWide, y.n)].c;
-    s->rs_wide = blocks <= nsm / 8 * 7;
-    if (!s->rs_wide && !res_table_fits(s)) s->rs_wide = true;
+    const int was = s->rs_table;
+    for (s->rs_table = 0; s->rs_table + 1 < kNTables; s->rs_table++) {
+        double sms = 0;
+        for (const auto &y : s->sys) {
+            if (live && y.phase == kIdle) continue;
+            const RClass &K = kRClasses[res_class_of(s, y.n)];
+            sms += K.c * (K.w == 8 && K.r == 1 && K.p == 32 ? 1.0 / 3 : K.w / 16.0);
+        }
+        if (sms <= (s->rs_table ? nsm : nsm / 8 * 7)) break;
+    }
+    while (s->rs_table > 0 && !res_table_fits(s)) s->rs_table--;
+    if (s->rs_table != was) std::fill(std::begin(s->rs_fit), std::end(s->rs_fit), 0);
+}
+
+// the resident form holds every system: sizes and shared memory within limits
+// (the wide table's blocks are the smallest)
+static bool res_fits(ES *s) {
+    if (s->max_n > kResMaxN) return false;
+    res_choose(s, false);
     return res_table_fits(s);
 }
 
@@ -696,6 +713,7 @@ static int run_resident(ES *s, long long guard_limit) {
         if (most > guard_limit) return set_err(DPG_ERR_NOT_CONVERGED, "ensemble loop budget spent");
         if (sum == last_sum) return set_err(DPG_ERR_STATE, "resident launch made no progress");
         last_sum = sum;
+        res_choose(s, true);
         int nl = 0;
         TRY(launch_resident(s, kChunk, kSlice, (unsigned long long)turn, &nl));
         turn = std::min(1.07 * turn, (double)kSlice);
