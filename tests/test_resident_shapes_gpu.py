@@ -98,3 +98,14 @@ def test_cell_grids_that_fit(dpg, n, side, fits):
         with pytest.raises(Exception):
             e.setForm(FORM_RESIDENT)
     e.close()
+
+
+@pytest.mark.parametrize("n,copies", [(100, 140), (100, 290), (100, 500), (250, 140), (250, 290), (400, 140), (400, 200)])
+def test_every_table_gives_the_same_bits(dpg, n, copies):
+    """Batches of equal systems that fill half an SM, a third or a quarter each,
+    or more than there is: every copy is the system alone."""
+    st = packing(n, 500 + n)
+    alone, _ = run(dpg, [st], 100)
+    batch, _ = run(dpg, [st] * copies, 100)
+    for c in ("x", "y", "fx", "fy"):
+        np.testing.assert_array_equal(batch[c].reshape(copies, n), np.tile(alone[c], (copies, 1)), err_msg=c)
