@@ -36,7 +36,10 @@ __device__ __forceinline__ bool bumpy_rebuild(BumpySys *bs, LoopSync *ls, unsign
             atomicAdd(&d.w.cell_cnt[cell], 1);
         }
         if (!grid_bar(ls, bk, 0)) return false;
-        if (blockIdx.x == 0) cell_scan_block(d.w.cell_cnt, d.w.cell_start, p.ncells);
+        if (blockIdx.x == 0) {
+            const int all = scan_block(d.w.cell_cnt, d.w.cell_start, p.ncells);
+            if (t == 0) d.w.cell_start[p.ncells] = all;
+        }
         if (!grid_bar(ls, bk, 0)) return false;
         for (int i = r.first + t; i < r.last; i += nt) {
             const int c = d.w.cell_raw[i];
@@ -47,7 +50,7 @@ __device__ __forceinline__ bool bumpy_rebuild(BumpySys *bs, LoopSync *ls, unsign
         if (!grid_bar(ls, bk, 0)) return false;
         for (int i = r.first + t; i < r.last; i += nt) reorder_body(bs, i);
         if (!grid_bar(ls, bk, 0)) return false;
-        if (blockIdx.x == 0) cell_scan_block(x.nvb_t, x.start_t, p.n);
+        if (blockIdx.x == 0) scan_block(x.nvb_t, x.start_t, p.n);  // starts only: the array has no n + 1st
         if (!grid_bar(ls, bk, 0)) return false;
         for (int i = r.first + t / 32; i < r.last; i += nt / 32) reorder_vertices(bs, i, t & 31);
         if (!grid_bar(ls, bk, 0)) return false;
@@ -265,7 +268,8 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) kb_loop(BumpySys *bs, LoopSync
         if (t < np) m.vfirst[t] = x.start[r.first + t] - v0;
         if (t == 0) m.vfirst[np] = nv;
         __syncthreads();
-        cell_scan_block(m.count, m.row, nv);
+        const int rows = scan_block(m.count, m.row, nv);
+        if (t == 0) m.row[nv] = rows;
         __syncthreads();
         if (m.row[nv] <= kVertRows)
             for (int k = t; k < nv; k += nt)
@@ -437,10 +441,12 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) kb_loop(BumpySys *bs, LoopSync
             }
         }
         __syncthreads();
-        cell_scan_block(m.count, m.before, words);
-        if (t == 0 && (rows & 31) == 0) m.touch[words] = 0;  // rank(rows) reads this word
+        const int entries = scan_block(m.count, m.before, words);
+        if (t == 0) {  // rank(rows) reads these words
+            m.before[words] = entries;
+            if ((rows & 31) == 0) m.touch[words] = 0;
+        }
         __syncthreads();
-        const int entries = m.before[words];
         // the vertices that have a term
         const int vwords = (nv + 31) / 32;
         for (int w = wid; w < vwords; w += nw) {

@@ -97,17 +97,19 @@ __device__ __forceinline__ unsigned long long grid_bar(LoopSync *ls, unsigned &k
     return done;
 }
 
-// exclusive scan of the cell counts by one block (the arithmetic of k_cell_scan)
-__device__ __forceinline__ void cell_scan_block(const int *cnt, int *start, int ncells) {
+// Exclusive scan of n counts into start[0 .. n) by one block (the arithmetic of
+// k_cell_scan).  Returns the total on every thread; a caller whose array holds
+// n + 1 values stores it there itself.
+__device__ __forceinline__ int scan_block(const int *cnt, int *start, int n) {
     __shared__ int wsum[32];
     __shared__ int carry_s;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     int carry = 0;
-    for (int base = 0; base < ncells; base += 4 * blockDim.x) {
+    for (int base = 0; base < n; base += 4 * blockDim.x) {
         const int idx = base + 4 * threadIdx.x;
         int a[4];
 #pragma unroll
-        for (int k = 0; k < 4; k++) a[k] = idx + k < ncells ? cnt[idx + k] : 0;
+        for (int k = 0; k < 4; k++) a[k] = idx + k < n ? cnt[idx + k] : 0;
         const int t = a[0] + a[1] + a[2] + a[3];
         int incl = t;
 #pragma unroll
@@ -132,13 +134,13 @@ __device__ __forceinline__ void cell_scan_block(const int *cnt, int *start, int 
         int ex = carry + wsum[wid] + incl - t;
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            if (idx + k < ncells) start[idx + k] = ex;
+            if (idx + k < n) start[idx + k] = ex;
             ex += a[k];
         }
         carry += carry_s;
         __syncthreads();
     }
-    if (threadIdx.x == 0) start[ncells] = carry;
+    return carry;
 }
 
 // a block's slots and the tiles it walks them in: every thread runs the same
@@ -178,7 +180,10 @@ __device__ bool loop_rebuild(DevSys *ds, LoopSync *ls, unsigned &bk, int kind, R
             atomicAdd(&ds->w.cell_cnt[c], 1);
         }
         if (!grid_bar(ls, bk, 0)) return false;
-        if (blockIdx.x == 0) cell_scan_block(ds->w.cell_cnt, ds->w.cell_start, p.ncells);
+        if (blockIdx.x == 0) {
+            const int all = scan_block(ds->w.cell_cnt, ds->w.cell_start, p.ncells);
+            if (t == 0) ds->w.cell_start[p.ncells] = all;
+        }
         if (!grid_bar(ls, bk, 0)) return false;
         for (int i = r.first + t; i < r.last; i += nt) {
             const int c = ds->w.cell_raw[i];
