@@ -42,6 +42,7 @@ struct dpg_bumpy_system {
     double *xfer = nullptr;
     int mode = 2;  // 3 resident grid, 2 graph, 0 separate launches
     LoopSync *lsync = nullptr;          // resident grid: barrier state,
+    int polls = kBarPolls;              // looks before a barrier gives up,
     int lblocks = 0, lchunk = 0;        // blocks, bodies a block
     int max_nvb = 0;                    // most vertices of a body
     cudaGraphExec_t loop_exec[2] = {nullptr, nullptr};
@@ -142,6 +143,7 @@ extern "C" int dpg_bumpy_create(const dpg_bumpy_params *p, void *cuda_stream, dp
     const char *m = getenv("DPG_LOOP_MODE");
     if (m && (!strcmp(m, "stream") || !strcmp(m, "graph"))) s->mode = 0;
     else if (!(m && !strcmp(m, "cond"))) s->mode = 3;
+    if (const char *q = getenv("DPG_LOOP_POLLS")) s->polls = std::max(1, atoi(q));
     const size_t nb = s->nb, nv = s->nv;
     int rc = DPG_OK;
     auto A = [&](void **pp, size_t b) { if (rc == DPG_OK) rc = balloc(s, pp, b); };
@@ -790,18 +792,27 @@ static bool resident_holds(const BS *s) {
     return s->capv <= kVertSlots && (long long)s->lchunk * s->max_nvb <= kBodyVerts;
 }
 
+// A barrier failed: the bodies stand at different points of an iteration, so the
+// lists are gone until dpg_bumpy_setup_neighbors lays them out again.
+static int loop_failed(BS *s) {
+    s->have_neighbors = false;
+    TRY(put(s, &s->d->b.s.flags, 0));
+    return set_err(DPG_ERR_TIMEOUT, "a grid barrier of the resident loop ran out");
+}
+
 static int run_resident(BS *s, int kind) {
     void *fn = kind == 0 ? (void *)kb_loop<0> : (void *)kb_loop<1>;
     long long most = std::max<long long>(256, (1LL << 24) / (s->nb + 1024));
     double dt = s->loop_dt, tmax = s->loop_tmax;
-    void *args[] = {(void *)&s->d, (void *)&s->lsync, (void *)&dt, (void *)&tmax, (void *)&s->lchunk, (void *)&most};
+    void *args[] = {(void *)&s->d, (void *)&s->lsync, (void *)&dt, (void *)&tmax, (void *)&s->lchunk, (void *)&most,
+                    (void *)&s->polls};
     // 8 warps for the roles and the list builds, more where the vertices fill them
     const int threads = (long long)s->lchunk * s->max_nvb > 256 ? kLoopMaxTPB : 256;
     do {
         CK(cudaMemsetAsync(s->lsync, 0, sizeof(LoopSync), s->stream));
         CK(cudaLaunchCooperativeKernel(fn, dim3(s->lblocks), dim3(threads), args, sizeof(BodyMem), s->stream));
         TRY(pull(s));
-        if (s->hs->flags & kError) return set_err(DPG_ERR_TIMEOUT, "a grid barrier of the resident loop ran out");
+        if (s->hs->flags & kError) return loop_failed(s);
     } while (!s->hs->flags);
     return DPG_OK;
 }

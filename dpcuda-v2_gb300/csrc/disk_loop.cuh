@@ -17,9 +17,12 @@
 // the state back.  Block b owns the slots [b * chunk, (b + 1) * chunk).  Data
 // that other blocks write is read with ordinary loads after a barrier (the
 // acquire of the barrier's last poll, then __syncthreads); nothing here may be
-// read through the non-coherent path.  Every wait is bounded: a block whose
-// barrier does not complete sets LoopSync.err and leaves, and so does every
-// other block at its own limit.
+// read through the non-coherent path.  The waits of the grid barrier through L2
+// are bounded: a block whose barrier does not complete closes it, so that it
+// fails for every block alike and none goes on with data that another has not
+// written; all leave, and the call returns DPG_ERR_TIMEOUT.  A grid of one
+// cluster uses the hardware's cluster barrier, which has no limit (its blocks
+// are all resident or none is).
 #pragma once
 #include <cooperative_groups.h>
 
@@ -31,11 +34,11 @@ namespace {
 constexpr int kLoopMaxTPB = 512;
 constexpr int kClusterMax = 16;      // blocks of a cluster at most
 constexpr int kLoopBlocksMax = 160;  // blocks of a FIRE loop at most
-constexpr long long kBarPolls = 1LL << 22;  // ~1 s of polls
+constexpr int kBarPolls = 1 << 22;   // ~1 s of polls (DPG_LOOP_POLLS sets another limit)
 
 struct LoopSync {
     unsigned long long ring[4];  // barrier k uses ring[k & 3]: arrivals and flag counts
-    int err;                     // a barrier ran out of polls
+    int err;                     // a barrier failed: read by block 0 as it leaves
     int max_count;               // longest neighbour row of the last list build
     int max_vcount;              // longest vertex row (rigid bodies)
 };
@@ -43,57 +46,72 @@ struct LoopSync {
 // what a barrier carries besides the arrival count (bits 0 - 15): how many
 // blocks raised each flag
 constexpr unsigned long long kNeedList = 1ULL << 16, kNeedCell = 1ULL << 32, kFull = 1ULL << 48;
+constexpr unsigned long long kClosed = 1ULL << 63;  // the barrier failed (block counts stay below 2^9)
 __device__ __forceinline__ bool raised(unsigned long long v, unsigned long long flag) {
     return (v / flag & 0xffff) != 0;
 }
 
-// Grid barrier k; flags of thread 0 are added to the arrival.  Returns the
-// completed word (arrivals and flag counts) on every thread, 0 if the wait ran
-// out.  Barrier k + 2's word is cleared by block 0 once barrier k is complete:
-// every block has then left barrier k - 2, the word's last use, and reaches
-// k + 2 only after block 0's arrival at k + 1.
+// What a block knows of its barriers: the next one's number, and how often a
+// wait looks before it gives up.
+struct GridBar {
+    unsigned k;
+    int polls;
+};
+
+// Grid barrier bar.k; flags of thread 0 are added to the arrival.  Returns the
+// completed word (arrivals and flag counts) on every thread, 0 if the barrier
+// failed.  A block whose polls run out closes the word by compare-and-swap, which
+// succeeds only while arrivals are missing, and a closed word stays so: a
+// barrier completes for all blocks or fails for all.  Barrier k + 2's word is
+// cleared by block 0 once barrier k is complete: every block has then left
+// barrier k - 2, the word's last use, and reaches k + 2 only after block 0's
+// arrival at k + 1.
 // A grid of one thread-block cluster uses the cluster's barrier, the flags going
 // to every block's shared memory before it (two sets in turn: a block that
 // writes one again has passed a barrier that its readers entered later).
-__device__ __forceinline__ unsigned long long grid_bar(LoopSync *ls, unsigned &k, unsigned long long flags) {
+__device__ __forceinline__ unsigned long long grid_bar(LoopSync *ls, GridBar &bar, unsigned long long flags) {
     __shared__ unsigned long long done, said[2][kClusterMax];
     const auto cluster = cooperative_groups::this_cluster();
     if (cluster.num_blocks() > 1) {
         const int nb = (int)cluster.num_blocks(), t = threadIdx.x;
         flags = __shfl_sync(0xffffffffu, flags, 0);
-        if (t < nb) *cluster.map_shared_rank(&said[k & 1][cluster.block_rank()], t) = 1ULL + flags;
+        if (t < nb) *cluster.map_shared_rank(&said[bar.k & 1][cluster.block_rank()], t) = 1ULL + flags;
         cluster.sync();
         if (t < 32) {
-            unsigned long long v = t < nb ? said[k & 1][t] : 0;
+            unsigned long long v = t < nb ? said[bar.k & 1][t] : 0;
 #pragma unroll
             for (int o = kClusterMax / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
             if (t == 0) done = v;
         }
         __syncthreads();
-        k++;
+        bar.k++;
         return done;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        unsigned long long *w = &ls->ring[k & 3], v;
+        unsigned long long *w = &ls->ring[bar.k & 3], v;
         __threadfence();
         atomicAdd(w, 1ULL + flags);
-        long long polls = 0;
+        int polls = 0;
         do {
             asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(w) : "memory");
-        } while ((v & 0xffff) < gridDim.x && ++polls < kBarPolls);
-        if ((v & 0xffff) < gridDim.x) {
-            atomicExch(&ls->err, 1);
-            v = 0;
+        } while ((v & 0xffff) < gridDim.x && !(v & kClosed) && ++polls < bar.polls);
+        while ((v & 0xffff) < gridDim.x && !(v & kClosed)) {  // run out; an arrival makes it look again
+            const unsigned long long seen = atomicCAS(w, v, v | kClosed);
+            v = seen == v ? v | kClosed : seen;
+            __threadfence();
         }
-        if (blockIdx.x == 0) {
-            ls->ring[(k + 2) & 3] = 0;
+        if (v & kClosed) {
+            *(volatile int *)&ls->err = 1;
+            v = 0;
+        } else if (blockIdx.x == 0) {
+            ls->ring[(bar.k + 2) & 3] = 0;
             __threadfence();
         }
         done = v;
     }
     __syncthreads();
-    k++;
+    bar.k++;
     return done;
 }
 
@@ -167,7 +185,7 @@ __device__ __forceinline__ int nlist_all_row(const DevSys *ds, int i) {
 // Returns false if the loop has to leave (a row longer than the capacity, or a
 // barrier that ran out).
 template <bool M>
-__device__ bool loop_rebuild(DevSys *ds, LoopSync *ls, unsigned &bk, int kind, Range r) {
+__device__ bool loop_rebuild(DevSys *ds, LoopSync *ls, GridBar &bar, int kind, Range r) {
     const DevParams &p = ds->p;
     DevView &v = ds->v;
     DevState &s = ds->s;
@@ -179,19 +197,19 @@ __device__ bool loop_rebuild(DevSys *ds, LoopSync *ls, unsigned &bk, int kind, R
             ds->w.cell_raw[i] = c;
             atomicAdd(&ds->w.cell_cnt[c], 1);
         }
-        if (!grid_bar(ls, bk, 0)) return false;
+        if (!grid_bar(ls, bar, 0)) return false;
         if (blockIdx.x == 0) {
             const int all = scan_block(ds->w.cell_cnt, ds->w.cell_start, p.ncells);
             if (t == 0) ds->w.cell_start[p.ncells] = all;
         }
-        if (!grid_bar(ls, bk, 0)) return false;
+        if (!grid_bar(ls, bar, 0)) return false;
         for (int i = r.first + t; i < r.last; i += nt) {
             const int c = ds->w.cell_raw[i];
             ds->w.perm[ds->w.cell_start[c] + atomicAdd(&ds->w.cell_cur[c], 1)] = i;
         }
-        if (!grid_bar(ls, bk, 0)) return false;
+        if (!grid_bar(ls, bar, 0)) return false;
         for (int c = blockIdx.x * nt + t; c < p.ncells; c += gridDim.x * nt) cell_sort_one(ds, c);
-        if (!grid_bar(ls, bk, 0)) return false;
+        if (!grid_bar(ls, bar, 0)) return false;
         for (int i = r.first + t; i < r.last; i += nt) {
             const int o = ds->w.perm[i];
             const double2 x = v.pos[o];
@@ -206,7 +224,7 @@ __device__ bool loop_rebuild(DevSys *ds, LoopSync *ls, unsigned &bk, int kind, R
             ds->w.cell_of[i] = ds->w.cell_raw[o];
             ds->w.pos_c[i] = x;
         }
-        if (!grid_bar(ls, bk, 0)) return false;
+        if (!grid_bar(ls, bar, 0)) return false;
         if (t == 0) {
             swap_ptr(v.pos, v.pos_t);
             swap_ptr(v.vel, v.vel_t);
@@ -221,7 +239,7 @@ __device__ bool loop_rebuild(DevSys *ds, LoopSync *ls, unsigned &bk, int kind, R
         __syncthreads();
     } else if (M) {
         for (int i = r.first + t; i < r.last; i += nt) v.q[i] = quant_of(p, v.pos[i], v.rad[i]);
-        if (!grid_bar(ls, bk, 0)) return false;
+        if (!grid_bar(ls, bar, 0)) return false;
     }
     int mx = 0;
     if (p.method == 0) {
@@ -254,7 +272,7 @@ __device__ bool loop_rebuild(DevSys *ds, LoopSync *ls, unsigned &bk, int kind, R
     if ((t & 31) == 0) atomicMax(&bmx, mx);
     __syncthreads();
     if (t == 0) atomicMax(&ls->max_count, bmx);
-    const unsigned long long w = grid_bar(ls, bk, bmx > p.cap ? kFull : 0);
+    const unsigned long long w = grid_bar(ls, bar, bmx > p.cap ? kFull : 0);
     if (!w) return false;
     if (t == 0) {
         s.n_rebuilds++;
@@ -320,7 +338,7 @@ __device__ __forceinline__ void warp_totals(double &sum, double (&mx)[K - 2]) {
         for (int k = 0; k < K - 2; k++) mx[k] = max_pos(mx[k], __shfl_down_sync(0xffffffffu, mx[k], o));
 }
 template <int K>
-__device__ __forceinline__ bool grid_totals(double (&v)[K], int nwr, double *part, LoopSync *ls, unsigned &bk,
+__device__ __forceinline__ bool grid_totals(double (&v)[K], int nwr, double *part, LoopSync *ls, GridBar &bar,
                                             double *sm) {
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nb = gridDim.x;
     double mx[K - 2], sum;
@@ -342,7 +360,7 @@ __device__ __forceinline__ bool grid_totals(double (&v)[K], int nwr, double *par
         for (int w = 1; w < nwr; w++) a = t < 2 ? a + sm[w * K + t] : max_pos(a, sm[w * K + t]);
         part[t * nb + blockIdx.x] = a;
     }
-    if (!grid_bar(ls, bk, 0)) return false;
+    if (!grid_bar(ls, bar, 0)) return false;
     if (wid == 0) {
         // all loads in flight at once (one trip to L2), then added in order
         const double *mine = part + (lane < 16 ? 0 : nb);
@@ -376,7 +394,7 @@ __device__ __forceinline__ bool grid_totals(double (&v)[K], int nwr, double *par
 // End of a resident loop: the displacement maxima of the last move (zero where
 // a build followed), after every block has handed in its own.  True on thread 0
 // of block 0, which then writes its copy of the system back.
-__device__ __forceinline__ bool loop_exit(DevSys *L, LoopSync *ls, unsigned &bk, Range r, double *red) {
+__device__ __forceinline__ bool loop_exit(DevSys *L, LoopSync *ls, GridBar &bar, Range r, double *red) {
     const int t = threadIdx.x, nb = gridDim.x;
     double m[2] = {0.0, 0.0};
     for (int i = r.first + t; i < r.last; i += blockDim.x) {
@@ -392,7 +410,7 @@ __device__ __forceinline__ bool loop_exit(DevSys *L, LoopSync *ls, unsigned &bk,
         part[blockIdx.x] = m[0];
         part[nb + blockIdx.x] = m[1];
     }
-    const bool all = grid_bar(ls, bk, 0) != 0;
+    const bool all = grid_bar(ls, bar, 0) != 0;
     if (blockIdx.x != 0) return false;
     m[0] = 0.0;
     m[1] = 0.0;
@@ -406,7 +424,8 @@ __device__ __forceinline__ bool loop_exit(DevSys *L, LoopSync *ls, unsigned &bk,
         L->s.max_nd2 = m[0];
         L->s.max_cd2 = m[1];
         L->s.rebuild = 0;
-        if (!all) L->s.flags |= kError;
+        // a barrier fails for every block alike: this thread has set err then
+        if (!all || *(volatile int *)&ls->err) L->s.flags |= kError;
     }
     return t == 0;
 }
@@ -460,7 +479,7 @@ __device__ __forceinline__ TileMem tile_mem(unsigned char *base, int np) {
 // order of sums as k_loop.
 template <int KIND, int G, bool M>
 __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *ls, double dt, int chunk,
-                                                        long long iters) {
+                                                        long long iters, int polls) {
     extern __shared__ __align__(16) unsigned char loop_smem[];
     __shared__ DevSys L;
     __shared__ double red[32 * 3];
@@ -485,7 +504,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
     const int lim_n = __double2hiint(p.nthr2 / 3.0), lim_c = __double2hiint(p.cthr2 / 3.0);
     // the sums' threads: component t / np of particle t % np
     const int sum_k = np > 0 ? t / np : 3, sum_g = np > 0 ? t % np : 0;
-    unsigned bk = 0;
+    GridBar bar = {0, polls};
     bool ok = true, stored = false;
     long long it = 0;
 
@@ -546,7 +565,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
     // the barrier after a move, the buffer swap (NVE) and a rebuild if any
     // particle asks for one; false: leave
     auto after_move = [&](unsigned long long fl) {
-        const unsigned long long bw = grid_bar(ls, bk, block_flags(fl));
+        const unsigned long long bw = grid_bar(ls, bar, block_flags(fl));
         if (!bw) return false;
         if (KIND == 1) {
             if (t == 0) {
@@ -560,7 +579,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
         if (!kind) return true;
         store_own();
         stored = true;
-        if (!loop_rebuild<M>(&L, ls, bk, kind, r)) return false;
+        if (!loop_rebuild<M>(&L, ls, bar, kind, r)) return false;
         load_own();
         stored = false;
         return true;
@@ -726,7 +745,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
                 tot[1] = f.x * u.x + f.y * u.y;
                 tot[2] = f.x * f.x + f.y * f.y;
             }
-            ok = grid_totals<3>(tot, (np + 31) / 32, w.partials, ls, bk, red);
+            ok = grid_totals<3>(tot, (np + 31) / 32, w.partials, ls, bar, red);
             if (!ok) break;
             if (t == 0) fire_epilogue<M>(s, tot);
             __syncthreads();
@@ -737,7 +756,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
         store_own();
         if (mine) w.pe[own] = pe;
     }
-    if (loop_exit(&L, ls, bk, r, red)) {
+    if (loop_exit(&L, ls, bar, r, red)) {
         ds->v = v;
         ds->s = s;
     }
@@ -763,7 +782,7 @@ __device__ __forceinline__ void loop_sums(const DevSys *ds, const PairArgs &f, i
 // `iters` iterations are done.
 template <int KIND, int G, bool M>
 __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_loop(DevSys *ds, LoopSync *ls, double dt, int chunk,
-                                                      long long iters) {
+                                                      long long iters, int polls) {
     extern __shared__ __align__(16) unsigned char loop_smem[];
     ForceWarp *fw = reinterpret_cast<ForceWarp *>(loop_smem);
     // the block's copy of the system: pointers, parameters and control state
@@ -780,7 +799,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_loop(DevSys *ds, LoopSync *l
     if (s.flags) return;  // the same for every block: nothing writes the state before a barrier
     const int n = p.n;
     const Range r = {min((int)blockIdx.x * chunk, n), min(((int)blockIdx.x + 1) * chunk, n)};
-    unsigned bk = 0;
+    GridBar bar = {0, polls};
     bool ok = true;
     long long it = 0;
     const double dt_half = 0.5 * dt;
@@ -815,12 +834,12 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_loop(DevSys *ds, LoopSync *l
         unsigned long long fl = 0;
         for (int i = r.first + t; i < r.last; i += nt)
             drift_to_other(i, v.vel[i], v.frc[i], over_mass(dt_half, v.mass[i]), fl);
-        const unsigned long long bw = grid_bar(ls, bk, block_flags(fl));
+        const unsigned long long bw = grid_bar(ls, bar, block_flags(fl));
         ok = bw != 0;
         if (ok) {
             swap_moved();
             const int kind = rebuild_kind(bw);
-            if (kind) ok = loop_rebuild<M>(&L, ls, bk, kind, r);
+            if (kind) ok = loop_rebuild<M>(&L, ls, bar, kind, r);
         }
     }
     while (ok) {
@@ -853,11 +872,11 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_loop(DevSys *ds, LoopSync *l
                 moved2(x, w.pos_n[i], w.pos_c[i], d2);
                 fl |= move_flags(p, lim_n, lim_c, d2[0], d2[1]);
             }
-            const unsigned long long bw = grid_bar(ls, bk, block_flags(fl));
+            const unsigned long long bw = grid_bar(ls, bar, block_flags(fl));
             ok = bw != 0;
             if (!ok) break;
             const int kind = rebuild_kind(bw);
-            if (kind) ok = loop_rebuild<M>(&L, ls, bk, kind, r);
+            if (kind) ok = loop_rebuild<M>(&L, ls, bar, kind, r);
             if (!ok) break;
         }
         // ---- forces and kick (k_fire_force, k_nve_second); NVE: the next
@@ -903,21 +922,21 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_loop(DevSys *ds, LoopSync *l
             if (t == 0 && ++s.nve_steps_done >= s.max_steps) s.flags |= kDone;
             __syncthreads();
             if (last) break;
-            const unsigned long long bw = grid_bar(ls, bk, block_flags(fl));
+            const unsigned long long bw = grid_bar(ls, bar, block_flags(fl));
             ok = bw != 0;
             if (!ok) break;
             swap_moved();
             const int kind = rebuild_kind(bw);
-            if (kind) ok = loop_rebuild<M>(&L, ls, bk, kind, r);
+            if (kind) ok = loop_rebuild<M>(&L, ls, bar, kind, r);
         } else {
-            ok = grid_totals<3>(tot, nt / 32, w.partials, ls, bk, red);
+            ok = grid_totals<3>(tot, nt / 32, w.partials, ls, bar, red);
             if (!ok) break;
             if (t == 0) fire_epilogue<M>(s, tot);
             __syncthreads();
             if (s.flags || it >= iters) break;
         }
     }
-    if (loop_exit(&L, ls, bk, r, red)) {
+    if (loop_exit(&L, ls, bar, r, red)) {
         ds->v = v;
         ds->s = s;
     }

@@ -10,7 +10,8 @@
 // (disk_loop.cuh); above, the loop body is a CUDA graph whose neighbour rebuild
 // sits under a conditional (IF) node inside a WHILE node.  Either way a whole
 // minimisation runs without host round trips.  DPG_LOOP_MODE=cond keeps the
-// graph at every size, graph and stream the chunked forms.
+// graph at every size, graph and stream the chunked forms; DPG_LOOP_POLLS is the
+// number of looks after which a barrier of a resident loop gives up.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -89,6 +90,7 @@ struct dpg_system {
     // resident grid (kModeResident): barrier state; lanes per particle, threads,
     // blocks, particles per block and shared memory of its two kernels
     LoopSync *lsync = nullptr;
+    int polls = kBarPolls;
     struct Plan {
         int lanes = 1, threads = 0, blocks = 0, chunk = 0;
         size_t smem = 0;
@@ -273,6 +275,7 @@ extern "C" int dpg_create(const dpg_params *p, void *cuda_stream, dpg_handle *ou
     if (m && !strcmp(m, "stream")) s->mode = kModeStream;
     else if (m && !strcmp(m, "graph")) s->mode = kModeGraph;
     else if (!(m && !strcmp(m, "cond")) && s->n <= kLoopMaxN) s->mode = kModeResident;
+    if (const char *q = getenv("DPG_LOOP_POLLS")) s->polls = std::max(1, atoi(q));
     const size_t n = s->n;
     int dev = 0, nsm = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -1200,6 +1203,15 @@ static int plan_resident(dpg_system *s) {
     return DPG_OK;
 }
 
+// A barrier of the resident loop failed: the particles stand at different points
+// of an iteration and the cell counters may be half used, so the lists are gone
+// until dpg_setup_neighbors lays them out again.
+static int loop_failed(dpg_system *s) {
+    s->have_neighbors = false;
+    TRY(put_field(s, &s->d->s.flags, 0));
+    return set_err(DPG_ERR_TIMEOUT, "a grid barrier of the resident loop ran out");
+}
+
 // Launches of the resident loop until a flag is raised, each of at most `most`
 // iterations (a fraction of a second).
 static int run_resident(dpg_system *s, int kind) {
@@ -1210,7 +1222,7 @@ static int run_resident(dpg_system *s, int kind) {
     long long most = std::max<long long>(256, (1LL << 26) / (s->n + 1024));
     double dt = s->chunk_dt;
     int chunk = q.chunk;
-    void *args[] = {(void *)&s->d, (void *)&s->lsync, (void *)&dt, (void *)&chunk, (void *)&most};
+    void *args[] = {(void *)&s->d, (void *)&s->lsync, (void *)&dt, (void *)&chunk, (void *)&most, (void *)&s->polls};
     do {
         CK(cudaMemsetAsync(s->lsync, 0, sizeof(LoopSync), s->stream));
         if (q.cluster) {
@@ -1221,7 +1233,7 @@ static int run_resident(dpg_system *s, int kind) {
             CK(cudaLaunchCooperativeKernel(fn, dim3(q.blocks), dim3(q.threads), args, q.smem, s->stream));
         }
         TRY(pull_state(s));
-        if (s->hs->flags & kError) return set_err(DPG_ERR_TIMEOUT, "a grid barrier of the resident loop ran out");
+        if (s->hs->flags & kError) return loop_failed(s);
     } while (!s->hs->flags);
     return DPG_OK;
 }
