@@ -800,7 +800,8 @@ static int loop_failed(BS *s) {
     return set_err(DPG_ERR_TIMEOUT, "a grid barrier of the resident loop ran out");
 }
 
-static int run_resident(BS *s, int kind) {
+// *refused: the launch was, and the state is that between two iterations
+static int run_resident(BS *s, int kind, bool *refused) {
     void *fn = kind == 0 ? (void *)kb_loop<0> : (void *)kb_loop<1>;
     long long most = std::max<long long>(256, (1LL << 24) / (s->nb + 1024));
     double dt = s->loop_dt, tmax = s->loop_tmax;
@@ -810,7 +811,12 @@ static int run_resident(BS *s, int kind) {
     const int threads = (long long)s->lchunk * s->max_nvb > 256 ? kLoopMaxTPB : 256;
     do {
         CK(cudaMemsetAsync(s->lsync, 0, sizeof(LoopSync), s->stream));
-        CK(cudaLaunchCooperativeKernel(fn, dim3(s->lblocks), dim3(threads), args, sizeof(BodyMem), s->stream));
+        const cudaError_t err = cudaLaunchCooperativeKernel(fn, dim3(s->lblocks), dim3(threads), args, sizeof(BodyMem), s->stream);
+        *refused = err != cudaSuccess;
+        if (*refused) {
+            (void)cudaGetLastError();
+            return set_err(DPG_ERR_CUDA, "resident loop: %s", cudaGetErrorString(err));
+        }
         TRY(pull(s));
         if (s->hs->flags & kError) return loop_failed(s);
     } while (!s->hs->flags);
@@ -825,9 +831,13 @@ static int run_loop(BS *s, int kind, int *ovf) {
         s->mode = 2;
     }
     if (s->mode == 3 && resident_holds(s)) {
-        TRY(run_resident(s, kind));
-        if (s->hs->flags & kOverflow) *ovf = 1;
-        return DPG_OK;
+        bool refused = true;
+        const int rc = run_resident(s, kind, &refused);
+        if (!refused) {
+            if (rc == DPG_OK && (s->hs->flags & kOverflow)) *ovf = 1;
+            return rc;
+        }
+        s->mode = 2;
     }
     if (s->mode >= 2) {
         if (build_graph(s, kind) != DPG_OK) {

@@ -1213,8 +1213,10 @@ static int loop_failed(dpg_system *s) {
 }
 
 // Launches of the resident loop until a flag is raised, each of at most `most`
-// iterations (a fraction of a second).
-static int run_resident(dpg_system *s, int kind) {
+// iterations (a fraction of a second).  *refused: the launch was (a context or a
+// stream may own fewer SMs than the device has); the state is then that between
+// two iterations, and the graph goes on from it.
+static int run_resident(dpg_system *s, int kind, bool *refused) {
     const bool tile = s->tile.blocks > 0 && s->cap <= kTileSlots;
     const dpg_system::Plan &q = tile ? s->tile : s->loop;
     void *fn = tile ? (kind == kLoopFire ? tile_fn<kLoopFire>(s) : tile_fn<kLoopNve>(s))
@@ -1225,12 +1227,18 @@ static int run_resident(dpg_system *s, int kind) {
     void *args[] = {(void *)&s->d, (void *)&s->lsync, (void *)&dt, (void *)&chunk, (void *)&most, (void *)&s->polls};
     do {
         CK(cudaMemsetAsync(s->lsync, 0, sizeof(LoopSync), s->stream));
+        cudaError_t err;
         if (q.cluster) {
             cudaLaunchAttribute attr[1];
             const cudaLaunchConfig_t cfg = cluster_config(q, s->stream, attr);
-            CK(cudaLaunchKernelExC(&cfg, fn, args));
+            err = cudaLaunchKernelExC(&cfg, fn, args);
         } else {
-            CK(cudaLaunchCooperativeKernel(fn, dim3(q.blocks), dim3(q.threads), args, q.smem, s->stream));
+            err = cudaLaunchCooperativeKernel(fn, dim3(q.blocks), dim3(q.threads), args, q.smem, s->stream);
+        }
+        *refused = err != cudaSuccess;
+        if (*refused) {
+            (void)cudaGetLastError();
+            return set_err(DPG_ERR_CUDA, "resident loop: %s", cudaGetErrorString(err));
         }
         TRY(pull_state(s));
         if (s->hs->flags & kError) return loop_failed(s);
@@ -1247,15 +1255,15 @@ static int run_loop(dpg_system *s, int kind, int *halted_overflow) {
     if (s->mixed) s->q_fresh = false;
     else TRY(quant_refresh(s));
     if (s->mode == kModeResident) {
-        const int rc = s->loop.blocks ? DPG_OK : plan_resident(s);
-        if (rc != DPG_OK) {
-            (void)cudaGetLastError();
-            s->mode = kModeCond;
-        } else {
-            TRY(run_resident(s, kind));
-            if (s->hs->flags & kOverflow) *halted_overflow = 1;
-            return DPG_OK;
+        bool refused = true;
+        int rc = s->loop.blocks ? DPG_OK : plan_resident(s);
+        if (rc == DPG_OK) rc = run_resident(s, kind, &refused);
+        if (!refused) {
+            if (rc == DPG_OK && (s->hs->flags & kOverflow)) *halted_overflow = 1;
+            return rc;
         }
+        (void)cudaGetLastError();
+        s->mode = kModeCond;
     }
     if (s->mode == kModeCond) {
         int rc = build_cond_graph(s, kind);
