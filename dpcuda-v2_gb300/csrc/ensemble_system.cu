@@ -610,7 +610,10 @@ static int launch_resident(ES *s, long long budget, unsigned long long slice_ns,
         res_most(s, c, &ncmax[c], &nmax);
         lcap[c] = res_list_entries(K.per_block(), K.w, ncmax[c], res_smem_room());
         smem[c] = res_smem_bytes(K.per_block(), K.w, nmax, ncmax[c], lcap[c]);
-        CK(cudaFuncSetAttribute((const void *)K.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[c]));
+        // a limit of the function, which several shapes, batches and threads share:
+        // always the same one; smem[c] is what the launch takes
+        CK(cudaFuncSetAttribute((const void *)K.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)res_smem_room()));
         if (!s->rs_fit[c]) {
             cudaLaunchAttribute attr[1];
             const cudaLaunchConfig_t cfg = res_config(K, (int)order[c].size(), smem[c], s->stream, attr);
