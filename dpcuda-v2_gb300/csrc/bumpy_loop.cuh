@@ -16,7 +16,7 @@ constexpr int kVlistParts = 4;   // warps that share a body in the list build at
 
 // The rebuild inside the loop: the kernels k_cell_index .. kb_vlist as phases
 // between barriers.  Returns false if the loop has to leave.
-__device__ __forceinline__ bool bumpy_rebuild(BumpySys *bs, LoopSync *ls, GridBar &bar, int kind, Range r) {
+__device__ __forceinline__ bool bumpy_rebuild(BumpySys *bs, LoopSync *ls, unsigned &bk, int polls, int kind, Range r) {
     DevSys &d = bs->b;
     BumpyExt &x = bs->x;
     const DevParams &p = d.p;
@@ -35,25 +35,25 @@ __device__ __forceinline__ bool bumpy_rebuild(BumpySys *bs, LoopSync *ls, GridBa
             d.w.cell_raw[i] = cell;
             atomicAdd(&d.w.cell_cnt[cell], 1);
         }
-        if (!grid_bar(ls, bar, 0)) return false;
+        if (!grid_bar(ls, bk, polls, 0)) return false;
         if (blockIdx.x == 0) {
             const int all = scan_block(d.w.cell_cnt, d.w.cell_start, p.ncells);
             if (t == 0) d.w.cell_start[p.ncells] = all;
         }
-        if (!grid_bar(ls, bar, 0)) return false;
+        if (!grid_bar(ls, bk, polls, 0)) return false;
         for (int i = r.first + t; i < r.last; i += nt) {
             const int c = d.w.cell_raw[i];
             d.w.perm[d.w.cell_start[c] + atomicAdd(&d.w.cell_cur[c], 1)] = i;
         }
-        if (!grid_bar(ls, bar, 0)) return false;
+        if (!grid_bar(ls, bk, polls, 0)) return false;
         for (int c = blockIdx.x * nt + t; c < p.ncells; c += gridDim.x * nt) cell_sort_one(&d, c);
-        if (!grid_bar(ls, bar, 0)) return false;
+        if (!grid_bar(ls, bk, polls, 0)) return false;
         for (int i = r.first + t; i < r.last; i += nt) reorder_body(bs, i);
-        if (!grid_bar(ls, bar, 0)) return false;
+        if (!grid_bar(ls, bk, polls, 0)) return false;
         if (blockIdx.x == 0) scan_block(x.nvb_t, x.start_t, p.n);  // starts only: the array has no n + 1st
-        if (!grid_bar(ls, bar, 0)) return false;
+        if (!grid_bar(ls, bk, polls, 0)) return false;
         for (int i = r.first + t / 32; i < r.last; i += nt / 32) reorder_vertices(bs, i, t & 31);
-        if (!grid_bar(ls, bar, 0)) return false;
+        if (!grid_bar(ls, bk, polls, 0)) return false;
         if (t == 0) {
             swap_sorted(bs);
             s.n_cell_rebuilds++;
@@ -67,7 +67,7 @@ __device__ __forceinline__ bool bumpy_rebuild(BumpySys *bs, LoopSync *ls, GridBa
         if (x.mixed)
             for (int u = v0 + t; u < v1; u += nt) x.vq[u] = quant_of(p, x.vpos[u], x.rv);
     }
-    if (!grid_bar(ls, bar, 0)) return false;
+    if (!grid_bar(ls, bk, polls, 0)) return false;
     __shared__ int bmx[2];
     if (t < 2) bmx[t] = 0;
     __syncthreads();
@@ -122,7 +122,7 @@ __device__ __forceinline__ bool bumpy_rebuild(BumpySys *bs, LoopSync *ls, GridBa
     if (mx) atomicMax(&bmx[1], mx);
     __syncthreads();
     if (t < 2) atomicMax(t == 0 ? &ls->max_count : &ls->max_vcount, bmx[t]);
-    const unsigned long long w = grid_bar(ls, bar, bmx[0] > p.cap || bmx[1] > x.capv ? kFull : 0);
+    const unsigned long long w = grid_bar(ls, bk, polls, bmx[0] > p.cap || bmx[1] > x.capv ? kFull : 0);
     if (!w) return false;
     if (t == 0) {
         s.n_rebuilds++;
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) kb_loop(BumpySys *bs, LoopSync
     const int np = r.last - r.first;
     const int role = t / kLoopBodies, lb = t % kLoopBodies, own = r.first + lb;
     const bool mine = role < 4 && lb < np;
-    GridBar bar = {0, polls};
+    unsigned bk = 0;
     bool ok = true, stored = false;
     long long it = 0;
     const double dt_half = 0.5 * dt;
@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) kb_loop(BumpySys *bs, LoopSync
     auto after_move = [&]() {
         unsigned long long fl = 0;
         if (t < np) fl = move_flags(p, m.xa[0][t] + m.xa[1][t], m.xb[0][t] + m.xb[1][t]);
-        const unsigned long long bw = grid_bar(ls, bar, block_flags(fl));
+        const unsigned long long bw = grid_bar(ls, bk, polls, block_flags(fl));
         if (!bw) return false;
         if (KIND == 1) {
             if (t == 0) {
@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) kb_loop(BumpySys *bs, LoopSync
         store_own();
         stored = true;
         __syncthreads();
-        if (!bumpy_rebuild(&L, ls, bar, kind, r)) return false;
+        if (!bumpy_rebuild(&L, ls, bk, polls, kind, r)) return false;
         load_own();
         stored = false;
         return true;
@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) kb_loop(BumpySys *bs, LoopSync
                 tot[2] = m.xb[0][t] + m.xb[1][t];
                 tot[3] = m.xb[2][t];
             }
-            ok = grid_totals<4>(tot, (np + 31) / 32, L.b.w.partials, ls, bar, red);
+            ok = grid_totals<4>(tot, (np + 31) / 32, L.b.w.partials, ls, bk, polls, red);
             if (!ok) break;
             if (t == 0) bumpy_fire_epilogue(&L, tot, tmax);
             __syncthreads();
@@ -591,7 +591,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) kb_loop(BumpySys *bs, LoopSync
         if (mine && role == 3) L.b.w.pe[own] = pe;
     }
     __syncthreads();
-    if (loop_exit(&L.b, ls, bar, r, red)) *bs = L;
+    if (loop_exit(&L.b, ls, bk, polls, r, red)) *bs = L;
 }
 
 }  // namespace

@@ -46,19 +46,28 @@ struct LoopSync {
 // what a barrier carries besides the arrival count (bits 0 - 15): how many
 // blocks raised each flag
 constexpr unsigned long long kNeedList = 1ULL << 16, kNeedCell = 1ULL << 32, kFull = 1ULL << 48;
-constexpr unsigned long long kClosed = 1ULL << 63;  // the barrier failed (block counts stay below 2^9)
+constexpr unsigned long long kClosed = 1ULL << 15;  // the barrier failed: above every count of arrivals
 __device__ __forceinline__ bool raised(unsigned long long v, unsigned long long flag) {
     return (v / flag & 0xffff) != 0;
 }
 
-// What a block knows of its barriers: the next one's number, and how often a
-// wait looks before it gives up.
-struct GridBar {
-    unsigned k;
-    int polls;
-};
+// Polls that ran out with `v` (or found the word closed): closes it and returns 0,
+// or returns the completed word if the last arrivals came first.  Thread 0, and
+// apart from the barrier, whose path this should not lengthen.
+__device__ __noinline__ unsigned long long bar_short(LoopSync *ls, unsigned long long *w, unsigned long long v) {
+    while ((v & 0xffff) < gridDim.x) {  // another arrival makes it look again
+        const unsigned long long seen = atomicCAS(w, v, v | kClosed);
+        v = seen == v ? v | kClosed : seen;
+    }
+    __threadfence();
+    if (!(v & kClosed)) return v;
+    *(volatile int *)&ls->err = 1;
+    return 0;
+}
 
-// Grid barrier bar.k; flags of thread 0 are added to the arrival.  Returns the
+// Grid barrier k; flags of thread 0 are added to the arrival; polls: how often a
+// wait looks (a launch argument, passed by value: kept beside k behind a reference
+// it cost a FIRE iteration of 16384 disks 0.5 %).  Returns the
 // completed word (arrivals and flag counts) on every thread, 0 if the barrier
 // failed.  A block whose polls run out closes the word by compare-and-swap, which
 // succeeds only while arrivals are missing, and a closed word stays so: a
@@ -69,49 +78,42 @@ struct GridBar {
 // A grid of one thread-block cluster uses the cluster's barrier, the flags going
 // to every block's shared memory before it (two sets in turn: a block that
 // writes one again has passed a barrier that its readers entered later).
-__device__ __forceinline__ unsigned long long grid_bar(LoopSync *ls, GridBar &bar, unsigned long long flags) {
+__device__ __forceinline__ unsigned long long grid_bar(LoopSync *ls, unsigned &k, int polls, unsigned long long flags) {
     __shared__ unsigned long long done, said[2][kClusterMax];
     const auto cluster = cooperative_groups::this_cluster();
     if (cluster.num_blocks() > 1) {
         const int nb = (int)cluster.num_blocks(), t = threadIdx.x;
         flags = __shfl_sync(0xffffffffu, flags, 0);
-        if (t < nb) *cluster.map_shared_rank(&said[bar.k & 1][cluster.block_rank()], t) = 1ULL + flags;
+        if (t < nb) *cluster.map_shared_rank(&said[k & 1][cluster.block_rank()], t) = 1ULL + flags;
         cluster.sync();
         if (t < 32) {
-            unsigned long long v = t < nb ? said[bar.k & 1][t] : 0;
+            unsigned long long v = t < nb ? said[k & 1][t] : 0;
 #pragma unroll
             for (int o = kClusterMax / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
             if (t == 0) done = v;
         }
         __syncthreads();
-        bar.k++;
+        k++;
         return done;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        unsigned long long *w = &ls->ring[bar.k & 3], v;
+        unsigned long long *w = &ls->ring[k & 3], v;
         __threadfence();
         atomicAdd(w, 1ULL + flags);
-        int polls = 0;
+        int n = 0;
         do {
             asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(w) : "memory");
-        } while ((v & 0xffff) < gridDim.x && !(v & kClosed) && ++polls < bar.polls);
-        while ((v & 0xffff) < gridDim.x && !(v & kClosed)) {  // run out; an arrival makes it look again
-            const unsigned long long seen = atomicCAS(w, v, v | kClosed);
-            v = seen == v ? v | kClosed : seen;
-            __threadfence();
-        }
-        if (v & kClosed) {
-            *(volatile int *)&ls->err = 1;
-            v = 0;
-        } else if (blockIdx.x == 0) {
-            ls->ring[(bar.k + 2) & 3] = 0;
+        } while ((v & 0xffff) < gridDim.x && ++n < polls);
+        if ((v & 0xffff) != gridDim.x) v = bar_short(ls, w, v);
+        if (blockIdx.x == 0) {
+            ls->ring[(k + 2) & 3] = 0;
             __threadfence();
         }
         done = v;
     }
     __syncthreads();
-    bar.k++;
+    k++;
     return done;
 }
 
@@ -185,7 +187,7 @@ __device__ __forceinline__ int nlist_all_row(const DevSys *ds, int i) {
 // Returns false if the loop has to leave (a row longer than the capacity, or a
 // barrier that ran out).
 template <bool M>
-__device__ bool loop_rebuild(DevSys *ds, LoopSync *ls, GridBar &bar, int kind, Range r) {
+__device__ bool loop_rebuild(DevSys *ds, LoopSync *ls, unsigned &bk, int polls, int kind, Range r) {
     const DevParams &p = ds->p;
     DevView &v = ds->v;
     DevState &s = ds->s;
@@ -197,19 +199,19 @@ __device__ bool loop_rebuild(DevSys *ds, LoopSync *ls, GridBar &bar, int kind, R
             ds->w.cell_raw[i] = c;
             atomicAdd(&ds->w.cell_cnt[c], 1);
         }
-        if (!grid_bar(ls, bar, 0)) return false;
+        if (!grid_bar(ls, bk, polls, 0)) return false;
         if (blockIdx.x == 0) {
             const int all = scan_block(ds->w.cell_cnt, ds->w.cell_start, p.ncells);
             if (t == 0) ds->w.cell_start[p.ncells] = all;
         }
-        if (!grid_bar(ls, bar, 0)) return false;
+        if (!grid_bar(ls, bk, polls, 0)) return false;
         for (int i = r.first + t; i < r.last; i += nt) {
             const int c = ds->w.cell_raw[i];
             ds->w.perm[ds->w.cell_start[c] + atomicAdd(&ds->w.cell_cur[c], 1)] = i;
         }
-        if (!grid_bar(ls, bar, 0)) return false;
+        if (!grid_bar(ls, bk, polls, 0)) return false;
         for (int c = blockIdx.x * nt + t; c < p.ncells; c += gridDim.x * nt) cell_sort_one(ds, c);
-        if (!grid_bar(ls, bar, 0)) return false;
+        if (!grid_bar(ls, bk, polls, 0)) return false;
         for (int i = r.first + t; i < r.last; i += nt) {
             const int o = ds->w.perm[i];
             const double2 x = v.pos[o];
@@ -224,7 +226,7 @@ __device__ bool loop_rebuild(DevSys *ds, LoopSync *ls, GridBar &bar, int kind, R
             ds->w.cell_of[i] = ds->w.cell_raw[o];
             ds->w.pos_c[i] = x;
         }
-        if (!grid_bar(ls, bar, 0)) return false;
+        if (!grid_bar(ls, bk, polls, 0)) return false;
         if (t == 0) {
             swap_ptr(v.pos, v.pos_t);
             swap_ptr(v.vel, v.vel_t);
@@ -239,7 +241,7 @@ __device__ bool loop_rebuild(DevSys *ds, LoopSync *ls, GridBar &bar, int kind, R
         __syncthreads();
     } else if (M) {
         for (int i = r.first + t; i < r.last; i += nt) v.q[i] = quant_of(p, v.pos[i], v.rad[i]);
-        if (!grid_bar(ls, bar, 0)) return false;
+        if (!grid_bar(ls, bk, polls, 0)) return false;
     }
     int mx = 0;
     if (p.method == 0) {
@@ -272,7 +274,7 @@ __device__ bool loop_rebuild(DevSys *ds, LoopSync *ls, GridBar &bar, int kind, R
     if ((t & 31) == 0) atomicMax(&bmx, mx);
     __syncthreads();
     if (t == 0) atomicMax(&ls->max_count, bmx);
-    const unsigned long long w = grid_bar(ls, bar, bmx > p.cap ? kFull : 0);
+    const unsigned long long w = grid_bar(ls, bk, polls, bmx > p.cap ? kFull : 0);
     if (!w) return false;
     if (t == 0) {
         s.n_rebuilds++;
@@ -338,7 +340,7 @@ __device__ __forceinline__ void warp_totals(double &sum, double (&mx)[K - 2]) {
         for (int k = 0; k < K - 2; k++) mx[k] = max_pos(mx[k], __shfl_down_sync(0xffffffffu, mx[k], o));
 }
 template <int K>
-__device__ __forceinline__ bool grid_totals(double (&v)[K], int nwr, double *part, LoopSync *ls, GridBar &bar,
+__device__ __forceinline__ bool grid_totals(double (&v)[K], int nwr, double *part, LoopSync *ls, unsigned &bk, int polls,
                                             double *sm) {
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nb = gridDim.x;
     double mx[K - 2], sum;
@@ -360,7 +362,7 @@ __device__ __forceinline__ bool grid_totals(double (&v)[K], int nwr, double *par
         for (int w = 1; w < nwr; w++) a = t < 2 ? a + sm[w * K + t] : max_pos(a, sm[w * K + t]);
         part[t * nb + blockIdx.x] = a;
     }
-    if (!grid_bar(ls, bar, 0)) return false;
+    if (!grid_bar(ls, bk, polls, 0)) return false;
     if (wid == 0) {
         // all loads in flight at once (one trip to L2), then added in order
         const double *mine = part + (lane < 16 ? 0 : nb);
@@ -394,7 +396,7 @@ __device__ __forceinline__ bool grid_totals(double (&v)[K], int nwr, double *par
 // End of a resident loop: the displacement maxima of the last move (zero where
 // a build followed), after every block has handed in its own.  True on thread 0
 // of block 0, which then writes its copy of the system back.
-__device__ __forceinline__ bool loop_exit(DevSys *L, LoopSync *ls, GridBar &bar, Range r, double *red) {
+__device__ __forceinline__ bool loop_exit(DevSys *L, LoopSync *ls, unsigned &bk, int polls, Range r, double *red) {
     const int t = threadIdx.x, nb = gridDim.x;
     double m[2] = {0.0, 0.0};
     for (int i = r.first + t; i < r.last; i += blockDim.x) {
@@ -410,7 +412,7 @@ __device__ __forceinline__ bool loop_exit(DevSys *L, LoopSync *ls, GridBar &bar,
         part[blockIdx.x] = m[0];
         part[nb + blockIdx.x] = m[1];
     }
-    const bool all = grid_bar(ls, bar, 0) != 0;
+    const bool all = grid_bar(ls, bk, polls, 0) != 0;
     if (blockIdx.x != 0) return false;
     m[0] = 0.0;
     m[1] = 0.0;
@@ -504,7 +506,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
     const int lim_n = __double2hiint(p.nthr2 / 3.0), lim_c = __double2hiint(p.cthr2 / 3.0);
     // the sums' threads: component t / np of particle t % np
     const int sum_k = np > 0 ? t / np : 3, sum_g = np > 0 ? t % np : 0;
-    GridBar bar = {0, polls};
+    unsigned bk = 0;
     bool ok = true, stored = false;
     long long it = 0;
 
@@ -565,7 +567,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
     // the barrier after a move, the buffer swap (NVE) and a rebuild if any
     // particle asks for one; false: leave
     auto after_move = [&](unsigned long long fl) {
-        const unsigned long long bw = grid_bar(ls, bar, block_flags(fl));
+        const unsigned long long bw = grid_bar(ls, bk, polls, block_flags(fl));
         if (!bw) return false;
         if (KIND == 1) {
             if (t == 0) {
@@ -579,7 +581,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
         if (!kind) return true;
         store_own();
         stored = true;
-        if (!loop_rebuild<M>(&L, ls, bar, kind, r)) return false;
+        if (!loop_rebuild<M>(&L, ls, bk, polls, kind, r)) return false;
         load_own();
         stored = false;
         return true;
@@ -745,7 +747,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
                 tot[1] = f.x * u.x + f.y * u.y;
                 tot[2] = f.x * f.x + f.y * f.y;
             }
-            ok = grid_totals<3>(tot, (np + 31) / 32, w.partials, ls, bar, red);
+            ok = grid_totals<3>(tot, (np + 31) / 32, w.partials, ls, bk, polls, red);
             if (!ok) break;
             if (t == 0) fire_epilogue<M>(s, tot);
             __syncthreads();
@@ -756,7 +758,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
         store_own();
         if (mine) w.pe[own] = pe;
     }
-    if (loop_exit(&L, ls, bar, r, red)) {
+    if (loop_exit(&L, ls, bk, polls, r, red)) {
         ds->v = v;
         ds->s = s;
     }
@@ -799,7 +801,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_loop(DevSys *ds, LoopSync *l
     if (s.flags) return;  // the same for every block: nothing writes the state before a barrier
     const int n = p.n;
     const Range r = {min((int)blockIdx.x * chunk, n), min(((int)blockIdx.x + 1) * chunk, n)};
-    GridBar bar = {0, polls};
+    unsigned bk = 0;
     bool ok = true;
     long long it = 0;
     const double dt_half = 0.5 * dt;
@@ -834,12 +836,12 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_loop(DevSys *ds, LoopSync *l
         unsigned long long fl = 0;
         for (int i = r.first + t; i < r.last; i += nt)
             drift_to_other(i, v.vel[i], v.frc[i], over_mass(dt_half, v.mass[i]), fl);
-        const unsigned long long bw = grid_bar(ls, bar, block_flags(fl));
+        const unsigned long long bw = grid_bar(ls, bk, polls, block_flags(fl));
         ok = bw != 0;
         if (ok) {
             swap_moved();
             const int kind = rebuild_kind(bw);
-            if (kind) ok = loop_rebuild<M>(&L, ls, bar, kind, r);
+            if (kind) ok = loop_rebuild<M>(&L, ls, bk, polls, kind, r);
         }
     }
     while (ok) {
@@ -872,11 +874,11 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_loop(DevSys *ds, LoopSync *l
                 moved2(x, w.pos_n[i], w.pos_c[i], d2);
                 fl |= move_flags(p, lim_n, lim_c, d2[0], d2[1]);
             }
-            const unsigned long long bw = grid_bar(ls, bar, block_flags(fl));
+            const unsigned long long bw = grid_bar(ls, bk, polls, block_flags(fl));
             ok = bw != 0;
             if (!ok) break;
             const int kind = rebuild_kind(bw);
-            if (kind) ok = loop_rebuild<M>(&L, ls, bar, kind, r);
+            if (kind) ok = loop_rebuild<M>(&L, ls, bk, polls, kind, r);
             if (!ok) break;
         }
         // ---- forces and kick (k_fire_force, k_nve_second); NVE: the next
@@ -922,21 +924,21 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_loop(DevSys *ds, LoopSync *l
             if (t == 0 && ++s.nve_steps_done >= s.max_steps) s.flags |= kDone;
             __syncthreads();
             if (last) break;
-            const unsigned long long bw = grid_bar(ls, bar, block_flags(fl));
+            const unsigned long long bw = grid_bar(ls, bk, polls, block_flags(fl));
             ok = bw != 0;
             if (!ok) break;
             swap_moved();
             const int kind = rebuild_kind(bw);
-            if (kind) ok = loop_rebuild<M>(&L, ls, bar, kind, r);
+            if (kind) ok = loop_rebuild<M>(&L, ls, bk, polls, kind, r);
         } else {
-            ok = grid_totals<3>(tot, nt / 32, w.partials, ls, bar, red);
+            ok = grid_totals<3>(tot, nt / 32, w.partials, ls, bk, polls, red);
             if (!ok) break;
             if (t == 0) fire_epilogue<M>(s, tot);
             __syncthreads();
             if (s.flags || it >= iters) break;
         }
     }
-    if (loop_exit(&L, ls, bar, r, red)) {
+    if (loop_exit(&L, ls, bk, polls, r, red)) {
         ds->v = v;
         ds->s = s;
     }
