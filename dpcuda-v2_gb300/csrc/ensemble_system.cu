@@ -472,7 +472,8 @@ typedef void (*res_kernel_fn)(EDev *, const int *, int, int, long long, unsigned
 // cluster): a system goes to the first shape of its table that holds it.  The
 // wide table spreads a system over many blocks and lanes, which shortens its
 // iterations; the later ones pack it into fewer SMs, so that more systems run
-// side by side.  No result depends on the shape.
+// side by side.  No result depends on the shape; what adds FP64 totals by block,
+// the four-pass shape, is therefore in every table, and alone for its sizes.
 struct RClass {
     int w, p, r, c;
     res_kernel_fn fn;
