@@ -47,9 +47,11 @@ struct dpg_ensemble_system {
     static constexpr int kShapes = 17;
     cudaStream_t rs_stream[kShapes] = {};
     cudaEvent_t rs_fork = nullptr, rs_join[kShapes] = {};
-    int rs_fit[kShapes] = {};    // clusters of each class the GPU holds at once (0: not yet asked)
+    int rs_fit[kShapes] = {};    // clusters of each class the GPU holds at once ...
+    size_t rs_smem[kShapes] = {};  // ... with this much shared memory a block (0: not yet asked)
     int rs_rot[kShapes] = {};    // rotation of each class's systems between launches
     int rs_table = 0;            // the table of shapes (see kResTables)
+    bool rs_fp64 = true;         // systems in FP64 take their own rows (see kResFp64)
     int *d_rs_blocks = nullptr;
 };
 
@@ -499,8 +501,22 @@ static int res_class_in(const int *table, int n) {
         if (n <= kRClasses[table[k]].capacity()) return table[k];
     return -1;
 }
-static int res_class_of(const ES *s, int n) {
-    return res_class_in(kResTables[s->rs_table], n);
+// FP64 passes cost their instructions, whatever lanes these have, and a particle
+// of more than 64 / 128 disks has 2 / 1 partial sums (res_order): more lanes than
+// that, or a second block, only spread the same instructions thinner.  So a system
+// in FP64 takes, of the first two tables, the shape with as many lanes as sums.
+// 300 iterations of one system by the wide table, by these: 100 disks 13.6 -> 8.9
+// ms, 200 23.9 -> 13.9, 256 24.6 -> 16.0, 300 24.3 -> 18.9, 512 24.4 -> 28.3.
+struct ResRow {
+    int most, shape;
+};
+static const ResRow kResFp64[2][3] = {{{64, 0}, {128, 14}, {384, 15}}, {{64, 0}, {128, 14}, {512, 15}}};
+
+static int res_class_of(const ES *s, const ESys &y) {
+    if (s->rs_fp64 && y.prec == 1 && s->rs_table < 2)
+        for (const ResRow &q : kResFp64[s->rs_table])
+            if (y.n <= q.most) return q.shape;
+    return res_class_in(kResTables[s->rs_table], y.n);
 }
 
 // largest cell count and system of class c
@@ -508,7 +524,7 @@ static void res_most(const ES *s, int c, int *ncmax, int *nmax) {
     *ncmax = 1;
     *nmax = 1;
     for (const auto &y : s->sys)
-        if (res_class_of(s, y.n) == c) {
+        if (res_class_of(s, y) == c) {
             *ncmax = std::max(*ncmax, y.ncd * y.ncd);
             *nmax = std::max(*nmax, y.n);
         }
@@ -545,18 +561,18 @@ static bool res_table_fits(const ES *s) {
 static void res_choose(ES *s, bool live) {
     int dev = 0, nsm = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const int was = s->rs_table;
+    s->rs_fp64 = true;
     for (s->rs_table = 0; s->rs_table + 1 < kNTables; s->rs_table++) {
         double sms = 0;
         for (const auto &y : s->sys) {
             if (live && y.phase == kIdle) continue;
-            const RClass &K = kRClasses[res_class_of(s, y.n)];
+            const RClass &K = kRClasses[res_class_of(s, y)];
             sms += K.c * (K.w == 8 && K.r == 1 && K.p == 32 ? 1.0 / 3 : K.w / 16.0);
         }
         if (sms <= (s->rs_table ? nsm : nsm / 8 * 7)) break;
     }
     while (s->rs_table > 0 && !res_table_fits(s)) s->rs_table--;
-    if (s->rs_table != was) std::fill(std::begin(s->rs_fit), std::end(s->rs_fit), 0);
+    if (!res_table_fits(s)) s->rs_fp64 = false;
 }
 
 // the resident form holds every system: sizes and shared memory within limits
@@ -597,7 +613,7 @@ static int launch_resident(ES *s, long long budget, unsigned long long slice_ns,
     for (int k = 0; k < s->S; k++) {
         const ESys &y = s->sys[k];
         if (y.phase == kIdle) continue;
-        order[res_class_of(s, y.n)].push_back(k);
+        order[res_class_of(s, y)].push_back(k);
     }
     std::vector<int> flat;
     int first[kNClass];
@@ -615,7 +631,8 @@ static int launch_resident(ES *s, long long budget, unsigned long long slice_ns,
         // always the same one; smem[c] is what the launch takes
         CK(cudaFuncSetAttribute((const void *)K.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)res_smem_room()));
-        if (!s->rs_fit[c]) {
+        if (s->rs_smem[c] != smem[c]) {
+            s->rs_smem[c] = smem[c];
             cudaLaunchAttribute attr[1];
             const cudaLaunchConfig_t cfg = res_config(K, (int)order[c].size(), smem[c], s->stream, attr);
             int fit = 0;

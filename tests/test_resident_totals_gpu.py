@@ -71,3 +71,15 @@ def test_every_table_reports_the_same(dpg, n, copies, mixed):
         np.testing.assert_array_equal(batch[c].reshape(copies, n), np.tile(alone[c], (copies, 1)), err_msg=c)
     for r in all_:
         assert {k: r[k] for k in REPORTED} == {k: one[0][k] for k in REPORTED}
+
+
+@pytest.mark.parametrize("n,side", [(64, 168), (100, 168), (200, 166), (300, 160)])
+def test_fp64_systems_keep_the_widest_grids(dpg, n, side):
+    """The shapes that FP64 systems prefer leave less room for the cells; where they
+    do not fit, the wide table's run the system."""
+    st = packing(n)
+    st = dict(st, box=side * 1.1 * 1.7 * 1.0001)
+    out, res = run(dpg, [st], False, 40)
+    assert res[0]["fire_steps"] > 0
+    for c in ("x", "y", "fx", "fy"):
+        assert np.all(np.isfinite(out[c]))
