@@ -702,14 +702,15 @@ static int grow_lists(ES *s, const EDev &cur) {
 // for at most kSlice of device time per block (so the classes' launches end
 // together and the host sees progress); termination is the device state
 // machine's (every minimisation has a step cap, jamming a compression cap);
-// Where a class has more systems than fit, they take turns of 0.5 ms at first,
-// growing to stay a fifteenth of the time spent: whole runs one after the other
-// would leave the last ones on a mostly idle GPU.
+// where a class has more systems than fit, they take turns of 0.5 ms at first
+// (DPG_TURN_NS: of that many ns), growing to stay a fifteenth of the time spent:
+// whole runs one after the other would leave the last ones on a mostly idle GPU;
 // the host stops with an error when some system's FIRE passes in this run
 // exceed guard_limit or a launch makes no progress.
 static int run_resident(ES *s, long long guard_limit) {
     const unsigned long long kSlice = 200ull * 1000 * 1000;  // 0.2 s
     double turn = 0.5e6;
+    if (const char *q = getenv("DPG_TURN_NS")) turn = std::max(1.0, atof(q));
     const long long kChunk = 1LL << 24;
     std::vector<long long> base(s->S, -1);
     if (!res_fits(s)) return set_err(DPG_ERR_ARG, "resident form: the systems do not fit");
