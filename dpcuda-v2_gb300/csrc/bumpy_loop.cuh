@@ -151,33 +151,37 @@ __device__ __forceinline__ bool bumpy_rebuild(BumpySys *bs, LoopSync *ls, unsign
 //  - the vertex pairs that the filter lets through form one queue per block,
 //    evaluated on full warps; only the vertices that have a term compute a
 //    torque and enter the body sums (in vertex order, one thread a sum).
-constexpr int kBodyVerts = 1536;  // vertices per block at most
-constexpr int kVertSlots = 32;    // vertex-list capacity at most
-constexpr int kVertRows = 6144;   // list entries kept on chip (more are read from memory)
-constexpr int kVertQueue = 2048;  // queued vertex pairs evaluated at a time
+constexpr int kBodyVerts = 1536;      // vertices per block at most
+constexpr int kBodyVertsSmall = 256;  // ... of a block of 256 threads, two of which share an SM,
+                                      // so that two small systems run side by side: 301 bodies
+                                      // on two streams, 2000 steps each, 67.3 -> 35.7 ms
+constexpr int kVertSlots = 32;        // vertex-list capacity at most
 
+template <int V>  // vertices at most
 struct BodyMem {
-    double2 vpos[kBodyVerts];           // current vertex positions
-    double res[3][kVertQueue];          // terms of the queued pairs
-    double term[4][kBodyVerts];         // terms of the vertices that have one
+    static constexpr int kRows = V == kBodyVerts ? 6144 : 2048;   // list entries kept on chip (more are read from memory)
+    static constexpr int kQueue = V == kBodyVerts ? 2048 : 1024;  // queued vertex pairs evaluated at a time
+    double2 vpos[V];                    // current vertex positions
+    double res[3][kQueue];              // terms of the queued pairs
+    double term[4][V];                  // terms of the vertices that have one
     double2 p[kLoopBodies], n[kLoopBodies], cs[kLoopBodies];  // a move: from, to, cosine and sine
     double sum[4][kLoopBodies];         // force x, force y, torque, energy
     double xa[4][kLoopBodies], xb[4][kLoopBodies];  // exchanged between the roles
     // the vertex rows of the block as one list: entry e belongs to vertex k for
     // row[k] <= e < row[k + 1]
-    int row[kBodyVerts + 1];
-    int other[kVertRows];               // the other vertex
-    unsigned short of[kVertRows];       // k
+    int row[V + 1];
+    int other[kRows];               // the other vertex
+    unsigned short of[kRows];       // k
     // a force pass: which entries may touch (bit e), and how many before each
     // word: the queue position of entry e is rank(e)
-    unsigned touch[kBodyVerts + 1];
-    int count[kBodyVerts], before[kBodyVerts + 1];
-    unsigned short ent[kVertQueue];     // entry at each queue position
-    unsigned vmask[kBodyVerts / 32];    // vertices that have a term
-    unsigned short tv[kBodyVerts];      // the term vertices
+    unsigned touch[V + 1];
+    int count[V], before[V + 1];
+    unsigned short ent[kQueue];     // entry at each queue position
+    unsigned vmask[V / 32];    // vertices that have a term
+    unsigned short tv[V];      // the term vertices
     int first[kLoopBodies + 1];         // first term vertex of each body
     int vfirst[kLoopBodies + 1];        // first vertex of each body (block-local)
-    unsigned char vb[kBodyVerts];       // body of each vertex (block-local)
+    unsigned char vb[V];       // body of each vertex (block-local)
     __device__ __forceinline__ int rank(int e) const {
         return before[e >> 5] + __popc(touch[e >> 5] & ((1u << (e & 31)) - 1u));
     }
@@ -185,8 +189,9 @@ struct BodyMem {
 
 // vertex and other vertex of entry e: from the chip, or by a search of the rows
 // and a load
-__device__ __forceinline__ void entry_of(const BodyMem &m, const BumpySys &L, int nv, int v0, int e, int &k, int &j) {
-    if (m.row[nv] <= kVertRows) {
+template <int V>
+__device__ __forceinline__ void entry_of(const BodyMem<V> &m, const BumpySys &L, int nv, int v0, int e, int &k, int &j) {
+    if (m.row[nv] <= m.kRows) {
         k = m.of[e];
         j = m.other[e];
         return;
@@ -211,11 +216,12 @@ __device__ __forceinline__ double vertex_pair(const PairArgs &f, const VertConst
     return contact_terms<true>(dx, dy, c.rs, c.inv, f.e_c, f.n_c, fx, fy);
 }
 
-template <int KIND>
+template <int KIND, int V>
 __global__ void __launch_bounds__(kLoopMaxTPB, 1) kb_loop(BumpySys *bs, LoopSync *ls, double dt, double tmax,
                                                          int chunk, long long iters, int polls) {
     extern __shared__ __align__(16) unsigned char loop_smem[];
-    BodyMem &m = *reinterpret_cast<BodyMem *>(loop_smem);
+    BodyMem<V> &m = *reinterpret_cast<BodyMem<V> *>(loop_smem);
+    constexpr int kQueue = BodyMem<V>::kQueue;
     __shared__ BumpySys L;
     __shared__ double red[32 * 4];
     const int t = threadIdx.x, nt = blockDim.x, lane = t & 31, wid = t >> 5, nw = nt >> 5;
@@ -271,7 +277,7 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) kb_loop(BumpySys *bs, LoopSync
         const int rows = scan_block(m.count, m.row, nv);
         if (t == 0) m.row[nv] = rows;
         __syncthreads();
-        if (m.row[nv] <= kVertRows)
+        if (m.row[nv] <= m.kRows)
             for (int k = t; k < nv; k += nt)
                 for (int q = 0; q < m.count[k]; q++) {
                     m.other[m.row[k] + q] = x.vnbr[(size_t)q * x.nv + v0 + k];
@@ -456,11 +462,11 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) kb_loop(BumpySys *bs, LoopSync
             if (lane == 0) m.vmask[w] = b;
         }
         // evaluate the queue, a window at a time (one, but far above any packing)
-        for (int q0 = 0; q0 < entries || q0 == 0; q0 += kVertQueue) {
-            const int q1 = min(entries, q0 + kVertQueue);
+        for (int q0 = 0; q0 < entries || q0 == 0; q0 += kQueue) {
+            const int q1 = min(entries, q0 + kQueue);
             for (int w = wid; w < words; w += nw) {
                 const int at = m.before[w] + __popc(m.touch[w] & ((1u << lane) - 1u)) - q0;
-                if ((m.touch[w] >> lane & 1u) && at >= 0 && at < kVertQueue) m.ent[at] = (unsigned short)(w * 32 + lane);
+                if ((m.touch[w] >> lane & 1u) && at >= 0 && at < kQueue) m.ent[at] = (unsigned short)(w * 32 + lane);
             }
             __syncthreads();
             if (q0 == 0) {  // the term vertices, their bodies' first
@@ -480,9 +486,9 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) kb_loop(BumpySys *bs, LoopSync
                 if (fp32) {
                     float *rf = reinterpret_cast<float *>(&m.res[0][0]);
                     float fx, fy;
-                    rf[2 * kVertQueue + q] = mixed_pair(p, x.vpk[v0 + k], x.vpk[j], e_cf, n_cf, fx, fy);
+                    rf[2 * kQueue + q] = mixed_pair(p, x.vpk[v0 + k], x.vpk[j], e_cf, n_cf, fx, fy);
                     rf[q] = fx;
-                    rf[kVertQueue + q] = fy;
+                    rf[kQueue + q] = fy;
                 } else {
                     double fx, fy;
                     const double ee = vertex_pair(fa, vc, m.vpos[k], fa.pos[j], fx, fy);
@@ -505,8 +511,8 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) kb_loop(BumpySys *bs, LoopSync
                     }
                     for (int e = b0; e < b1; e++) {
                         sx += rf[e - q0];
-                        sy += rf[kVertQueue + e - q0];
-                        se += rf[2 * kVertQueue + e - q0];
+                        sy += rf[kQueue + e - q0];
+                        se += rf[2 * kQueue + e - q0];
                     }
                     ax = (double)sx; ay = (double)sy; en = (double)se;
                 } else {

@@ -769,6 +769,18 @@ static int build_graph(BS *s, int kind) {
 // The resident grid: a block an SM.  It holds at most kLoopBodies bodies,
 // kBodyVerts vertices and list rows of kVertSlots; larger systems run the
 // loops as graphs of full-size kernels.
+struct BodyLoop {  // of a system: what its blocks' vertices need
+    void *fn[2];   // by kind
+    size_t smem;
+    int threads;   // 8 warps for the roles and the list builds, more where the vertices fill them
+};
+static const BodyLoop kBodyLoops[2] = {
+    {{(void *)kb_loop<0, kBodyVertsSmall>, (void *)kb_loop<1, kBodyVertsSmall>}, sizeof(BodyMem<kBodyVertsSmall>), 256},
+    {{(void *)kb_loop<0, kBodyVerts>, (void *)kb_loop<1, kBodyVerts>}, sizeof(BodyMem<kBodyVerts>), kLoopMaxTPB}};
+static const BodyLoop &body_loop(const BS *s) {
+    return kBodyLoops[(long long)s->lchunk * s->max_nvb > kBodyVertsSmall];
+}
+
 static int plan_resident(BS *s) {
     int dev = 0, nsm = 0, coop = 0;
     CK(cudaGetDevice(&dev));
@@ -777,12 +789,13 @@ static int plan_resident(BS *s) {
     nsm = std::min(nsm, kLoopBlocksMax);
     const int per = (s->nb + nsm - 1) / nsm;
     if (!coop || per > kLoopBodies) return set_err(DPG_ERR_STATE, "no resident loop for this system");
-    for (void *fn : {(void *)kb_loop<0>, (void *)kb_loop<1>}) {
-        int occ = 0;
-        CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BodyMem)));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kLoopMaxTPB, sizeof(BodyMem)));
-        if (occ < 1) return set_err(DPG_ERR_CUDA, "the resident loop does not fit an SM");
-    }
+    for (const BodyLoop &q : kBodyLoops)
+        for (void *fn : q.fn) {
+            int occ = 0;
+            CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)q.smem));
+            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, q.threads, q.smem));
+            if (occ < 1) return set_err(DPG_ERR_CUDA, "the resident loop does not fit an SM");
+        }
     s->lchunk = per;
     s->lblocks = (s->nb + per - 1) / per;
     return DPG_OK;
@@ -802,16 +815,14 @@ static int loop_failed(BS *s) {
 
 // *refused: the launch was, and the state is that between two iterations
 static int run_resident(BS *s, int kind, bool *refused) {
-    void *fn = kind == 0 ? (void *)kb_loop<0> : (void *)kb_loop<1>;
+    const BodyLoop &q = body_loop(s);
     long long most = std::max<long long>(256, (1LL << 24) / (s->nb + 1024));
     double dt = s->loop_dt, tmax = s->loop_tmax;
     void *args[] = {(void *)&s->d, (void *)&s->lsync, (void *)&dt, (void *)&tmax, (void *)&s->lchunk, (void *)&most,
                     (void *)&s->polls};
-    // 8 warps for the roles and the list builds, more where the vertices fill them
-    const int threads = (long long)s->lchunk * s->max_nvb > 256 ? kLoopMaxTPB : 256;
     do {
         CK(cudaMemsetAsync(s->lsync, 0, sizeof(LoopSync), s->stream));
-        const cudaError_t err = cudaLaunchCooperativeKernel(fn, dim3(s->lblocks), dim3(threads), args, sizeof(BodyMem), s->stream);
+        const cudaError_t err = cudaLaunchCooperativeKernel(q.fn[kind], dim3(s->lblocks), dim3(q.threads), args, q.smem, s->stream);
         *refused = err != cudaSuccess;
         if (*refused) {
             (void)cudaGetLastError();
