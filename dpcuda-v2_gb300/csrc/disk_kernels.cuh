@@ -1254,8 +1254,8 @@ __device__ __forceinline__ bool fire_energy(DevState &s, double &avg) {
 __device__ __forceinline__ void fire_switch(DevState &s, double f2) {
     if (f2 < 0.81 * s.best_f2) { s.best_f2 = f2; s.best_it = s.iter; }
     bool go = s.f_nbad > 5;
-    // far above 100 switch_fmax the root is not needed to tell
-    if (!go && f2 < 1.001e4 * s.switch_fmax * s.switch_fmax) {
+    // above 100 switch_fmax (which may be 0, as may f2) the root is not needed to tell
+    if (!go && !(f2 > 1.001e4 * s.switch_fmax * s.switch_fmax)) {
         const double fm = sqrt(f2);
         go = fm <= s.switch_fmax || (fm < 100.0 * s.switch_fmax && s.iter - s.best_it > 2000);
     }
