@@ -367,6 +367,12 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) kb_loop(BumpySys *bs, LoopSync
 
     load_own();
     if (KIND == 1) ok = nve_first();
+    if (KIND == 0 && s.pe_diff_target > 0) {  // as in k_tile
+        double tot[4] = {t < np ? L.b.w.pe[r.first + t] : 0.0, 0.0, 0.0, 0.0};
+        ok = grid_totals<4>(tot, (np + 31) / 32, L.b.w.partials, ls, bk, polls, red);
+        if (ok && t == 0) s.last_avg_pe = tot[0] / s.dof;
+        __syncthreads();
+    }
     while (ok) {
         if (KIND == 0) {
             // ---- move (src/integrator/fire.cu:29-40 with the rigid overrides)

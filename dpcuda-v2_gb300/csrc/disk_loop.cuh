@@ -589,6 +589,13 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_tile(DevSys *ds, LoopSync *l
 
     load_own();
     if (KIND == 1) ok = after_move(nve_first());
+    // the energy that the first iteration's is compared with, summed in the same order
+    if (KIND == 0 && s.pe_diff_target > 0) {
+        double tot[3] = {mine ? w.pe[own] : 0.0, 0.0, 0.0};
+        ok = grid_totals<3>(tot, (np + 31) / 32, w.partials, ls, bk, polls, red);
+        if (ok && t == 0) s.last_avg_pe = tot[0] / s.dof;
+        __syncthreads();
+    }
     while (ok) {
         if (KIND == 0) {
             // ---- move (k_fire_move)
@@ -843,6 +850,14 @@ __global__ void __launch_bounds__(kLoopMaxTPB, 1) k_loop(DevSys *ds, LoopSync *l
             const int kind = rebuild_kind(bw);
             if (kind) ok = loop_rebuild<M>(&L, ls, bk, polls, kind, r);
         }
+    }
+    if (KIND == 0 && s.pe_diff_target > 0) {  // as in k_tile
+        double tot[3] = {0.0, 0.0, 0.0};
+        for (int i = r.first + t / G; i < r.last; i += tile)
+            if (sub == 0) tot[0] += w.pe[i];
+        ok = grid_totals<3>(tot, nt / 32, w.partials, ls, bk, polls, red);
+        if (ok && t == 0) s.last_avg_pe = tot[0] / s.dof;
+        __syncthreads();
     }
     while (ok) {
         if (KIND == 0) {
