@@ -502,18 +502,21 @@ static int res_class_in(const int *table, int n) {
     return -1;
 }
 // FP64 passes cost their instructions, whatever lanes these have, and a particle
-// of more than 64 / 128 disks has 2 / 1 partial sums (res_order): more lanes than
-// that, or a second block, only spread the same instructions thinner.  So a system
-// in FP64 takes, of the first two tables, the shape with as many lanes as sums.
-// 300 iterations of one system by the wide table, by these: 100 disks 13.6 -> 8.9
-// ms, 200 23.9 -> 13.9, 256 24.6 -> 16.0, 300 24.3 -> 18.9, 512 24.4 -> 28.3.
+// of a system of up to 64 / up to 128 / more disks has 4 / 2 / 1 partial sums
+// (res_order): more lanes than that, or a second block, only spread the same
+// instructions thinner.  The double-word passes that an energy-change target asks
+// for run a lane a partial sum as well.  So such systems take, of the first two
+// tables, the shape with as many lanes as sums.  One system of 100 / 200 / 256 /
+// 300 / 512 disks by the wide table and by these, us an iteration: FP64 45 / 80 /
+// 82 / 81 / 81 and 30 / 46 / 53 / 63 / 94; double words with an energy-change
+// target 8.5 / 14.4 / 14.5 / 14.8 / 15.1 and 6.0 / 8.8 / 8.7 / 10.3 / 12.5.
 struct ResRow {
     int most, shape;
 };
 static const ResRow kResFp64[2][3] = {{{64, 0}, {128, 14}, {384, 15}}, {{64, 0}, {128, 14}, {512, 15}}};
 
 static int res_class_of(const ES *s, const ESys &y) {
-    if (s->rs_fp64 && y.prec == 1 && s->rs_table < 2)
+    if (s->rs_fp64 && (y.prec == 1 || s->h.p.pe_diff_target > 0) && s->rs_table < 2)
         for (const ResRow &q : kResFp64[s->rs_table])
             if (y.n <= q.most) return q.shape;
     return res_class_in(kResTables[s->rs_table], y.n);
