@@ -51,20 +51,6 @@ __device__ __forceinline__ bool raised(unsigned long long v, unsigned long long 
     return (v / flag & 0xffff) != 0;
 }
 
-// Polls that ran out with `v` (or found the word closed): closes it and returns 0,
-// or returns the completed word if the last arrivals came first.  Thread 0, and
-// apart from the barrier, whose path this should not lengthen.
-__device__ __noinline__ unsigned long long bar_short(LoopSync *ls, unsigned long long *w, unsigned long long v) {
-    while ((v & 0xffff) < gridDim.x) {  // another arrival makes it look again
-        const unsigned long long seen = atomicCAS(w, v, v | kClosed);
-        v = seen == v ? v | kClosed : seen;
-    }
-    __threadfence();
-    if (!(v & kClosed)) return v;
-    *(volatile int *)&ls->err = 1;
-    return 0;
-}
-
 // Grid barrier k; flags of thread 0 are added to the arrival; polls: how often a
 // wait looks (a launch argument, passed by value: kept beside k behind a reference
 // it cost a FIRE iteration of 16384 disks 0.5 %).  Returns the
@@ -105,7 +91,17 @@ __device__ __forceinline__ unsigned long long grid_bar(LoopSync *ls, unsigned &k
         do {
             asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(w) : "memory");
         } while ((v & 0xffff) < gridDim.x && ++n < polls);
-        if ((v & 0xffff) != gridDim.x) v = bar_short(ls, w, v);
+        if ((v & 0xffff) != gridDim.x) {  // run out, or closed
+            while ((v & 0xffff) < gridDim.x) {  // another arrival makes it look again
+                const unsigned long long seen = atomicCAS(w, v, v | kClosed);
+                v = seen == v ? v | kClosed : seen;
+            }
+            __threadfence();
+            if (v & kClosed) {
+                *(volatile int *)&ls->err = 1;
+                v = 0;
+            }
+        }
         if (blockIdx.x == 0) {
             ls->ring[(k + 2) & 3] = 0;
             __threadfence();
