@@ -946,6 +946,7 @@ extern "C" int dpg_bumpy_fire_minimize(dpg_bumpy_handle s, const dpg_fire_params
     DevState st = *s->hs;
     st.flags = 0; st.iter = 0; st.max_steps = p->max_steps; st.result_step = 0;
     st.pe_target = p->avg_pe_target; st.pe_diff_target = p->avg_pe_diff_target;
+    st.pe_read = pe_is_read(st.pe_target, st.pe_diff_target, s->prm.e_c, s->prm.n_c);
     st.fmax_target = p->fmax_target; st.dof = (double)s->nb;
     st.guard = 0; st.guard_limit = p->max_steps + 4; st.h_loop = 0; st.h_rb = 0;
     st.fp64_now = 0; st.switch_fmax = s->switch_fmax; st.best_f2 = INFINITY; st.best_it = 0;

@@ -1237,11 +1237,11 @@ __global__ void k_fire_move(DevSys *ds) {
 }
 
 // Mean energy of a FIRE iteration (s.pe) and whether it has stopped changing.
-// Without energy targets an energy that is not negative is below none, and the
-// FP64 division stays off the iteration's serial path (0: below no target).
+// Where no test reads it the FP64 division stays off the iteration's serial path
+// (0: below no target).
 __device__ __forceinline__ bool fire_energy(DevState &s, double &avg) {
     avg = 0.0;
-    if (!(s.pe_target > 0) && !(s.pe_diff_target > 0) && __double2hiint(s.pe) >= 0) return false;
+    if (!s.pe_read) return false;
     avg = s.pe / s.dof;
     const bool still = s.pe_diff_target > 0 && fabs(avg / s.last_avg_pe - 1) < s.pe_diff_target;
     s.last_avg_pe = avg;

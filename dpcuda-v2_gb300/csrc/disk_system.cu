@@ -1496,6 +1496,7 @@ static int fire_minimize(dpg_system *s, const dpg_fire_params *p, dpg_fire_resul
     st.result_step = 0;
     st.pe_target = p->avg_pe_target;
     st.pe_diff_target = p->avg_pe_diff_target;
+    st.pe_read = pe_is_read(st.pe_target, st.pe_diff_target, s->prm.e_c, s->prm.n_c);
     st.fmax_target = p->fmax_target;
     st.dof = (double)s->n;
     st.guard = 0;
@@ -1556,6 +1557,7 @@ extern "C" int dpg_profile_loop(dpg_handle s, int kind, int iters, double dt, do
         TRY(pull_state(s));
         DevState st = *s->hs;
         st.flags = 0; st.iter = 0; st.max_steps = p.max_steps; st.pe_target = 0; st.pe_diff_target = 0;
+        st.pe_read = pe_is_read(0, 0, s->prm.e_c, s->prm.n_c);
         st.fmax_target = 0; st.dof = (double)s->n; st.h_loop = 0; st.h_rb = 0;
         CK(cudaMemcpyAsync(&s->d->s, &st, sizeof(DevState), cudaMemcpyHostToDevice, s->stream));
         LAUNCH(k_zero_vel, s->grid(s->n), s->tpb, s->d);

@@ -11,6 +11,12 @@ namespace dpg {
 // Records a message for dpg_last_error() (thread-local) and returns `code`.
 int set_error(int code, const char *fmt, ...);
 
+// Whether a FIRE minimisation tests its mean energy: against a target, or against
+// zero where energies can be negative.
+inline int pe_is_read(double pe_target, double pe_diff_target, double e_c, double n_c) {
+    return pe_target > 0 || pe_diff_target > 0 || !(e_c > 0) || !(n_c > 0);
+}
+
 // cudaMemcpyAsync to the caller's host memory.  Into pages that were not touched
 // yet (every array that a caller has just allocated) the driver copies at
 // 1.2 GB/s, four arrays of 262144 doubles in 6.7 ms; a byte written to each page
