@@ -31,7 +31,6 @@ struct BumpyExt {
     double2 *vpos, *vpos_t;
     double *vmass, *vmass_t;
     int *vbody, *vbody_t, *svidx, *svidx_t;
-    int *o2n;                // old -> new body slot during a re-sort
     int *vnbr, *vcount;      // vertex neighbour list, column-major [capv][nv]
     float4 *vpk;             // mixed form: packed FP32 vertex offsets (see mixed_pack)
     uint4 *vq;               // fixed-point vertex positions (see Quant in dpg_device.cuh)
@@ -437,7 +436,6 @@ __device__ __forceinline__ void reorder_body(BumpySys *bs, int s) {
     DevSys &d = bs->b;
     BumpyExt &x = bs->x;
     int o = d.w.perm[s];
-    x.o2n[o] = s;
     double2 p = d.v.pos[o];
     d.v.pos_t[s] = p;
     d.v.vel_t[s] = d.v.vel[o];

@@ -169,7 +169,7 @@ extern "C" int dpg_bumpy_create(const dpg_bumpy_params *p, void *cuda_stream, dp
     A((void **)&x.w, nb * 8); A((void **)&x.th, nb * 8); A((void **)&x.tq, nb * 8); A((void **)&x.I, nb * 8);
     A((void **)&x.nvb, nb * 4); A((void **)&x.start, nb * 4);
     A((void **)&x.w_t, nb * 8); A((void **)&x.th_t, nb * 8); A((void **)&x.tq_t, nb * 8); A((void **)&x.I_t, nb * 8);
-    A((void **)&x.nvb_t, nb * 4); A((void **)&x.start_t, nb * 4); A((void **)&x.o2n, nb * 4);
+    A((void **)&x.nvb_t, nb * 4); A((void **)&x.start_t, nb * 4);
     A((void **)&x.vpos, nv * 16); A((void **)&x.vpos_t, nv * 16); A((void **)&x.vmass, nv * 8);
     A((void **)&x.vmass_t, nv * 8); A((void **)&x.vbody, nv * 4); A((void **)&x.vbody_t, nv * 4);
     A((void **)&x.svidx, nv * 4); A((void **)&x.svidx_t, nv * 4); A((void **)&x.vcount, nv * 4);
