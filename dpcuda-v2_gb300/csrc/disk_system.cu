@@ -153,7 +153,10 @@ struct dpg_system {
 };
 
 // The loops run as one resident grid up to kLoopMaxN particles, as a graph of
-// full-size kernels above (see plan_resident).
+// full-size kernels above (see plan_resident).  Resident against graph, us a step
+// or iteration: 65536 disks NVE 32 / 48, FIRE 47 / 70, mixed 15 / 33 and 29 / 50;
+// 131072 disks 55 / 77, 79 / 111, mixed 27 / 45 and 45 / 74.  So the line is not
+// where the graph becomes faster but as far as the resident loops are tested.
 constexpr int kLoopMaxN = 1 << 17;
 // Up to kClusterN particles k_tile runs on one cluster of at most 16 blocks,
 // whose barrier is shorter than the grid's through L2; more particles want more
