@@ -38,7 +38,7 @@ extern "C" {
 #define DPG_ERR_OVERFLOW 3     /* neighbour capacity exceeded and could not grow */
 #define DPG_ERR_NOT_CONVERGED 4
 #define DPG_ERR_STATE 5        /* call out of order (e.g. forces before neighbours) */
-#define DPG_ERR_TIMEOUT 6      /* a bounded device wait ran out */
+#define DPG_ERR_TIMEOUT 6      /* a bounded device wait ran out (set state and lists up again) */
 
 #define DPG_HOST 0
 #define DPG_DEVICE 1
